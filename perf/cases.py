@@ -409,7 +409,7 @@ def _exact_samples(data, scan, el, angles, t_start, geom, config, *, speed=None,
             sample = (tau - start) * geom.fs
             valid = (sample >= 0) & (sample <= ns - 1)
             if geom.fnumber is not None:
-                valid &= distance.abs() <= z / (2 * geom.fnumber)
+                valid &= distance.abs() <= z / (2 * float(np.float32(geom.fnumber)))
             sample = sample.clamp(0, ns - 1)
             row = sample.floor()
             weight = sample - row
@@ -475,7 +475,7 @@ def _exact_angles(scan, data, el, angles, t_start, geom, config):
             magnitude += channel.abs()
     coords = scan[:, 2 if config else 0, None] - torch.as_tensor(np.asarray(el, np.float32),
                                                                  device=scan.device).double()
-    limit = math.inf if geom.fnumber is None else scan[:, 1:2] / (2 * geom.fnumber)
+    limit = math.inf if geom.fnumber is None else scan[:, 1:2] / (2 * float(np.float32(geom.fnumber)))
     return per_angle, root, magnitude, (coords.abs() <= limit).sum(1).double()
 
 
