@@ -292,7 +292,8 @@ rcabeam_status rcabeam_opw_offsets_adjoint_device(const void* rc, const void* cr
  * own grid (scan, optional traversal order from rcabeam_voxel_order_device),
  * geometry, power output (2 * nv floats, result in the even entries) and
  * method: 0 OPW, 1 XDoppler, 3 DMAS-CCF-ACF.  frames_per_chunk (16, 32, 64;
- * 0 = 64) is the staged methods' frame chunk, chosen by an autotuner. */
+ * 0 = 64), chosen by an autotuner: 64 leaves the split of an ensemble into work
+ * items to the library, 16 and 32 bound an item's frames. */
 typedef struct rcabeam_batch_ensemble {
   const void* rc;
   const void* cr;
@@ -319,9 +320,9 @@ rcabeam_status rcabeam_batch_prepare(size_t n, const rcabeam_batch_ensemble* lis
 
 /* Enqueues on `stream` (a cudaStream_t; capturable into a CUDA graph): clears
  * the counters and every pd, then runs the persistent kernel with ctas_per_sm
- * (1-3) CTAs per SM (a queue of one method runs that method's own kernel), or
- * with ctas_per_sm = 0 launches every ensemble through the single-ensemble
- * kernels in queue order.  times (device, n + 1 uint64): start, then each
+ * (1-3; at most as many as fit) CTAs per SM, or with ctas_per_sm = 0, and for
+ * queues of several methods, launches every ensemble through the
+ * single-ensemble kernels in queue order.  times (device, n + 1 uint64): start, then each
  * ensemble's completion, in global-timer nanoseconds. */
 rcabeam_status rcabeam_batch_run_device(size_t n, const rcabeam_batch_ensemble* list, void* table,
                                         size_t table_bytes, unsigned long long* times, int ctas_per_sm,

@@ -9,10 +9,7 @@ large ensembles share the GPU without launch gaps or per-ensemble tails, with
 a kernel compiled for that method alone) or as per-ensemble launches of the
 single-ensemble kernels (``ctas_per_sm`` 0), whichever ``autotune`` measures
 faster for that method on bounded samples of its ensembles (it also picks the
-staged pipeline's frame chunk per shape class).  Ensembles that fill the GPU
-alone run the single-ensemble kernels faster than the persistent loop for
-OPW and DMAS-CCF-ACF; XDoppler's persistent kernel is the faster one.  The
-sub-queues run one after another on one stream (run concurrently, their
+most frames of an item per shape class).  The sub-queues run one after another on one stream (run concurrently, their
 sample windows compete for L2) and the whole queue is captured into one CUDA
 graph.  Per-ensemble completion times come from the device's global timer.
 
@@ -87,7 +84,7 @@ class Ensemble:
         t = dict(scan=scan, xe=f32(self.geom.x_el), ye=f32(self.geom.y_el), angles=f32(self.angles),
                  starts=f32(np.broadcast_to(np.asarray(self.t_start, np.float32), (na,))),
                  pd=torch.zeros((nv, 2), dtype=torch.float32, device=device), order=None)
-        if order and nv >= 128:  # every method's 64-voxel tiles want compact (Morton) voxel sets
+        if order and nv >= 128:  # every method's voxel tiles want compact (Morton) voxel sets
             size = ctypes.c_size_t(0)
             _lib.check(_lib.lib().rcabeam_voxel_order_workspace_bytes(nv, ctypes.byref(size)), "voxel_order")
             ws = torch.empty(int(size.value), dtype=torch.uint8, device=device)
@@ -144,15 +141,13 @@ class _SubQueue:
 
     def kernel_launches(self) -> int:
         """Kernels one launch() enqueues: the persistent kernel, or per ensemble its
-        single-ensemble kernels (64-frame chunks plus a tail launch; XDoppler's
-        magnitude pass; DMAS one) and a completion stamp, plus the start stamp."""
+        delay-and-sum (XDoppler with its magnitude pass) and a completion stamp,
+        plus the start stamp."""
         if self.ctas_per_sm:
             return 1
         total = 1
         for e in self.ensembles:
-            nt = e.shape[3]
-            das = 1 if e.method == "dmas" else (nt >= 64) + (nt % 64 > 0) + (e.method == "xdoppler")
-            total += das + 1
+            total += 2 + (e.method == "xdoppler")
         return total
 
     def launch(self, stream) -> None:

@@ -1,14 +1,10 @@
-// Frame-batched nonlinear beamformers that need per-angle or per-channel
-// partial sums: RC-FMAS (method 2) and DMAS-CCF-ACF (method 3), plus the
-// per-frame entry points of the reference's single-frame API (core.cu).
-// One warp owns one voxel; lanes own frames (four register frames each), the
-// float64 taps are formed once per (channel, angle) by every lane in lockstep.
-// These are not on the OPW hot path; they keep the reference's method set and
-// the batching form's mixed queue complete.
+// St-SW (method 4) of the frame-batched path and the per-frame entry points of
+// the reference's single-frame API (core.cu).  One warp owns one voxel; lanes
+// own frames.
 #pragma once
 
 #include "common.cuh"
-#include "das_staged.cuh"
+#include "das_rows.cuh"
 
 namespace rcb {
 namespace generic {
@@ -66,166 +62,6 @@ __device__ __forceinline__ Tap lane_tap_tx(const das::Args& p, const Voxel& q, i
   bool act;
   const double trx = receive_delay(config ? q.y : q.x, q.z, double((config ? p.ye : p.xe)[ch]), p.c, p.fn, &act);
   return make_tap(__dadd_rn(config ? tx.cr : tx.rc, trx), tx.start, p.fs, p.fd, p.ns, act);
-}
-
-__device__ __forceinline__ Tap shfl_tap(const Tap& t, int src) {
-  Tap o;
-  o.i0 = __shfl_sync(0xffffffffu, t.i0, src);
-  o.w = __shfl_sync(0xffffffffu, t.w, src);
-  o.phase.x = __shfl_sync(0xffffffffu, t.phase.x, src);
-  o.phase.y = __shfl_sync(0xffffffffu, t.phase.y, src);
-  return o;
-}
-
-// Taps of one aperture for channel `outer` (all angles, chan_major = false) or
-// angle `outer` (all channels, chan_major = true), computed one per lane for
-// the 32 inner indices starting at `first`; lanes past the end get an empty tap.
-__device__ __forceinline__ Tap lane_tap(const das::Args& p, const Voxel& q, int config, bool chan_major, int outer,
-                                        int first) {
-  const int inner = first + (threadIdx.x & 31);
-  const int limit = chan_major ? p.nc : p.na;
-  if (inner >= limit) return Tap{-1, 0.f, make_float2(0.f, 0.f)};
-  const int ch = chan_major ? inner : outer, a = chan_major ? outer : inner;
-  return tap_of(q, config, config ? p.ye : p.xe, ch, p.angles, p.starts, a, p.c, p.fs, p.fd, p.fn, p.ns);
-}
-
-// One warp: voxel v (its row in scan / pd / signal), frames [128 fblock, 128 fblock + 128).
-// The float64 taps of every (channel, angle) are formed once per warp, one per
-// lane, and broadcast with shuffles.
-template <int METHOD>
-__device__ void nonlinear_voxel(const das::Args& p, size_t v, int fblock) {
-  const int lane = threadIdx.x & 31;
-  const int fbase = fblock * 32 * kRegFrames + lane;
-  const Voxel q = load_voxel(p.scan, v);
-  const float2* rc = static_cast<const float2*>(p.rc);
-  const float2* cr = static_cast<const float2*>(p.cr);
-  float power[kRegFrames];
-  if constexpr (METHOD == 2) {
-    // RC-FMAS: sum over angles of signed square roots of channel sums, RC * CR.
-    float2 r[kRegFrames] = {}, s[kRegFrames] = {};
-    // Each lane forms one channel's taps; the warp reads them back from shared memory.
-    __shared__ __align__(16) Tap taps[kWarps][2][32];
-    Tap* tap_rc = taps[threadIdx.x >> 5][0];
-    Tap* tap_cr = taps[threadIdx.x >> 5][1];
-    for (int a = 0; a < p.na; ++a) {
-      float2 ar[kRegFrames] = {}, aq[kRegFrames] = {};
-      const AngleTx tx = angle_tx(p, q, a);
-      for (int c0 = 0; c0 < p.nc; c0 += 32) {
-        __syncwarp();  // the previous chunk's reads are done
-        tap_rc[lane] = lane_tap_tx(p, q, 0, c0, tx);
-        tap_cr[lane] = lane_tap_tx(p, q, 1, c0, tx);
-        __syncwarp();
-        const int count = min(32, p.nc - c0);
-        for (int j = 0; j < count; ++j) {
-          const int ch = c0 + j;
-          const Tap tr = tap_rc[j], tq = tap_cr[j];
-#pragma unroll
-          for (int f = 0; f < kRegFrames; ++f) {
-            int frame = fbase + 32 * f;
-            ar[f] = cadd(ar[f], packed_sample(rc, tr, ch, a, frame, p.ns, p.na, p.nt));
-            aq[f] = cadd(aq[f], packed_sample(cr, tq, ch, a, frame, p.ns, p.na, p.nt));
-          }
-        }
-      }
-#pragma unroll
-      for (int f = 0; f < kRegFrames; ++f) {
-        r[f] = cadd(r[f], csroot(ar[f]));
-        s[f] = cadd(s[f], csroot(aq[f]));
-      }
-    }
-#pragma unroll
-    for (int f = 0; f < kRegFrames; ++f) {
-      float2 val = cmul(r[f], s[f]);
-      int frame = fbase + 32 * f;
-      if (frame < p.nt && p.signal) p.signal[v * p.nt + frame] = val;
-      power[f] = frame < p.nt ? cabs2(val) : 0.f;
-    }
-  } else {
-    // DMAS-CCF-ACF (reference ensemble.cu:143-232): pass 1 over channels for the
-    // signed-sqrt DMAS and CCF terms, pass 2 over angles for the ACF terms.
-    float2 sqrt_sum[kRegFrames] = {};
-    float abs_sum[kRegFrames] = {};
-    float active = 0.f;
-    for (int ch = 0; ch < p.nc; ++ch) {
-      float2 sr[kRegFrames] = {}, sq[kRegFrames] = {};
-      bool act_r = false, act_q = false;
-      for (int a0 = 0; a0 < p.na; a0 += 32) {
-        const Tap lr = lane_tap(p, q, 0, false, ch, a0), lq = lane_tap(p, q, 1, false, ch, a0);
-        const int count = min(32, p.na - a0);
-        for (int j = 0; j < count; ++j) {
-          const int a = a0 + j;
-          const Tap tr = shfl_tap(lr, j), tq = shfl_tap(lq, j);
-#pragma unroll
-          for (int f = 0; f < kRegFrames; ++f) {
-            int frame = fbase + 32 * f;
-            sr[f] = cadd(sr[f], packed_sample(rc, tr, ch, a, frame, p.ns, p.na, p.nt));
-            sq[f] = cadd(sq[f], packed_sample(cr, tq, ch, a, frame, p.ns, p.na, p.nt));
-          }
-        }
-      }
-      receive_delay(q.x, q.z, double(p.xe[ch]), p.c, p.fn, &act_r);
-      receive_delay(q.y, q.z, double(p.ye[ch]), p.c, p.fn, &act_q);
-      active += float(act_r) + float(act_q);
-#pragma unroll
-      for (int f = 0; f < kRegFrames; ++f) {
-        sqrt_sum[f] = cadd(sqrt_sum[f], cadd(csroot(sr[f]), csroot(sq[f])));
-        abs_sum[f] += hypotf(sr[f].x, sr[f].y) + hypotf(sq[f].x, sq[f].y);
-      }
-    }
-    float2 r[kRegFrames] = {}, s[kRegFrames] = {};
-    float er[kRegFrames] = {}, eq[kRegFrames] = {};
-    for (int a = 0; a < p.na; ++a) {
-      float2 ar[kRegFrames] = {}, aq[kRegFrames] = {};
-      for (int c0 = 0; c0 < p.nc; c0 += 32) {
-        const Tap lr = lane_tap(p, q, 0, true, a, c0), lq = lane_tap(p, q, 1, true, a, c0);
-        const int count = min(32, p.nc - c0);
-        for (int j = 0; j < count; ++j) {
-          const int ch = c0 + j;
-          const Tap tr = shfl_tap(lr, j), tq = shfl_tap(lq, j);
-#pragma unroll
-          for (int f = 0; f < kRegFrames; ++f) {
-            int frame = fbase + 32 * f;
-            ar[f] = cadd(ar[f], packed_sample(rc, tr, ch, a, frame, p.ns, p.na, p.nt));
-            aq[f] = cadd(aq[f], packed_sample(cr, tq, ch, a, frame, p.ns, p.na, p.nt));
-          }
-        }
-      }
-#pragma unroll
-      for (int f = 0; f < kRegFrames; ++f) {
-        r[f] = cadd(r[f], ar[f]);
-        s[f] = cadd(s[f], aq[f]);
-        er[f] += cabs2(ar[f]);
-        eq[f] += cabs2(aq[f]);
-      }
-    }
-    const float inv = 1.0f / float(p.na);
-#pragma unroll
-    for (int f = 0; f < kRegFrames; ++f) {
-      float dm = cabs2(sqrt_sum[f]) - abs_sum[f];
-      float wc = (active > 0.f && abs_sum[f] > 0.f) ? fmaxf(dm, 0.f) / active / abs_sum[f] : 0.f;
-      float nr = cabs2(r[f]) * inv * inv, nq = cabs2(s[f]) * inv * inv;
-      float var = fmaxf(er[f] * inv - nr, 0.f) + fmaxf(eq[f] * inv - nq, 0.f);
-      float num = sqrtf(nr) * sqrtf(nq), den = nr + nq + var / 2 - num;
-      float pw = den > 0.f ? dm * wc * (num / den) : 0.f;
-      if (!isfinite(pw)) pw = 0.f;
-      int frame = fbase + 32 * f;
-      if (frame < p.nt && p.signal) p.signal[v * p.nt + frame] = make_float2(pw, 0.f);
-      power[f] = frame < p.nt ? pw : 0.f;
-    }
-  }
-  float total = 0.f;
-#pragma unroll
-  for (int f = 0; f < kRegFrames; ++f) total += power[f];
-#pragma unroll
-  for (int off = 16; off > 0; off >>= 1) total += __shfl_xor_sync(0xffffffffu, total, off);
-  if (lane == 0) atomicAdd(p.pd + 2 * v, total / float(p.nt));
-}
-
-template <int METHOD>
-__global__ void __launch_bounds__(kWarps * 32) ensemble_nonlinear(das::Args p) {
-  const size_t v = size_t(blockIdx.x) * kWarps + (threadIdx.x >> 5);
-  if (v >= size_t(p.nv)) return;
-  nonlinear_voxel<METHOD>(p, v, blockIdx.y);
 }
 
 // ------------------------------------------------------------ St-SW --

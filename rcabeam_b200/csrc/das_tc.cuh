@@ -54,7 +54,7 @@
 #include <climits>
 
 #include "common.cuh"
-#include "das_staged.cuh"
+#include "das_rows.cuh"
 
 namespace rcb {
 namespace tc {

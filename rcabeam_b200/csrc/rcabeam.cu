@@ -19,7 +19,7 @@
 #include "batch.cuh"
 #include "das_adjoint.cuh"
 #include "das_generic.cuh"
-#include "das_staged.cuh"
+#include "das_rows.cuh"
 #include "das_tc.cuh"
 #include "gram_tc.cuh"
 #include "pack.cuh"
@@ -48,21 +48,6 @@ static PFN_cuTensorMapEncodeTiled_v12000 encode_fn() {
       fn = reinterpret_cast<PFN_cuTensorMapEncodeTiled_v12000>(p);
   });
   return fn;
-}
-
-// Packed (slabs = nc * na, ns, nt) ensemble as a 3-D tensor of elem_bytes elements.
-static bool make_slab_map(CUtensorMap* map, const void* base, int elem_bytes, size_t nt, size_t ns, size_t slabs,
-                          int box_frames, int box_rows) {
-  auto fn = encode_fn();
-  if (!fn) return false;
-  cuuint64_t dims[3] = {nt, ns, slabs};
-  cuuint64_t strides[2] = {nt * elem_bytes, nt * ns * elem_bytes};
-  cuuint32_t box[3] = {cuuint32_t(box_frames), cuuint32_t(box_rows), 1};
-  cuuint32_t estr[3] = {1, 1, 1};
-  CUtensorMapDataType dt = elem_bytes == 8 ? CU_TENSOR_MAP_DATA_TYPE_UINT64 : CU_TENSOR_MAP_DATA_TYPE_UINT32;
-  return fn(map, dt, 3, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-            CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-            CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
 // Packed 16-bit (re, im) plane (slabs, ns, 2 nt) as 16-bit elements with 64 x 16
@@ -143,11 +128,12 @@ __global__ void morton_kernel(const float* scan, size_t nv, const unsigned* box,
   vals[i] = unsigned(i);
 }
 
+constexpr size_t kOrderMin = 128;  // voxels below which a call runs in identity order
 static size_t align256(size_t x) { return (x + 255) & ~size_t(255); }
 
 // Scratch bytes of voxel_order for nv voxels (0 when no order is built).
 static size_t order_bytes(size_t nv, size_t* temp_bytes) {
-  if (nv < 2 * das::kTileVoxels || nv > 0x7fffffffull) return 0;
+  if (nv < kOrderMin || nv > 0x7fffffffull) return 0;
   cub::DoubleBuffer<unsigned> keys(nullptr, nullptr), vals(nullptr, nullptr);
   size_t temp = 0;
   if (cub::DeviceRadixSort::SortPairs(nullptr, temp, keys, vals, int(nv), 0, 30, cudaStream_t(0)) != cudaSuccess)
@@ -183,87 +169,156 @@ static const unsigned* voxel_order(const float* scan, size_t nv, void* workspace
 }
 
 // ---------------------------------------------------------- dispatch --
-static unsigned pow2_at_least(unsigned x) {
-  unsigned p = 1;
-  while (p < x) p <<= 1;
-  return p;
+static int sm_count() {
+  int dev = 0, sms = 148;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  return sms;
 }
 
-template <int LPV, bool HALF, int MODE, bool TMA>
-static rcabeam_status launch_staged(const CUtensorMap& mr, const CUtensorMap& mq, const das::Args& a, dim3 grid,
-                                    cudaStream_t stream) {
-  using S = das::Shape<LPV, HALF>;
-  auto kern = das::opw_staged<LPV, HALF, MODE, TMA>;
-  size_t smem = S::bytes(a.na);
-  if (smem > 48 * 1024 &&
-      cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)) != cudaSuccess)
+// Packed (slabs = nc * na, ns, nt) complex64 channels as a 3-D tensor with
+// boxes of box_frames x 8 rows.
+static bool make_row_map(CUtensorMap* map, const void* base, size_t nt, size_t ns, size_t slabs, int box_frames) {
+  auto fn = encode_fn();
+  if (!fn) return false;
+  cuuint64_t dims[3] = {nt, ns, slabs};
+  cuuint64_t strides[2] = {nt * 8, nt * ns * 8};
+  cuuint32_t box[3] = {cuuint32_t(box_frames), cuuint32_t(das::kBoxRows), 1};
+  cuuint32_t estr[3] = {1, 1, 1};
+  return fn(map, CU_TENSOR_MAP_DATA_TYPE_UINT64, 3, const_cast<void*>(base), dims, strides, box, estr,
+            CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+            CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+// Split of one ensemble over the delay-and-sum kernel (das_rows.cuh).
+struct RowsPlan {
+  das::Maps maps;
+  das::Shape shape;
+  das::Layout layout;
+  int width;  // frame pairs the kernel variant is compiled for
+};
+
+// Items of up to 104 frames (OPW; fewer for the methods that keep partial
+// results in shared memory).  13 pairs per thread keep a tap's cost small beside
+// its 26 frames; up to 32 frames run 8 pairs, whose kernel leaves room for
+// several CTAs per SM.
+template <int MODE>
+static RowsPlan plan_items(const das::Args& a, bool half, int sms, int most) {
+  constexpr int kStash = das::kStash<MODE>;
+  const int elem = half ? 4 : 8;
+  RowsPlan r{};
+  das::Shape& sp = r.shape;
+  das::Layout& lt = r.layout;
+  const int tiles = int((size_t(a.nv) + das::kTileVoxels - 1) / das::kTileVoxels);
+  int chunks = (a.nt + most - 1) / most;
+  // Few tiles: shorter items, so that every SM has one.
+  while ((long long)tiles * chunks < sms && (a.nt + chunks - 1) / chunks > 16) ++chunks;
+  const int per = (a.nt + chunks - 1) / chunks;
+  r.width = kStash == 0 && per > 32 ? 13 : 8;
+  sp.groups = (per + 2 * r.width - 1) / (2 * r.width);
+  sp.pairs = (per + 2 * sp.groups - 1) / (2 * sp.groups);
+  sp.frames = 2 * sp.pairs * sp.groups;
+  sp.chunks = (a.nt + sp.frames - 1) / sp.frames;
+  sp.contiguous = sp.chunks == 1;
+  sp.boxes = !half && a.nt % 2 == 0 && reinterpret_cast<uintptr_t>(a.rc) % 16 == 0 &&
+             reinterpret_cast<uintptr_t>(a.cr) % 16 == 0;
+  if (sp.boxes) {
+    // Rows 16 bytes beyond a multiple of 128 apart: the 16-byte loads of eight
+    // neighbouring rows then fall into distinct banks.
+    const int box = (sp.frames + 13) / 16 * 16 + 2;
+    sp.pitch = box * 8;
+    const size_t slabs = size_t(a.nc) * a.na;
+    if (!make_row_map(&r.maps.map[0], a.rc, size_t(a.nt), size_t(a.ns), slabs, box) ||
+        !make_row_map(&r.maps.map[1], a.cr, size_t(a.nt), size_t(a.ns), slabs, box))
+      sp.boxes = 0;
+  }
+  if (!sp.boxes)  // equal to the row stride modulo 16 (Builder::copy_rows)
+    sp.pitch = sp.contiguous ? a.nt * elem : das::align16(sp.frames * elem) + 16 + a.nt % (16 / elem) * elem;
+  const int consumers = das::kBlocks * sp.groups;
+  const int row_slack = sp.frames * elem + 64;  // threads past the last frame read on
+  lt.builders = 3;
+  lt.threads = 32 * (lt.builders + consumers);
+  lt.angles = a.na;
+  lt.zero_bytes = das::align16(2 * sp.pitch + row_slack);
+  lt.stash_bytes = kStash * 2 * sp.pairs * 4 * 32 * consumers;
+  sp.tx_table = 1;
+  lt.table_bytes = 12 * das::kTileVoxels * a.na;
+  // CTAs per SM that the registers leave room for.
+  const int resident = r.width == 8 && kStash == 0 ? std::max(1, 24 / (lt.threads / 32)) : 1;
+  auto fit = [&](int cap, int least) {
+    const int fixed = das::kFixedBytes + 24 * a.na + lt.zero_bytes + lt.stash_bytes + lt.table_bytes;
+    if (cap <= fixed) return false;
+    auto rows_of = [&](int bytes) {
+      const int n = (bytes - das::kTapBytes - row_slack) / sp.pitch;
+      return sp.boxes ? n / das::kBoxRows * das::kBoxRows : n;
+    };
+    // More rows than a compact tile needs would only cost a CTA its neighbours.
+    const long long enough = (das::kTapBytes + row_slack + 96ll * sp.pitch + 255) / 256 * 128;
+    lt.stages = 2 * lt.builders;
+    lt.stage_bytes = int(std::min<long long>((cap - fixed) / lt.stages / 128 * 128, enough));
+    sp.rows = rows_of(2 * lt.stage_bytes);
+    sp.rows_deep = std::max(rows_of(lt.stage_bytes), 0);
+    lt.smem = fixed + lt.stages * lt.stage_bytes;
+    return sp.rows >= least;
+  };
+  const int all = 227 * 1024;
+  if (fit(all / resident - (resident > 1 ? 1024 : 0), 40) || fit(all, 16)) return r;
+  sp.tx_table = lt.table_bytes = 0;  // many angles: transmit delays are formed per step
+  if (!fit(all, 16)) lt.smem = 0;
+  return r;
+}
+
+template <int MODE>
+static RowsPlan plan_rows(const das::Args& a, bool half, int sms, int max_frames = INT32_MAX) {
+  constexpr int kStash = das::kStash<MODE>;
+  int most = std::min(kStash == 0 ? 104 : kStash == 2 ? 64 : 48, std::max(max_frames, 2));
+  RowsPlan r = plan_items<MODE>(a, half, sms, most);
+  while (!r.layout.smem && most > 2) r = plan_items<MODE>(a, half, sms, most /= 2);  // very many angles
+  return r;
+}
+
+template <int MODE, int PAIRS, bool HALF, bool BOXES>
+static rcabeam_status launch_rows(const das::Args& a, const RowsPlan& r, unsigned items, cudaStream_t stream) {
+  auto kern = das::das_rows<MODE, PAIRS, HALF, BOXES>;
+  if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, r.layout.smem) != cudaSuccess)
     return RCABEAM_ERROR_CUDA;
-  kern<<<grid, das::kThreads, smem, stream>>>(mr, mq, a);
+  kern<<<items, r.layout.threads, r.layout.smem, stream>>>(r.maps, a, r.shape, r.layout);
   return launch_status();
 }
 
-template <bool HALF, int MODE, bool TMA>
-static rcabeam_status launch_lpv(int lpv, const CUtensorMap& mr, const CUtensorMap& mq, const das::Args& a,
-                                 dim3 grid, cudaStream_t stream) {
-  switch (lpv) {
-    case 32: return launch_staged<32, HALF, MODE, TMA>(mr, mq, a, grid, stream);
-    case 16: return launch_staged<16, HALF, MODE, TMA>(mr, mq, a, grid, stream);
-    case 8: return launch_staged<8, HALF, MODE, TMA>(mr, mq, a, grid, stream);
-    case 4: return launch_staged<4, HALF, MODE, TMA>(mr, mq, a, grid, stream);
-    default: return launch_staged<2, HALF, MODE, TMA>(mr, mq, a, grid, stream);
+template <int MODE, bool HALF>
+static rcabeam_status run_rows(const das::Args& a, cudaStream_t stream = 0) {
+  const RowsPlan r = plan_rows<MODE>(a, HALF, sm_count());
+  if (!r.layout.smem) return RCABEAM_ERROR_ARGUMENT;
+  const size_t items = (size_t(a.nv) + das::kTileVoxels - 1) / das::kTileVoxels * size_t(r.shape.chunks);
+  if (items > INT32_MAX) return RCABEAM_ERROR_ARGUMENT;
+  const unsigned n = unsigned(items);
+  if constexpr (HALF) {
+    return r.width == 13 ? launch_rows<MODE, 13, true, false>(a, r, n, stream)
+                         : launch_rows<MODE, 8, true, false>(a, r, n, stream);
+  } else {
+    if constexpr (MODE == das::kOpw) {
+      if (r.width == 13)
+        return r.shape.boxes ? launch_rows<MODE, 13, false, true>(a, r, n, stream)
+                             : launch_rows<MODE, 13, false, false>(a, r, n, stream);
+    }
+    return r.shape.boxes ? launch_rows<MODE, 8, false, true>(a, r, n, stream)
+                         : launch_rows<MODE, 8, false, false>(a, r, n, stream);
   }
 }
 
-template <bool HALF, int MODE>
-static rcabeam_status run_staged(das::Args a, size_t ntiles, cudaStream_t stream = 0) {
-  const int elem = HALF ? 4 : 8;
-  const size_t nt = size_t(a.nt);
-  const bool aligned = (nt * elem) % 16 == 0 && reinterpret_cast<uintptr_t>(a.rc) % 16 == 0 &&
-                       reinterpret_cast<uintptr_t>(a.cr) % 16 == 0 && encode_fn() != nullptr;
-  const int main_chunks = int(nt / 64);
-  const int tail = int(nt % 64);
-  struct Launch {
-    int lpv, frames, chunks, base;
-  } launches[2];
-  int count = 0;
-  if (main_chunks) launches[count++] = {32, 64, main_chunks, 0};
-  if (tail) {
-    int frames = int(pow2_at_least(unsigned(tail)));
-    if (frames < 4) frames = 4;
-    launches[count++] = {frames / 2, frames, 1, main_chunks * 64};
+// Methods 0-3 and 5 of the float32 path on `stream`.
+static rcabeam_status run_method(const das::Args& a, int method, cudaStream_t stream = 0) {
+  switch (method) {
+    case 0: return run_rows<das::kOpw, false>(a, stream);
+    case 2: return run_rows<das::kFmas, false>(a, stream);
+    case 3: return run_rows<das::kDmas, false>(a, stream);
+    case 5: return run_rows<das::kApertures, false>(a, stream);
+    default: break;
   }
-  for (int i = 0; i < count; ++i) {
-    CUtensorMap mr{}, mq{};
-    bool tma = aligned && make_slab_map(&mr, a.rc, elem, nt, size_t(a.ns), size_t(a.nc) * a.na,
-                                        launches[i].frames, das::kRows) &&
-               make_slab_map(&mq, a.cr, elem, nt, size_t(a.ns), size_t(a.nc) * a.na, launches[i].frames, das::kRows);
-    das::Args b = a;
-    b.frame_base = launches[i].base;
-    dim3 grid(unsigned(ntiles), unsigned(launches[i].chunks));
-    rcabeam_status st = tma ? launch_lpv<HALF, MODE, true>(launches[i].lpv, mr, mq, b, grid, stream)
-                            : launch_lpv<HALF, MODE, false>(launches[i].lpv, mr, mq, b, grid, stream);
-    if (st != RCABEAM_SUCCESS) return st;
-  }
-  return RCABEAM_SUCCESS;
-}
-
-// DMAS-CCF-ACF on the staged pipeline: 32-frame chunks, both passes per CTA.
-static rcabeam_status run_dmas_staged(das::Args a, size_t ntiles, cudaStream_t stream = 0) {
-  constexpr int kLpv = 16;
-  using S = das::Shape<kLpv, false>;
-  const size_t nt = size_t(a.nt);
-  const bool aligned = (nt * 8) % 16 == 0 && reinterpret_cast<uintptr_t>(a.rc) % 16 == 0 &&
-                       reinterpret_cast<uintptr_t>(a.cr) % 16 == 0 && encode_fn() != nullptr;
-  CUtensorMap mr{}, mq{};
-  const size_t slabs = size_t(a.nc) * a.na;
-  const bool tma = aligned && make_slab_map(&mr, a.rc, 8, nt, size_t(a.ns), slabs, S::kFrames, das::kRows) &&
-                   make_slab_map(&mq, a.cr, 8, nt, size_t(a.ns), slabs, S::kFrames, das::kRows);
-  const dim3 grid(unsigned(ntiles), unsigned((nt + S::kFrames - 1) / S::kFrames));
-  const size_t smem = S::bytes(a.na);
-  auto kern = tma ? das::dmas_staged<kLpv, true> : das::dmas_staged<kLpv, false>;
-  if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)) != cudaSuccess)
-    return RCABEAM_ERROR_CUDA;
-  kern<<<grid, das::kThreads, smem, stream>>>(mr, mq, a);
+  const rcabeam_status st = run_rows<das::kXdoppler, false>(a, stream);
+  if (st != RCABEAM_SUCCESS) return st;
+  das::finish_magnitude<<<unsigned((size_t(a.nv) + 255) / 256), 256, 0, stream>>>(a.pd, size_t(a.nv));
   return launch_status();
 }
 
@@ -438,12 +493,6 @@ static rcabeam_status ensemble_impl(const void* rc, const void* cr, const float*
   a.fd = double(fd);
   a.fn = double(fn);
   a.err = device_error_ptr();
-  if (method == 2) {
-    dim3 grid(unsigned((nv + generic::kWarps - 1) / generic::kWarps),
-              unsigned((nt + 32 * generic::kRegFrames - 1) / (32 * generic::kRegFrames)));
-    generic::ensemble_nonlinear<2><<<grid, generic::kWarps * 32>>>(a);
-    return launch_status();
-  }
   if (method == 4) {
     // St-SW: series into the caller's workspace (nv k^2 nt complex64), then
     // energies, pair sums, raw weights and the XDoppler magnitude.
@@ -465,8 +514,6 @@ static rcabeam_status ensemble_impl(const void* rc, const void* cr, const float*
   }
   // The caller owns 2 * nv * (nc + na) float4 of scratch (reference rcabeam.h:196).
   a.order = voxel_order(scan, nv, geometry_workspace, 2 * nv * (nc + na) * 16);
-  if (method == 3) return run_dmas_staged(a, (nv + das::kTileVoxels - 1) / das::kTileVoxels);
-  const size_t ntiles = (nv + das::kTileVoxels - 1) / das::kTileVoxels;
   const void* planes[2] = {rc, cr};
   if (HALF && tc_eligible(planes, 2, nt) && nv <= size_t(INT32_MAX) - tc::kVox && tc_smem_bytes(false, nt, na, 2)) {
     tc::Args t{};
@@ -492,19 +539,8 @@ static rcabeam_status ensemble_impl(const void* rc, const void* cr, const float*
     t.err = a.err;
     return run_tc<false>(t);
   }
-  rcabeam_status st;
-  if (method == 0)
-    st = run_staged<HALF, das::kOpw>(a, ntiles);
-  else if (method == 5)
-    st = run_staged<false, das::kApertures>(a, ntiles);
-  else
-    st = run_staged<false, das::kXdoppler>(a, ntiles);
-  if (st != RCABEAM_SUCCESS) return st;
-  if (method == 1) {
-    das::finish_magnitude<<<unsigned((nv + 255) / 256), 256>>>(pd, nv);
-    return launch_status();
-  }
-  return RCABEAM_SUCCESS;
+  if constexpr (HALF) return run_rows<das::kOpw, true>(a);
+  return run_method(a, method);
 }
 
 static generic::FrameArgs frame_args(const void* rc, const void* cr, const float* scan, const float* xe,
@@ -740,27 +776,11 @@ static rcabeam_status ensemble_static(const void* rc, const void* cr, const floa
   a.fd = double(fd);
   a.fn = double(fn);
   a.err = device_error_ptr();
-  if (method == 2) {
-    dim3 grid(unsigned((nv + generic::kWarps - 1) / generic::kWarps),
-              unsigned((nt + 32 * generic::kRegFrames - 1) / (32 * generic::kRegFrames)));
-    generic::ensemble_nonlinear<2><<<grid, generic::kWarps * 32>>>(a);
-    return launch_status();
-  }
   // The sort rewrites keys, values and the bounding box (cleared inside) on every call.
   // Calls too small to need an order run in identity order; a failed sort is an error.
   a.order = voxel_order(scan, nv, scratch, kStaticScratchBytes);
   if (!a.order && order_bytes(nv, nullptr)) return RCABEAM_ERROR_CUDA;
-  if (method == 3) return run_dmas_staged(a, (nv + das::kTileVoxels - 1) / das::kTileVoxels);
-  const size_t ntiles = (nv + das::kTileVoxels - 1) / das::kTileVoxels;
-  rcabeam_status st = method == 0   ? run_staged<false, das::kOpw>(a, ntiles)
-                      : method == 5 ? run_staged<false, das::kApertures>(a, ntiles)
-                                    : run_staged<false, das::kXdoppler>(a, ntiles);
-  if (st != RCABEAM_SUCCESS) return st;
-  if (method == 1) {
-    das::finish_magnitude<<<unsigned((nv + 255) / 256), 256>>>(pd, nv);
-    return launch_status();
-  }
-  return RCABEAM_SUCCESS;
+  return run_method(a, method);
 }
 
 }  // namespace rcb
@@ -1298,7 +1318,7 @@ rcabeam_status rcabeam_opw_offsets_power_device(const void* rc, const void* cr, 
   a.err = device_error_ptr();
   a.offsets = offsets;
   a.order = voxel_order(scan, nv, workspace, workspace_bytes);
-  return run_staged<false, das::kOpw>(a, (nv + das::kTileVoxels - 1) / das::kTileVoxels);
+  return run_rows<das::kOpw, false>(a);
 }
 
 rcabeam_status rcabeam_opw_offsets_adjoint_device(const void* rc, const void* cr, const float* scan,
@@ -1329,14 +1349,26 @@ rcabeam_status rcabeam_opw_offsets_adjoint_device(const void* rc, const void* cr
 // ---------------------------------------------------------- batch queue --
 namespace {
 struct BatchLayout {
-  size_t ens, maps, next, done, tile_done, total;
+  size_t ens, next, done, tile_done, total;
 };
 
+RowsPlan batch_item_plan(const das::Args& a, int method, int max_frames) {
+  // sms = 1: a queue fills the GPU, so its items need no extra split.
+  if (method == 3) return plan_rows<das::kDmas>(a, false, 1, max_frames);
+  return method == 1 ? plan_rows<das::kXdoppler>(a, false, 1, max_frames)
+                     : plan_rows<das::kOpw>(a, false, 1, max_frames);
+}
+
+// The table's ensembles and its layout; layout (of a persistent launch, smem 0
+// when the ensembles' items do not fit one) covers every ensemble's plan.
 bool batch_plan(size_t n, const rcabeam_batch_ensemble* list, std::vector<batch::Ensemble>* out, BatchLayout* L,
-                long long* total_items) {
+                long long* total_items, das::Layout* layout) {
   if (!n || !list || n > (1u << 20)) return false;
   long long items = 0, tiles_xd = 0;
   if (out) out->resize(n);
+  das::Layout lt{};
+  int consumers = 0, stash_unit = 0;
+  bool fits = true;
   for (size_t i = 0; i < n; ++i) {
     const rcabeam_batch_ensemble& d = list[i];
     if (!d.rc || !d.cr || !d.scan || !d.xe || !d.ye || !d.angles || !d.starts || !d.pd || d.ns < 2 || !d.nc ||
@@ -1348,26 +1380,6 @@ bool batch_plan(size_t n, const rcabeam_batch_ensemble* list, std::vector<batch:
     const int fpc = d.frames_per_chunk ? d.frames_per_chunk : 64;
     if (fpc != 16 && fpc != 32 && fpc != 64) return false;
     batch::Ensemble e{};
-    e.method = d.method;
-    e.lpv = fpc / 2;
-    if (d.method == 3) {
-      e.lpv = batch::kDmasLpv;
-      e.tiles = int((d.nv + das::kTileVoxels - 1) / das::kTileVoxels);
-      e.chunks = int((d.nt + 2 * batch::kDmasLpv - 1) / (2 * batch::kDmasLpv));
-    } else {
-      // Whole F-frame chunks, then one tail chunk of the next power of two >= 4 frames.
-      e.tiles = int((d.nv + das::kTileVoxels - 1) / das::kTileVoxels);
-      e.main_chunks = int(d.nt / fpc);
-      const unsigned tail = unsigned(d.nt % fpc);
-      e.lpv_tail = tail ? int(std::max(pow2_at_least(tail), 4u) / 2) : 0;
-      e.chunks = e.main_chunks + (tail ? 1 : 0);
-    }
-    e.tma = (d.nt * 8) % 16 == 0 && reinterpret_cast<uintptr_t>(d.rc) % 16 == 0 &&
-            reinterpret_cast<uintptr_t>(d.cr) % 16 == 0 && encode_fn() != nullptr;
-    e.first_item = items;
-    e.tile_base = tiles_xd;
-    items += (long long)e.tiles * e.chunks;
-    if (d.method == 1) tiles_xd += e.tiles;
     das::Args& a = e.args;
     a.rc = d.rc;
     a.cr = d.cr;
@@ -1388,32 +1400,60 @@ bool batch_plan(size_t n, const rcabeam_batch_ensemble* list, std::vector<batch:
     a.fs = d.fs;
     a.fd = d.fd;
     a.fn = d.fn;
-    a.frame_base = 0;
     a.err = device_error_ptr();
+    // 64: the planned split; 16 or 32: items of at most that many frames.
+    const RowsPlan r = batch_item_plan(a, d.method, fpc == 64 ? INT32_MAX : fpc);
+    fits = fits && r.layout.smem && (i == 0 || r.layout.builders == lt.builders);
+    e.method = d.method;
+    e.shape = r.shape;
+    e.maps = r.maps;
+    e.width = r.width;
+    e.tiles = int((d.nv + das::kTileVoxels - 1) / das::kTileVoxels);
+    e.first_item = items;
+    e.tile_base = tiles_xd;
+    items += (long long)e.tiles * e.shape.chunks;
+    if (d.method == 1) tiles_xd += e.tiles;
+    const int warps = r.layout.threads / 32 - r.layout.builders;
+    consumers = std::max(consumers, warps);
+    stash_unit = std::max(stash_unit, r.layout.stash_bytes / (32 * warps));
+    lt.builders = r.layout.builders;
+    lt.stage_bytes = std::max(lt.stage_bytes, r.layout.stage_bytes);
+    lt.zero_bytes = std::max(lt.zero_bytes, r.layout.zero_bytes);
+    lt.angles = std::max(lt.angles, r.layout.angles);
+    lt.table_bytes = std::max(lt.table_bytes, r.layout.table_bytes);
     if (out) (*out)[i] = e;
   }
   L->ens = 0;
-  L->maps = align256(n * sizeof(batch::Ensemble));
-  L->next = L->maps + align256(4 * n * sizeof(CUtensorMap));
+  L->next = L->ens + align256(n * sizeof(batch::Ensemble));
   L->done = L->next + 256;
   L->tile_done = L->done + align256(n * 4);
   L->total = L->tile_done + align256(size_t(tiles_xd > 0 ? tiles_xd : 1) * 4);
   *total_items = items;
+  if (layout) {
+    // A launch's ring stages are the largest any ensemble plans for itself.
+    lt.threads = 32 * (lt.builders + consumers);
+    lt.stages = 2 * lt.builders;
+    lt.stash_bytes = stash_unit * 32 * consumers;
+    lt.smem = das::kFixedBytes + 24 * lt.angles + lt.zero_bytes + lt.stash_bytes + lt.table_bytes +
+              lt.stages * lt.stage_bytes;
+    if (!fits || lt.smem > 227 * 1024) lt.smem = 0;
+    *layout = lt;
+  }
   return true;
 }
 
-batch::Queue batch_queue(void* table, size_t n, const BatchLayout& L, long long total, unsigned long long* times) {
+batch::Queue batch_queue(void* table, size_t n, const BatchLayout& L, long long total, const das::Layout& layout,
+                         unsigned long long* times) {
   unsigned char* t = static_cast<unsigned char*>(table);
   batch::Queue q{};
   q.ens = reinterpret_cast<const batch::Ensemble*>(t + L.ens);
-  q.maps = reinterpret_cast<const CUtensorMap*>(t + L.maps);
+  q.layout = layout;
   q.n = int(n);
   q.total_items = total;
   q.next = reinterpret_cast<unsigned long long*>(t + L.next);
   q.done = reinterpret_cast<unsigned*>(t + L.done);
   q.tile_done = reinterpret_cast<unsigned*>(t + L.tile_done);
   q.times = times;
-  q.err = device_error_ptr();
   return q;
 }
 }  // namespace
@@ -1423,7 +1463,7 @@ extern "C" {
 rcabeam_status rcabeam_batch_table_bytes(size_t n, const rcabeam_batch_ensemble* list, size_t* bytes) {
   BatchLayout L;
   long long total = 0;
-  if (!bytes || !batch_plan(n, list, nullptr, &L, &total)) return RCABEAM_ERROR_ARGUMENT;
+  if (!bytes || !batch_plan(n, list, nullptr, &L, &total, nullptr)) return RCABEAM_ERROR_ARGUMENT;
   *bytes = L.total;
   return RCABEAM_SUCCESS;
 }
@@ -1433,27 +1473,13 @@ rcabeam_status rcabeam_batch_prepare(size_t n, const rcabeam_batch_ensemble* lis
   BatchLayout L;
   long long total = 0;
   std::vector<batch::Ensemble> ens;
-  if (!table || reinterpret_cast<uintptr_t>(table) % 256 != 0 || !batch_plan(n, list, &ens, &L, &total) ||
-      table_bytes < L.total)
+  if (!table || reinterpret_cast<uintptr_t>(table) % 256 != 0 ||
+      !batch_plan(n, list, &ens, &L, &total, nullptr) || table_bytes < L.total)
     return RCABEAM_ERROR_ARGUMENT;
-  std::vector<CUtensorMap> maps(4 * n);
-  for (size_t i = 0; i < n; ++i) {
-    batch::Ensemble& e = ens[i];
-    if (!e.tma) continue;
-    const size_t slabs = size_t(e.args.nc) * e.args.na, nt = size_t(e.args.nt), ns = size_t(e.args.ns);
-    for (int part = 0; part < 2; ++part) {
-      const int frames = 2 * (part ? e.lpv_tail : e.lpv);
-      if (!frames) continue;
-      if (!make_slab_map(&maps[4 * i + 2 * part], e.args.rc, 8, nt, ns, slabs, frames, das::kRows) ||
-          !make_slab_map(&maps[4 * i + 2 * part + 1], e.args.cr, 8, nt, ns, slabs, frames, das::kRows))
-        return RCABEAM_ERROR_ARGUMENT;  // the run's kernel variant follows the plan's tma flags
-    }
-  }
-  unsigned char* t = static_cast<unsigned char*>(table);
-  if (cudaMemcpy(t + L.ens, ens.data(), n * sizeof(batch::Ensemble), cudaMemcpyHostToDevice) != cudaSuccess ||
-      cudaMemcpy(t + L.maps, maps.data(), 4 * n * sizeof(CUtensorMap), cudaMemcpyHostToDevice) != cudaSuccess)
-    return RCABEAM_ERROR_CUDA;
-  return RCABEAM_SUCCESS;
+  return cudaMemcpy(static_cast<unsigned char*>(table) + L.ens, ens.data(), n * sizeof(batch::Ensemble),
+                    cudaMemcpyHostToDevice) == cudaSuccess
+             ? RCABEAM_SUCCESS
+             : RCABEAM_ERROR_CUDA;
 }
 
 rcabeam_status rcabeam_batch_run_device(size_t n, const rcabeam_batch_ensemble* list, void* table,
@@ -1461,7 +1487,9 @@ rcabeam_status rcabeam_batch_run_device(size_t n, const rcabeam_batch_ensemble* 
                                         void* stream) {
   BatchLayout L;
   long long total = 0;
-  if (!table || !times || ctas_per_sm < 0 || ctas_per_sm > 3 || !batch_plan(n, list, nullptr, &L, &total) ||
+  das::Layout layout{};
+  std::vector<batch::Ensemble> ens;
+  if (!table || !times || ctas_per_sm < 0 || ctas_per_sm > 3 || !batch_plan(n, list, &ens, &L, &total, &layout) ||
       table_bytes < L.total)
     return RCABEAM_ERROR_ARGUMENT;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
@@ -1472,57 +1500,32 @@ rcabeam_status rcabeam_batch_run_device(size_t n, const rcabeam_batch_ensemble* 
     return RCABEAM_ERROR_CUDA;
   for (size_t i = 0; i < n; ++i)
     if (cudaMemsetAsync(list[i].pd, 0, 2 * list[i].nv * sizeof(float), st) != cudaSuccess) return RCABEAM_ERROR_CUDA;
-  int dev = 0, sms = 148;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  std::vector<batch::Ensemble> ens;
-  batch_plan(n, list, &ens, &L, &total);
-  if (ctas_per_sm == 0) {
-    // Grid mode: each ensemble through the single-ensemble kernels on the
-    // stream (for ensembles that fill the GPU alone, where those kernels run
-    // faster than the persistent loop), a completion stamp after each.
+  bool one_method = true;
+  for (size_t i = 1; i < n; ++i) one_method = one_method && list[i].method == list[0].method;
+  if (ctas_per_sm == 0 || !one_method || !layout.smem) {
+    // Each ensemble through the single-ensemble kernels on the stream, a
+    // completion stamp after each.
     batch::stamp<<<1, 1, 0, st>>>(times, 1);
     for (size_t i = 0; i < n; ++i) {
-      const das::Args& a = ens[i].args;
-      const size_t ntiles = (size_t(a.nv) + das::kTileVoxels - 1) / das::kTileVoxels;
-      rcabeam_status r = RCABEAM_SUCCESS;
-      if (list[i].method == 3) {
-        r = run_dmas_staged(a, ntiles, st);
-      } else if (list[i].method == 1) {
-        r = run_staged<false, das::kXdoppler>(a, ntiles, st);
-        if (r == RCABEAM_SUCCESS) das::finish_magnitude<<<unsigned((a.nv + 255) / 256), 256, 0, st>>>(a.pd, a.nv);
-      } else {
-        r = run_staged<false, das::kOpw>(a, ntiles, st);
-      }
+      const rcabeam_status r = run_method(ens[i].args, list[i].method, st);
       if (r != RCABEAM_SUCCESS) return r;
       batch::stamp<<<1, 1, 0, st>>>(times + 1 + i, 0);
     }
-    return cudaGetLastError() == cudaSuccess ? RCABEAM_SUCCESS : RCABEAM_ERROR_CUDA;
-  }
-  // A queue of one method whose ensembles all stage the same way (TMA or plain
-  // loads) at two or three CTAs per SM runs the kernel compiled for that
-  // method and staging alone; anything else runs the general kernel.
-  int kind = list[0].method, tma = ens[0].tma;
-  for (size_t i = 1; i < n; ++i) {
-    if (list[i].method != kind) kind = -1;
-    if (ens[i].tma != tma) tma = -1;
+    return launch_status();
   }
   using Kernel = void (*)(const batch::Queue);
-  static const Kernel general[3] = {batch::run<1, -1, -1>, batch::run<2, -1, -1>, batch::run<3, -1, -1>};
-  static const Kernel special[3][2][2] = {  // [kind][tma][ctas_per_sm - 2]
-      {{batch::run<2, 0, 0>, batch::run<3, 0, 0>}, {batch::run<2, 0, 1>, batch::run<3, 0, 1>}},
-      {{batch::run<2, 1, 0>, batch::run<3, 1, 0>}, {batch::run<2, 1, 1>, batch::run<3, 1, 1>}},
-      {{batch::run<2, 3, 0>, batch::run<3, 3, 0>}, {batch::run<2, 3, 1>, batch::run<3, 3, 1>}},
-  };
-  const bool specific = kind >= 0 && tma >= 0 && ctas_per_sm >= 2;
-  const Kernel kern = specific ? special[kind == 3 ? 2 : kind][tma][ctas_per_sm - 2] : general[ctas_per_sm - 1];
-  const size_t smem = specific && kind == 3 ? batch::Smem<batch::smem_lpv<3>()>::kBytes : batch::Smem<32>::kBytes;
-  if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)) != cudaSuccess)
+  const Kernel kern = list[0].method == 3   ? batch::run<das::kDmas>
+                      : list[0].method == 1 ? batch::run<das::kXdoppler>
+                                            : batch::run<das::kOpw>;
+  if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, layout.smem) != cudaSuccess)
     return RCABEAM_ERROR_CUDA;
-  const long long want = (long long)sms * ctas_per_sm;
-  const unsigned grid = unsigned(total < want ? total : want);
-  kern<<<grid, das::kThreads, smem, st>>>(batch_queue(table, n, L, total, times));
-  return cudaGetLastError() == cudaSuccess ? RCABEAM_SUCCESS : RCABEAM_ERROR_CUDA;
+  int resident = 1;
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, kern, layout.threads, layout.smem) != cudaSuccess)
+    return RCABEAM_ERROR_CUDA;
+  const long long want = (long long)sm_count() * std::max(1, std::min(resident, ctas_per_sm));
+  kern<<<unsigned(std::min(total, want)), layout.threads, layout.smem, st>>>(
+      batch_queue(table, n, L, total, layout, times));
+  return launch_status();
 }
 
 rcabeam_status rcabeam_simulate_scene_device(const float* scatterers, size_t n, const float* elements,

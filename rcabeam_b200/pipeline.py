@@ -306,13 +306,11 @@ class FilteredOpw:
 
     def launches_per_step(self) -> int:
         """Kernels of this library launched per ``run``: pack x2, voxel order (bounding box,
-        Morton codes, 4 radix-sort passes), DAS (one persistent tensor-core launch, or main +
-        tail staged launches), scale, Gram, Gram finish, projection (channel domain: per
-        aperture scale, Gram and projection)."""
-        das = 1 if self.storage != "float32" and self.channel_shape[3] % 4 == 0 else 2
+        Morton codes, 4 radix-sort passes), DAS, scale, Gram, Gram finish, projection (channel
+        domain: per aperture scale, Gram and projection)."""
         if self.domain == "channel":  # scale x2, Gram x2, finish, projection x2, pack x2, order, DAS
-            return 5 + 2 + 2 + 6 + das
-        return 2 + 6 + das + 4 + (1 if self.refine else 0)
+            return 5 + 2 + 2 + 6 + 1
+        return 2 + 6 + 1 + 4 + (1 if self.refine else 0)
 
 
 def synthetic_channels(shape, *, generator: torch.Generator, device, scale: float = 1.0):

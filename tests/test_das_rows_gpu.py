@@ -1,0 +1,98 @@
+"""Edges of the staged delay-and-sum kernel against the float64 oracle: item and
+thread splits of the frames, odd frame counts and unaligned buffers (bulk copies),
+windows longer than a ring stage, tiles that fall apart, many angles, apertures
+no voxel of a tile reaches.  Bars as in test_das_gpu.py (IQ 1e-5, products of
+sums 1e-4)."""
+
+from __future__ import annotations
+
+import numpy as np
+import pytest
+import torch
+
+from oracle import methods
+from rcabeam_b200 import _cuda_impl, _lib
+from tests._cases import rel_l2
+
+pytestmark = pytest.mark.gpu
+FS, FD, C = 20e6, 5e6, 1540.0
+
+
+@pytest.fixture(autouse=True)
+def _cuda():
+    if not torch.cuda.is_available():
+        pytest.skip("needs CUDA")
+    yield
+    assert _lib.device_error() == 0
+
+
+def _voxels(kind: str, nv: int, rng) -> np.ndarray:
+    """Positions (x, z, y): within a few sample rows, over the whole window, or in two distant clusters."""
+    span = {"dense": 0.2e-3, "coarse": 5e-3, "apart": 0.2e-3}[kind]
+    scan = rng.uniform([-1e-3, 3e-3, -1e-3], [1e-3, 3e-3 + span, 1e-3], (nv, 3))
+    if kind == "dense":
+        scan[:, ::2] *= 0.1
+    if kind == "apart":
+        scan[nv // 2:, 1] += 5e-3
+    return scan.astype(np.float32)
+
+
+def _reconstruct(rc, cr, scan, xe, ye, angles, starts, fn, method, shift):
+    ns, nc, na, nt = rc.shape
+    dev = lambda a: torch.from_numpy(np.ascontiguousarray(a)).cuda()  # noqa: E731
+    packed = []
+    for src in (rc, cr):  # packed (c, a, s, t), `shift` samples past a 16-byte boundary
+        buf = torch.zeros(rc.size + 2, dtype=torch.complex64, device="cuda")
+        dst = buf[shift:shift + rc.size]
+        dst.copy_(dev(src.transpose(1, 2, 0, 3)).reshape(-1))
+        packed.append(dst)
+    nv = len(scan)
+    pd = torch.empty((nv, 2), dtype=torch.float32, device="cuda")
+    planes = 2 if method == 5 else 1
+    signal = torch.full((nv * planes, nt), float("nan"), dtype=torch.complex64, device="cuda")
+    work = torch.empty(_cuda_impl.workspace_bytes(nv, nc, na), dtype=torch.uint8, device="cuda")
+    t = [dev(a) for a in (scan, xe, ye, angles, starts)]
+    _lib.call("rcabeam_ensemble_device", packed[0].data_ptr(), packed[1].data_ptr(), *(a.data_ptr() for a in t),
+              pd.data_ptr(), signal.data_ptr(), None, None, work.data_ptr(), ns, nc, na, nt, nv, C, FS, FD,
+              -1.0 if fn is None else fn, method, 2)
+    return pd[:, 0].cpu().numpy(), signal.cpu().numpy().reshape(nv, planes, nt)
+
+
+@pytest.mark.parametrize("frames,kind,nv,na,fn,shift", [
+    (1, "dense", 127, 3, None, 0), (16, "coarse", 129, 5, None, 0), (17, "coarse", 300, 5, 1.0, 1),
+    (26, "dense", 128, 4, 1.0, 1), (33, "apart", 257, 3, None, 0), (48, "coarse", 130, 2, 1.0, 0),
+    (49, "dense", 150, 3, None, 1), (64, "apart", 200, 3, None, 0), (65, "dense", 129, 3, 1.0, 0),
+    (104, "coarse", 140, 2, None, 0), (105, "coarse", 131, 2, 1.0, 1), (106, "dense", 129, 3, None, 0),
+    (209, "apart", 130, 2, None, 0), (6, "coarse", 140, 180, None, 0),
+])
+def test_staged_splits_match_oracle(frames, kind, nv, na, fn, shift):
+    rng = np.random.default_rng(frames + nv)
+    ns, nc = 200, 7
+    f64 = lambda a: np.asarray(a, np.float32).astype(np.float64)  # noqa: E731
+    scan = _voxels(kind, nv, rng)
+    xe = np.linspace(-4e-3, 4e-3, nc).astype(np.float32)
+    ye = np.linspace(-3.9e-3, 4.1e-3, nc).astype(np.float32)
+    angles = np.linspace(-0.17, 0.16, na).astype(np.float32)
+    starts = np.full(na, 2 * 3e-3 / C - 0.4e-6, np.float32)
+    shape = (ns, nc, na, frames)
+    rc, cr = ((rng.normal(size=shape) + 1j * rng.normal(size=shape)).astype(np.complex64) for _ in range(2))
+    geom = (f64(scan), f64(xe), f64(ye), f64(angles), f64(starts), C, FS, FD, fn)
+    chan_r, ang_r, n_r = methods.aperture_terms(rc, geom[0], geom[1], *geom[3:], "RC")
+    chan_q, ang_q, n_q = methods.aperture_terms(cr, geom[0], geom[2], *geom[3:], "CR")
+    r, q = ang_r.sum(axis=1), ang_q.sum(axis=1)
+    run = lambda method: _reconstruct(rc, cr, scan, xe, ye, angles, starts, fn, method, shift)  # noqa: E731
+    pd, iq = run(0)
+    assert rel_l2(iq[:, 0], r + q) <= 1e-5
+    assert rel_l2(pd, np.mean(np.abs(r + q) ** 2, axis=-1)) <= 1e-5
+    _, iq = run(5)
+    assert rel_l2(iq, np.stack((r, q), axis=1)) <= 1e-5
+    if na > 8:
+        return
+    pd, _ = run(1)
+    assert rel_l2(pd, np.abs(np.mean(r * q.conj(), axis=-1))) <= 1e-4
+    fmas = methods.signed_sqrt(ang_r).sum(axis=1) * methods.signed_sqrt(ang_q).sum(axis=1)
+    pd, signal = run(2)
+    assert rel_l2(signal[:, 0], fmas) <= 1e-4
+    assert rel_l2(pd, np.mean(np.abs(fmas) ** 2, axis=-1)) <= 1e-4
+    pd, _ = run(3)
+    assert rel_l2(pd, methods.dmas_ccf_acf_power(rc, cr, *geom)) <= 1e-4
