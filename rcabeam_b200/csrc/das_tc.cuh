@@ -32,10 +32,12 @@
 // registers at six stages still fit the register file):
 //   warps 0..S-1  builders, one per ring stage.  A warp owns whole steps:
 //               channels are dealt round robin to the warps, so each warp
-//               forms the float64 receive delay and phase of its channel once
+//               forms the receive delay and phase of its channel once
 //               for the 128 voxels (four per lane) and then, per angle, the
-//               taps (sample index, weight, phase by angle addition with a
-//               per-tile table of transmit delays and phases), the tile's row
+//               taps (sample position as a fixed-point sum and phase by angle
+//               addition with a per-tile table of transmit delays and phases;
+//               in float64 throughout, and with rows placed by 16 selects a
+//               word, the full-size launch took 2.4 % longer), the tile's row
 //               window (warp reductions) and the hi / lo coefficient pairs;
 //               then claims the next ring stage from a shared counter, issues
 //               the window's TMA copies (64-column x 16-row SWIZZLE_128B boxes,
@@ -120,6 +122,11 @@ struct Args {
   int* err;
 };
 
+// A voxel's transmit delay lies within 2^27 samples of its tile's first voxel's (or
+// it is left out), and three terms below 2^61 cannot bring kNever back.
+constexpr float kReachLimit = 134217728.f;
+constexpr long long kNever = -(3ll << 61);
+
 constexpr int kCtrlBytes = 512;  // barriers, stage tags, counters, TMEM slot
 
 template <bool BF16X3>
@@ -130,7 +137,7 @@ struct Layout {
     return 4 * kAMatBytes + size_t(kPlanes) * nbox * kBoxBytes;
   }
   // stages | control (barriers, meta, counters, TMEM slot) | angle table [na][3] double |
-  // per-tile transmit delay bases [2][na] double, offsets [2][na][128] float and
+  // per-tile transmit delay bases [2][na] and offsets [2][na][128] int, and
   // phases [2][na][128] float2 (the caller adds up to 1 KB to align the base).
   static size_t bytes(int nbox, int na, int stages) {
     return size_t(stages) * stage_bytes(nbox) + kCtrlBytes + size_t(na) * 5 * sizeof(double) +
@@ -250,42 +257,44 @@ __device__ __forceinline__ void split_pair(float c0, float c1, uint32_t& hi, uin
   }
 }
 
-// The eight 32-bit words of a 16-column row whose only nonzero entries are the
-// packed pair v at columns r, r + 1 (r = -1: an all-zero row).
+// Where a row of 16 columns (two 16-byte K cores) holds the packed pair of columns
+// r, r + 1 (r = -1: nowhere).  The core with column r is written from its four
+// words, the other core as zeros, with the pair's second half in its first word
+// when the pair straddles the cores (r = 7).
 struct RowPlace {
-  int word;   // word holding column r (-2 when the row is empty)
-  int shift;  // 0 or 16: bit offset of column r in that word
-  __device__ __forceinline__ explicit RowPlace(int r) : word(r >= 0 ? r >> 1 : -2), shift((r & 1) << 4) {}
-  __device__ __forceinline__ uint32_t at(int i, uint32_t v) const {
+  uint32_t core;      // byte offset of the core of column r: 0 or 128
+  int shift;          // 0 or 16: bit offset of column r in its word
+  bool at[4];         // word of the core that holds column r
+  bool straddle;
+  __device__ __forceinline__ explicit RowPlace(int r) : core((r & 8) << 4), shift((r & 1) << 4), straddle(r == 7) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) at[i] = r >= 0 && ((r & 7) >> 1) == i;
+    if (r < 0) core = 0;
+  }
+  // Writes both cores of the row at `row`.
+  __device__ __forceinline__ void put(unsigned char* row, uint32_t v) const {
     const uint32_t first = v << shift;                      // column r (and r + 1 when r is even)
     const uint32_t second = __funnelshift_l(v, 0u, shift);  // column r + 1 when r is odd
-    return i == word ? first : (i == word + 1 ? second : 0u);
+    uint4 w;
+    w.x = at[0] ? first : 0u;
+    w.y = at[1] ? first : (at[0] ? second : 0u);
+    w.z = at[2] ? first : (at[1] ? second : 0u);
+    w.w = at[3] ? first : (at[2] ? second : 0u);
+    *reinterpret_cast<uint4*>(row + core) = w;
+    *reinterpret_cast<uint4*>(row + (core ^ 128u)) = make_uint4(straddle ? second : 0u, 0u, 0u, 0u);
   }
 };
 
 // Writes the real (row m, m even) and imaginary (row m + 1) A rows of one voxel
-// into a K-major no-swizzle 128 x 16 matrix: four 16-byte stores, (row, K core)
-// pieces at offsets +0 / +16 / +128 / +144.  Lanes whose 8-row group is odd
-// swap the row order of each store pair, so that every store instruction of
-// the warp spreads over all 32 banks (four wavefronts for 512 bytes).
+// into a K-major no-swizzle 128 x 16 matrix.  Lanes whose 8-row group is odd
+// write the two rows in the other order, so that every store instruction of the
+// warp spreads over all 32 banks (four wavefronts for 512 bytes; the cores lie a
+// whole 128 bytes apart).
 __device__ __forceinline__ void put_rows(unsigned char* a, int m, const RowPlace& pl, uint32_t re, uint32_t im) {
   const bool odd = (m >> 3) & 1;
-  const uint32_t base = uint32_t((m >> 3) * 256 + (m & 7) * 16);
-#pragma unroll
-  for (int kc = 0; kc < 2; ++kc) {
-    uint4 pr, pi;
-    pr.x = pl.at(4 * kc + 0, re);
-    pr.y = pl.at(4 * kc + 1, re);
-    pr.z = pl.at(4 * kc + 2, re);
-    pr.w = pl.at(4 * kc + 3, re);
-    pi.x = pl.at(4 * kc + 0, im);
-    pi.y = pl.at(4 * kc + 1, im);
-    pi.z = pl.at(4 * kc + 2, im);
-    pi.w = pl.at(4 * kc + 3, im);
-    const uint32_t o = base + 128u * kc;
-    *reinterpret_cast<uint4*>(a + o + (odd ? 16u : 0u)) = odd ? pi : pr;
-    *reinterpret_cast<uint4*>(a + o + (odd ? 0u : 16u)) = odd ? pr : pi;
-  }
+  unsigned char* row = a + uint32_t((m >> 3) * 256 + (m & 7) * 16);
+  pl.put(row + (odd ? 16 : 0), odd ? im : re);
+  pl.put(row + (odd ? 0 : 16), odd ? re : im);
 }
 
 // mbarrier.expect_tx without an arrival: the writing warp's 32 lanes arrive
@@ -320,9 +329,9 @@ __device__ __forceinline__ int item_pass(const Args& p, int item) {
   return (chunk + item / int(gridDim.x)) % p.chunks;
 }
 
-// exp(+j 2 pi fd tau) with the cycle count reduced in float64.
-__device__ __forceinline__ float2 demod_phase(double fd, double tau) {
-  double cyc = fd * tau;
+// exp(+j 2 pi kc path) with the cycle count reduced in float64.
+__device__ __forceinline__ float2 demod_phase(double kc, double path) {
+  double cyc = kc * path;
   cyc -= rint(cyc);
   float sn, cs;
   sincospif(2.0f * float(cyc), &sn, &cs);
@@ -362,12 +371,11 @@ __global__ void __launch_bounds__(threads_for(STAGES), 1)
   volatile int* acc_item = item_steps + 4;               // work item of the pending flush
   int* meta_item = item_steps + 5;                       // [STAGES]: work item of each staged slot
   double* angle_tab = reinterpret_cast<double*>(ctrl + kCtrlBytes);
-  // Transmit delay of (aperture, angle, voxel) = tx_base[aperture, angle] (the
-  // tile's first voxel, float64) + tx_off (float: within a compact tile the
-  // offsets stay below a few hundred ns, so float keeps them to ~1e-14 s); the
-  // halved table is what lets a sixth ring stage fit beside 3xBF16 stages.
-  double* tx_base = angle_tab + 3 * p.na;                                  // [2][na]
-  float* tx_off = reinterpret_cast<float*>(tx_base + 2 * p.na);            // [2][na][128]
+  // Transmit delay (minus the angle's start) of (aperture, angle, voxel), in
+  // 2^-32 samples = tx_base[aperture, angle] (the tile's first voxel) + tx_off
+  // times the tile's unit (2^-22 samples in a compact tile).
+  long long* tx_base = reinterpret_cast<long long*>(angle_tab + 3 * p.na);  // [2][na]
+  int* tx_off = reinterpret_cast<int*>(tx_base + 2 * p.na);                 // [2][na][128]
   float2* tx_phase = reinterpret_cast<float2*>(tx_off + 2 * p.na * kVox);  // [2][na][128]
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -414,6 +422,8 @@ __global__ void __launch_bounds__(threads_for(STAGES), 1)
     int nbox = p.nbox;  // boxes per plane of the current item's pass
     uint32_t tx_bytes = uint32_t(kPlanes * nbox * kBoxBytes);
     const float sc = kCoefScale<BF16X3>;
+    const double ks = p.fs / p.c, kc = p.fd / p.c;  // samples and demodulation cycles per metre
+    const unsigned inner = unsigned(max(p.ns - 3, 0));
     auto builders_sync = [] { asm volatile("bar.sync 1, %0;" ::"n"(kBuilders * 32) : "memory"); };
     // Claims the next ring stage (uniform in the warp) and waits until it is free.
     auto claim = [&](uint32_t& k) -> bool {
@@ -470,38 +480,44 @@ __global__ void __launch_bounds__(threads_for(STAGES), 1)
       const int col0 = 2 * chunk * p.frames;
       nbox = pass_boxes(pass_frames(p, chunk));
       tx_bytes = uint32_t(kPlanes * nbox * kBoxBytes);
+      // The tile's first slot always holds a voxel (tiles are filled in order).
+      const size_t q0 = size_t(tile) * kVox;
+      const size_t r3 = 3 * size_t(p.order ? p.order[q0] : unsigned(q0));
+      const double x0 = double(p.scan[r3]), z0 = double(p.scan[r3 + 1]), y0 = double(p.scan[r3 + 2]);
       // Voxels of this lane: slots lane + 32 j (group = slot / 64).
       double px[4], pz[4], py[4];
       bool pv[4];
+      float reach = 0.f;  // samples by which a transmit delay can differ from the first voxel's
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
         const size_t q = size_t(tile) * kVox + lane + 32 * j;
         const unsigned v = q < size_t(p.nv) ? (p.order ? p.order[q] : unsigned(q)) : UINT_MAX;
         pv[j] = v != UINT_MAX;
-        const size_t b3 = pv[j] ? 3 * size_t(v) : 0;
-        px[j] = pv[j] ? double(p.scan[b3]) : 0.0;
-        pz[j] = pv[j] ? double(p.scan[b3 + 1]) : 0.0;
-        py[j] = pv[j] ? double(p.scan[b3 + 2]) : 0.0;
+        const size_t b3 = pv[j] ? 3 * size_t(v) : r3;
+        px[j] = double(p.scan[b3]);
+        pz[j] = double(p.scan[b3 + 1]);
+        py[j] = double(p.scan[b3 + 2]);
+        const float far = float((fabs(pz[j] - z0) + fmax(fabs(px[j] - x0), fabs(py[j] - y0))) * ks);
+        pv[j] = pv[j] && far < kReachLimit;
+        if (far < kReachLimit) reach = fmaxf(reach, far);
       }
+      // Offsets in units of 2^-bits samples: the finest that holds the tile, 2^-22 at most.
+      reach = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(reach)));
+      const int bits = min(22, 29 - ilogbf(reach + 1.f));
+      const int unit = 1 << (32 - bits);
       // Per-tile transmit table, filled cooperatively by the builder warps.
       builders_sync();  // previous item's table reads are complete
-      // The tile's first slot always holds a voxel (tiles are filled in order).
-      const size_t q0 = size_t(tile) * kVox;
-      const size_t r3 = 3 * size_t(p.order ? p.order[q0] : unsigned(q0));
-      const double x0 = double(p.scan[r3]), z0 = double(p.scan[r3 + 1]), y0 = double(p.scan[r3 + 2]);
       for (int e = warp * 32 + lane; e < 2 * p.na * kVox; e += kBuilders * 32) {
         const int v = e % kVox, ca = e / kVox, config = ca / p.na, a = ca % p.na;
         const size_t q = size_t(tile) * kVox + v;
         const unsigned vid = q < size_t(p.nv) ? (p.order ? p.order[q] : unsigned(q)) : UINT_MAX;
-        const size_t b3 = vid != UINT_MAX ? 3 * size_t(vid) : 0;
-        const double x = vid != UINT_MAX ? double(p.scan[b3]) : 0.0;
-        const double z = vid != UINT_MAX ? double(p.scan[b3 + 1]) : 0.0;
-        const double y = vid != UINT_MAX ? double(p.scan[b3 + 2]) : 0.0;
-        const double ttx = transmit_delay(config ? x : y, z, angle_tab[3 * a], angle_tab[3 * a + 1], p.c);
-        const double ref = transmit_delay(config ? x0 : y0, z0, angle_tab[3 * a], angle_tab[3 * a + 1], p.c);
-        tx_off[e] = float(ttx - ref);
-        if (v == 0) tx_base[ca] = ref;
-        tx_phase[e] = demod_phase(p.fd, ttx);
+        const size_t b3 = vid != UINT_MAX ? 3 * size_t(vid) : r3;
+        const double x = double(p.scan[b3]), z = double(p.scan[b3 + 1]), y = double(p.scan[b3 + 2]);
+        const double ref = fma(z0, angle_tab[3 * a], (config ? x0 : y0) * angle_tab[3 * a + 1]);
+        const double path = fma(z, angle_tab[3 * a], (config ? x : y) * angle_tab[3 * a + 1]);
+        tx_off[e] = __double2int_rn((path - ref) * ks * double(1 << bits));
+        if (v == 0) tx_base[ca] = das::fixed32(fma(ref, ks, -angle_tab[3 * a + 2] * p.fs));
+        tx_phase[e] = demod_phase(kc, path);
       }
       // Channel slots u = aperture * nc + channel are walked from the slot the
       // other CTAs are at (the global slot count over the grid size): static
@@ -519,30 +535,48 @@ __global__ void __launch_bounds__(threads_for(STAGES), 1)
         const int config = u / p.nc, ch = u - config * p.nc;
         const float* el = config ? p.ye : p.xe;
         {  // this channel's receive delays, then its angles' steps
-          double trx[4];
+          long long rx[4];
           float2 ph_rx[4];
-          bool act[4];
+          const double e = double(el[ch]);
 #pragma unroll
           for (int j = 0; j < 4; ++j) {
-            trx[j] = receive_delay(config ? py[j] : px[j], pz[j], double(el[ch]), p.c, p.fn, &act[j]);
-            act[j] = act[j] && pv[j];
-            ph_rx[j] = demod_phase(p.fd, trx[j]);
+            const double d = __dadd_rn(config ? py[j] : px[j], -e);
+            const double r = das::path_root(fma(d, d, pz[j] * pz[j]));
+            const bool act = pv[j] && (p.fn <= 0.0 || fabs(d) <= __ddiv_rn(pz[j], __dmul_rn(2.0, p.fn)));
+            rx[j] = act ? das::fixed32(r * ks) : kNever;
+            ph_rx[j] = demod_phase(kc, r);
           }
           for (int a = 0; a < p.na; ++a) {
-            const double start = angle_tab[3 * a + 2];
-            const double base_tx = tx_base[config * p.na + a];
+            const long long base_tx = tx_base[config * p.na + a];
             int i0[4];
             float w[4];
             int lo = INT_MAX, hi = -1;
+            unsigned edges = 0;
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
               const int ti = (config * p.na + a) * kVox + lane + 32 * j;
-              const double ttx = __dadd_rn(base_tx, double(tx_off[ti]));
-              const double sample = __dmul_rn(__dadd_rn(__dadd_rn(ttx, trx[j]), -start), p.fs);
-              const bool in_window = act[j] && sample >= 0.0 && sample <= double(p.ns - 1);
-              const double fl = floor(sample);
-              i0[j] = in_window ? int(fl) : -1;
-              w[j] = float(sample - fl);
+              const long long at = rx[j] + base_tx + (long long)(tx_off[ti]) * unit;
+              i0[j] = int(at >> 32);
+              w[j] = float(unsigned(at)) * 0x1p-32f;
+              // Rows 1 ... ns - 3 are inside; the window's ends are decided in float64.
+              if (unsigned(i0[j] - 1) >= inner) {
+                if (at < (-1ll << 32) || at >= (long long)(p.ns) << 32) i0[j] = -1;
+                else edges |= 1u << j;
+              }
+            }
+            if (__any_sync(0xffffffffu, edges != 0)) {
+#pragma unroll
+              for (int j = 0; j < 4; ++j) {
+                if (!(edges >> j & 1)) continue;
+                float edge_w = 0.f;
+                i0[j] = das::edge_tap(config ? py[j] : px[j], config ? px[j] : py[j], pz[j], e, 0.0,
+                                      angle_tab[3 * a], angle_tab[3 * a + 1], angle_tab[3 * a + 2], p.c, p.fs, p.ns,
+                                      &edge_w);
+                w[j] = edge_w;
+              }
+            }
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
               if (i0[j] >= 0) {
                 lo = min(lo, i0[j]);
                 hi = max(hi, i0[j]);
