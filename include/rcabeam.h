@@ -214,8 +214,9 @@ rcabeam_status rcabeam_heevd_device(double* gram, double* eigenvalues, size_t nt
  * it to out (input dtype).  power (device double[rows], optional when writing)
  * receives |residual|^2 / nt, or sum |y|^2 / nt without bit 0 (gpu_clutter.py:196-273).
  * nt <= 512.  flags (device unsigned, optional, cleared by the caller) is ORed
- * with 1 when an input component is not finite and with 2 when a power is not
- * finite, the two checks gpu_clutter.py:25-40 and :271-272 make, in the same pass. */
+ * with 1 when an input component is not finite, with 2 when a power is not
+ * finite and with 4 when a written residual or retained sample is not finite,
+ * the checks gpu_clutter.py:25-40, :236-239 and :271-272 make, in the same pass. */
 rcabeam_status rcabeam_project_device(const void* iq, void* out, double* power, size_t rows, size_t nt,
                                       int complex128, const double* vectors, size_t k, int mode,
                                       unsigned* flags);

@@ -410,7 +410,7 @@ __global__ void __launch_bounds__(kAsyncThreads, 2)
 #pragma unroll
   for (int d = 0; d < kAsyncDepth - 1; ++d) issue(row + d * stride, d);
   const bool subtract = mode & 1;
-  bool bad_in = false, bad_out = false;
+  bool bad_in = false, bad_out = false, bad_row = false;
   for (int i = 0; row < rows; ++i, row += stride) {
     issue(row + (kAsyncDepth - 1) * stride, (i + kAsyncDepth - 1) % kAsyncDepth);
     asm volatile("cp.async.wait_group %0;" ::"n"(kAsyncDepth - 1) : "memory");
@@ -470,9 +470,16 @@ __global__ void __launch_bounds__(kAsyncThreads, 2)
           pw += r.x * r.x + r.y * r.y;
           if (mode & 2) {
             if constexpr (sizeof(IN) == 8)
-              reinterpret_cast<float2*>(out)[row * nt + t] = make_float2(float(r.x), float(r.y));
+              {
+              const float2 w = make_float2(float(r.x), float(r.y));
+              bad_row |= !isfinite(w.x) || !isfinite(w.y);
+              reinterpret_cast<float2*>(out)[row * nt + t] = w;
+            }
             else
+              {
+              bad_row |= !isfinite(r.x) || !isfinite(r.y);
               reinterpret_cast<double2*>(out)[row * nt + t] = r;
+            }
           }
         }
       }
@@ -492,7 +499,8 @@ __global__ void __launch_bounds__(kAsyncThreads, 2)
   }
   asm volatile("cp.async.wait_all;" ::: "memory");
   if (flags) {
-    const unsigned bits = (__any_sync(0xffffffffu, bad_in) ? 1u : 0u) | (__any_sync(0xffffffffu, bad_out) ? 2u : 0u);
+    const unsigned bits = (__any_sync(0xffffffffu, bad_in) ? 1u : 0u) |
+                          (__any_sync(0xffffffffu, bad_out) ? 2u : 0u) | (__any_sync(0xffffffffu, bad_row) ? 4u : 0u);
     if (bits && lane == 0) atomicOr(flags, bits);
   }
 }
@@ -593,7 +601,7 @@ __global__ void __launch_bounds__(kRegThreads, 3)
 #pragma unroll
   for (int d = 0; d < kAsyncDepth - 1; ++d) issue(row + d * stride, d);
   const bool subtract = mode & 1;
-  bool bad_in = false, bad_out = false;
+  bool bad_in = false, bad_out = false, bad_row = false;
   for (int i = 0; row < rows; ++i, row += stride) {
     issue(row + (kAsyncDepth - 1) * stride, (i + kAsyncDepth - 1) % kAsyncDepth);
     asm volatile("cp.async.wait_group %0;" ::"n"(kAsyncDepth - 1) : "memory");
@@ -650,7 +658,11 @@ __global__ void __launch_bounds__(kRegThreads, 3)
           }
           const double2 r = subtract ? make_double2(xv[f].x - proj.x, xv[f].y - proj.y) : proj;
           pw += r.x * r.x + r.y * r.y;
-          if (mode & 2) out[row * nt + t] = make_float2(float(r.x), float(r.y));
+          if (mode & 2) {
+            const float2 w = make_float2(float(r.x), float(r.y));
+            bad_row |= !isfinite(w.x) || !isfinite(w.y);
+            out[row * nt + t] = w;
+          }
         }
       }
     }
@@ -675,7 +687,8 @@ __global__ void __launch_bounds__(kRegThreads, 3)
   }
   asm volatile("cp.async.wait_all;" ::: "memory");
   if (flags) {
-    const unsigned bits = (__any_sync(0xffffffffu, bad_in) ? 1u : 0u) | (__any_sync(0xffffffffu, bad_out) ? 2u : 0u);
+    const unsigned bits = (__any_sync(0xffffffffu, bad_in) ? 1u : 0u) |
+                          (__any_sync(0xffffffffu, bad_out) ? 2u : 0u) | (__any_sync(0xffffffffu, bad_row) ? 4u : 0u);
     if (bits && lane == 0) atomicOr(flags, bits);
   }
 }
@@ -754,7 +767,7 @@ __global__ void __launch_bounds__(kDmmaThreads, 3)
   __syncthreads();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, q = lane & 3;
   const size_t groups = (rows + 7) / 8;
-  bool bad_in = false, bad_out = false;
+  bool bad_in = false, bad_out = false, bad_row = false;
   for (size_t g = size_t(blockIdx.x) * kDmmaWarps + warp; g < groups;
        g += size_t(gridDim.x) * kDmmaWarps) {
     const size_t r = 8 * g + (lane >> 2);
@@ -810,7 +823,11 @@ __global__ void __launch_bounds__(kDmmaThreads, 3)
           dmma_f64(d0, d1, a[0], b2[(2 * j) * 32 + lane], double(cur[i].x), double(cur[i].y));
           dmma_f64(d0, d1, a[1], b2[(2 * j + 1) * 32 + lane], d0, d1);
           pw[i & 1] = fma(d0, d0, fma(d1, d1, pw[i & 1]));
-          if (out && live && 4 * j + q < nt) out[r * size_t(nt) + 4 * j + q] = make_float2(float(d0), float(d1));
+          if (out && live && 4 * j + q < nt) {
+            const float2 w = make_float2(float(d0), float(d1));
+            bad_row |= !isfinite(w.x) || !isfinite(w.y);
+            out[r * size_t(nt) + 4 * j + q] = w;
+          }
         }
       }
 #pragma unroll
@@ -825,19 +842,21 @@ __global__ void __launch_bounds__(kDmmaThreads, 3)
     }
   }
   if (flags) {
-    const unsigned bits = (__any_sync(0xffffffffu, bad_in) ? 1u : 0u) | (__any_sync(0xffffffffu, bad_out) ? 2u : 0u);
+    const unsigned bits = (__any_sync(0xffffffffu, bad_in) ? 1u : 0u) |
+                          (__any_sync(0xffffffffu, bad_out) ? 2u : 0u) | (__any_sync(0xffffffffu, bad_row) ? 4u : 0u);
     if (bits && lane == 0) atomicOr(flags, bits);
   }
 }
 
-// The flags of project_rows_async for the other projection kernels: bit 0 for
-// a non-finite input component, bit 1 for a non-finite power (when given).
+// The flags of project_rows_async for the other projection kernels: `bit` 1 for
+// a non-finite input component or 4 for a non-finite filtered one; power_flags
+// sets 2 for a non-finite power.
 template <typename IN>
-__global__ void input_flags(const IN* __restrict__ x, size_t n, unsigned* __restrict__ flags) {
+__global__ void sample_flags(const IN* __restrict__ x, size_t n, unsigned bit, unsigned* __restrict__ flags) {
   bool bad = false;
   for (size_t i = size_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += size_t(gridDim.x) * blockDim.x)
     bad |= !isfinite(double(x[i].x)) || !isfinite(double(x[i].y));
-  if (__any_sync(0xffffffffu, bad) && (threadIdx.x & 31) == 0) atomicOr(flags, 1u);
+  if (__any_sync(0xffffffffu, bad) && (threadIdx.x & 31) == 0) atomicOr(flags, bit);
 }
 
 __global__ void power_flags(const double* __restrict__ power, size_t rows, unsigned* __restrict__ flags) {

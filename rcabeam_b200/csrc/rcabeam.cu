@@ -696,7 +696,7 @@ static void project_dispatch(const void* iq, void* out, double* power, size_t ro
     if (nt <= 256 && launch_async<IN, 8>(iq, out, power, rows, nt, vec, k, mode, flags)) return;
     if (nt > 256 && launch_async<IN, 16>(iq, out, power, rows, nt, vec, k, mode, flags)) return;
   }
-  if (flags) clutter::input_flags<IN><<<296, 256>>>(static_cast<const IN*>(iq), rows * nt, flags);
+  if (flags) clutter::sample_flags<IN><<<296, 256>>>(static_cast<const IN*>(iq), rows * nt, 1u, flags);
   size_t f = (nt + 31) / 32;
   if (f <= 1) launch_project<IN, 1>(iq, out, power, rows, nt, vec, k, mode);
   else if (f <= 2) launch_project<IN, 2>(iq, out, power, rows, nt, vec, k, mode);
@@ -704,6 +704,40 @@ static void project_dispatch(const void* iq, void* out, double* power, size_t ro
   else if (f <= 8) launch_project<IN, 8>(iq, out, power, rows, nt, vec, k, mode);
   else launch_project<IN, 16>(iq, out, power, rows, nt, vec, k, mode);
   if (flags && power) clutter::power_flags<<<148, 256>>>(power, rows, flags);
+  if (flags && (mode & 2)) clutter::sample_flags<IN><<<296, 256>>>(static_cast<const IN*>(out), rows * nt, 4u, flags);
+}
+
+// Float64 Gram on the tensor cores: from 32768 samples on (1000 x 33: 16 us
+// against 15 us of gram_simt; 2048 x 200: 34 against 74 us), which also keeps
+// the few rows of tiny inputs in gram_simt's sequential order.
+static bool gram_f64_eligible(size_t rows, size_t nt) {
+  return nt <= size_t(gramf64::kMaxFrames) && rows >= 256 && rows * nt >= 32768;
+}
+
+template <typename IN>
+static rcabeam_status gram_f64_launch(const void* iq, size_t rows, size_t nt, const double* scale, double* upper) {
+  gramf64::Params prm{};
+  prm.rows = rows;
+  prm.nt = int(nt);
+  prm.blocks = int((2 * nt + gramf64::kTile - 1) / gramf64::kTile);
+  prm.tiles = prm.blocks * (prm.blocks + 1) / 2;
+  prm.units = (prm.tiles + gramf64::kWarps - 1) / gramf64::kWarps;
+  // Slices of at most 4096 rows in whole waves: longer float64 sums lose accuracy
+  // (524288 x 130: 5.9e-15 relative with one wave, 2.6e-15 with this, 4.0e-15 for
+  // gram_simt's slices); and at least 64 rows, so that few rows do not drown in atomics.
+  const size_t wave = size_t(std::max(1, sm_count() / prm.units));
+  const size_t waves = std::max<size_t>(1, (rows + wave * 4096 - 1) / (wave * 4096));
+  prm.slices = int(std::min(wave * waves, (rows + 63) / 64));
+  prm.pitch = gramf64::row_pitch(prm.blocks);
+  prm.scale = scale;
+  prm.upper = upper;
+  const int stage = gramf64::stage_rows(int(nt));
+  const size_t smem = size_t(2) * stage * prm.pitch * sizeof(double);
+  auto kern = stage == 16 ? gramf64::gram_dmma<IN, 16> : gramf64::gram_dmma<IN, 8>;
+  if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)) != cudaSuccess)
+    return RCABEAM_ERROR_CUDA;
+  kern<<<unsigned(prm.units) * unsigned(prm.slices), gramf64::kThreads, smem>>>(static_cast<const IN*>(iq), prm);
+  return launch_status();
 }
 
 // ---------------------------------------------- no-allocation entry point --

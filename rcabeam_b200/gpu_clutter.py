@@ -207,19 +207,26 @@ def _project(matrix: torch.Tensor, vectors_cm: torch.Tensor, k: int, mode: int, 
 
 def apply_temporal_filter(iq, basis, *, rank_start: int, rank_stop: int | None = None):
     """Filtered IQ keeping ranks [start, stop) via the smaller projector (gpu_clutter.py:219-241)."""
-    arrays = _inputs(iq)
+    arrays = _inputs(iq, check_finite=False)  # the projection flags non-finite samples
     frames = arrays[0].shape[-1]
-    start, stop = _rank_interval(frames, rank_start, rank_stop)
-    vectors, subtract = _filter_vectors(basis, frames, start, stop)
+    try:
+        start, stop = _rank_interval(frames, rank_start, rank_stop)
+        vectors, subtract = _filter_vectors(basis, frames, start, stop)
+    except ValueError:
+        _inputs(iq)  # non-finite IQ is reported first
+        raise
     k = vectors.shape[0]
-    result = []
-    for a in arrays:
+    result, flags = [], torch.zeros(len(arrays), dtype=torch.int32, device=arrays[0].device)
+    for i, a in enumerate(arrays):
         m = _rows(a)
         out = torch.empty_like(m)
-        _project(m, vectors, k, (1 if subtract else 0) | 2, out, None)
-        if not bool(torch.isfinite(torch.view_as_real(out)).all()):
-            raise np.linalg.LinAlgError("Nonfinite filtered IQ; rescale the input")
+        _project(m, vectors, k, (1 if subtract else 0) | 2, out, None, flags[i:])
         result.append(out.reshape(a.shape))
+    bits = flags.tolist()
+    if any(b & 1 for b in bits):
+        raise ValueError("IQ must be finite")
+    if any(b & 4 for b in bits):
+        raise np.linalg.LinAlgError("Nonfinite filtered IQ; rescale the input")
     return tuple(result) if isinstance(iq, tuple) else result[0]
 
 
@@ -249,8 +256,12 @@ def filtered_power(iq, basis, *, rank_start: int, rank_stop: int | None = None) 
 def svd_clutter_filter(iq, *, rank_start: int, rank_stop: int | None = None, method: str = "gram",
                        precision: str = "complex128"):
     """Gram-EVD temporal filter keeping ranks [start, stop); no silent precision fallback (gpu_clutter.py:322-336)."""
-    arrays = _inputs(iq)
-    _rank_interval(arrays[0].shape[-1], rank_start, rank_stop)
+    arrays = _inputs(iq, check_finite=False)  # temporal_basis reports non-finite samples
+    try:
+        _rank_interval(arrays[0].shape[-1], rank_start, rank_stop)
+    except ValueError:
+        _inputs(iq)  # non-finite IQ is reported first
+        raise
     _, basis = temporal_basis(iq, method=method, precision=precision)
     return apply_temporal_filter(iq, basis, rank_start=rank_start, rank_stop=rank_stop)
 

@@ -430,3 +430,43 @@ def test_projection_flags_non_finite_rows():
     assert int(flags.item()) == 3
     pw = power.cpu().numpy()
     assert not np.isfinite(pw[17]) and np.isfinite(np.delete(pw, 17)).all()
+
+
+@pytest.mark.parametrize("rows,nt", [(8192, 4), (2048, 16), (1025, 33), (700, 75), (4099, 128), (513, 256), (300, 257),
+                                     (333, 512)])
+@pytest.mark.parametrize("dtype", [torch.complex64, torch.complex128])
+def test_float64_gram_tiles_and_slices(rows, nt, dtype):
+    """The float64 tensor-core Gram off its 32-column tiles, 8/16-row stages and row slices, few
+    tiles shared by several warps included: 16 float64 roundings per sqrt(rows) of the sum."""
+    gen = torch.Generator(device="cuda").manual_seed(rows)
+    x = torch.randn((rows, nt), dtype=dtype, generator=gen, device="cuda")
+    gram = gpu_clutter.Gram(nt, x.device)
+    assert gram.accumulate((x,), "complex128") == rows
+    scaled = x.to(torch.complex128) / gram.scale
+    expected = scaled.mH @ scaled / rows
+    error = torch.linalg.matrix_norm(gram.vectors() - expected) / torch.linalg.matrix_norm(expected)
+    assert float(error) <= 16 * 2.0**-53 * rows**0.5
+
+
+def test_filter_flags_non_finite_rows_and_keeps_error_order():
+    """apply_temporal_filter reports non-finite IQ before a bad rank or basis, and an overflowing result."""
+    iq = torch.ones((40, 36), dtype=torch.complex64, device="cuda")
+    eye = torch.eye(36, dtype=torch.complex128, device="cuda")
+    bad = iq.clone()
+    bad[7, 3] = complex(float("nan"), 0.0)
+    for basis, rank in ((eye, 2), (eye, 99), (2 * eye, 2)):
+        with pytest.raises(ValueError, match="IQ must be finite"):
+            gpu_clutter.apply_temporal_filter(bad, basis, rank_start=rank)
+    with pytest.raises(ValueError, match="IQ must be finite"):
+        gpu_clutter.svd_clutter_filter(bad, rank_start=99)
+    # |x| fits float32 in every frame, the share of a row along v does not in frame 0.
+    v = torch.full((36, 1), 0.6 / 35**0.5, dtype=torch.complex128, device="cuda")
+    v[0] = 0.8
+    basis, _ = torch.linalg.qr(torch.cat((v, eye[:, 1:]), dim=1))
+    spike = torch.zeros((9, 36), dtype=torch.complex64, device="cuda")
+    spike[5] = 3e38
+    for ranks in ({"rank_start": 0, "rank_stop": 1}, {"rank_start": 1}):
+        with pytest.raises(np.linalg.LinAlgError, match="Nonfinite filtered IQ"):
+            gpu_clutter.apply_temporal_filter(spike, basis, **ranks)
+        with pytest.raises(np.linalg.LinAlgError, match="Nonfinite filtered IQ"):
+            gpu_clutter.apply_temporal_filter(spike.to(torch.complex128) * 5e269, basis, **ranks)
