@@ -21,6 +21,7 @@
 #include "das_generic.cuh"
 #include "das_rows.cuh"
 #include "das_tc.cuh"
+#include "gram_f64.cuh"
 #include "gram_tc.cuh"
 #include "pack.cuh"
 #include "scene.cuh"
@@ -908,6 +909,9 @@ rcabeam_status rcabeam_gram_accumulate_device(const void* iq, size_t rows, size_
       return RCABEAM_ERROR_ARGUMENT;
     return gram_tc_launch(iq, rows, nt, scale, precision == 2, upper);
   }
+  if (precision == 0 && gram_f64_eligible(rows, nt))
+    return complex128 ? gram_f64_launch<double2>(iq, rows, nt, scale, upper)
+                      : gram_f64_launch<float2>(iq, rows, nt, scale, upper);
   int nb = int((nt + clutter::kGramTile - 1) / clutter::kGramTile);
   unsigned tiles = unsigned(nb * (nb + 1) / 2);
   size_t want = (148 * 8 + tiles - 1) / tiles;
