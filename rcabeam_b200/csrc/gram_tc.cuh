@@ -15,7 +15,10 @@
 // the same time (one HBM read, the rest from L2).  TMEM holds the unit's four
 // 128 x 128 float32 accumulators (512 columns); every kFlushRows rows (and at
 // the end of the slice) the epilogue adds them, in float64, to the upper
-// triangle with atomics, which bounds the float32 accumulation length.
+// triangle with atomics, which bounds the float32 accumulation length.  The
+// accumulators pass through shared memory first, so that a warp's atomics fall on
+// two runs of 128 bytes; with accumulator rows on the lanes every one was a sector
+// of its own, and the MMAs stood still for a quarter of the kernel.
 //
 // Precision (both with float32 accumulation):
 //   tf32   : operands rounded to nearest TF32 (cvt.rna) -- one MMA per K=8;
@@ -25,18 +28,30 @@
 // bounds the Casorati scale s (max |component|), which keeps the products in
 // range exactly as the scaled float64 Gram does; the epilogue applies (2^e/s)^2.
 //
-// Roles (256 threads, one CTA per SM):
+// Roles (448 threads, one CTA per SM):
 //   warp 0       TMA producer: raw float32 boxes (32 columns x 16 rows;
 //                SWIZZLE_128B_ATOM_32B for TF32, SWIZZLE_128B for 3xBF16) of
 //                the unit's staged blocks into the staging ring;
 //   warp 1       TMEM allocator; lane 0 issues tcgen05.mma and commits;
-//   warps 2-7    converters: TF32 rounds the staged floats in place (the
+//   warps 2-13   converters: TF32 rounds the staged floats in place (the
 //                layouts coincide), so the staging ring is the operand ring
 //                (2 x ring stages, eight with three staged blocks); 3xBF16
 //                writes hi/lo operands in the UMMA MN-major SWIZZLE_128B
 //                layout (ring staging stages and ring operand stages in the
 //                same shared memory; ring = 4 with three staged blocks);
-//   warps 4-7    also the epilogue (TMEM lane quarters 0-3) at every flush.
+//                they are also the epilogue at every flush, three warps per
+//                TMEM lane quarter.
+//
+// What bounds it: the hand-over of 16-row stages between the roles.  Per stage the
+// MMA thread issues up to 12 MMAs and has to find the stage converted, so its
+// descriptors are held in registers and the converters (twelve warps, all their
+// loads in flight; eight or sixteen were slower) work a stage ahead; every flush
+// stops it, so flushes write whole sectors; pairs of outputs share MMAs of 256
+// columns, which read less shared memory.  Each of these alone gave little, since
+// the next one bound (4194304 x 400 3xBF16, one B200): 16.9 ms before, 14.8 to
+// 18.9 with some, 11.6 with all of them; TF32 14.0 -> 8.6 ms; 4194304 x 200 3xBF16
+// 7.3 -> 4.65, TF32 6.0 -> 3.6 ms; 1000000 x 16 TF32 0.27 -> 0.20 ms.  The MMAs
+// themselves take about 7 ms at 400 frames in 3xBF16.
 #pragma once
 
 #include <cuda_bf16.h>
@@ -54,14 +69,18 @@ constexpr int kMaxTasks = 4;       // output blocks per unit (4 x 128 TMEM colum
 constexpr int kMaxUnits = 48;      // nb <= 16 blocks (T <= 1024): 136 upper blocks -> 43 units
 constexpr int kMaxBlocks = 16;
 constexpr int kMaxRing = 4;        // deepest 3xBF16 staging and operand rings (TF32: one ring of 2 x ring)
-constexpr int kThreads = 256;
-constexpr int kConverters = 6 * 32;
+constexpr int kConvWarps = 12;
+constexpr int kConverters = kConvWarps * 32;
+constexpr int kThreads = 64 + kConverters;
 constexpr int kSlotBytes = kBlock * kRows * 4;  // 8192: one staged block per stage (f32 or bf16 hi+lo)
 // The tensor core rounds each float32 accumulation toward zero (a shrink of
 // ~1.3e-8 per update); flushing to float64 every 2048 rows (256 TF32 or 384
 // BF16 updates) keeps that bias near 3e-6 of a Gram entry.
 constexpr int kFlushRows = 2048;
 constexpr int kTmemCols = 512;
+constexpr int kControlBytes = 1024;  // barriers and the TMEM slot
+constexpr int kTilePitch = 17;       // floats between rows of an epilogue warp's transposition tile
+constexpr int kFlushTile = 32 * kTilePitch;
 // MN-major TF32 operands take the 128-byte swizzle with 32-byte granules (the
 // TMA's SWIZZLE_128B_ATOM_32B): 4-row K atoms, so SBO = 512 B; BF16 operands
 // take the plain 128-byte swizzle (8-row atoms, SBO = 1024 B).
@@ -71,8 +90,11 @@ struct Unit {
   int nload;
   int load[kMaxLoads];  // staged block per slot
   int ntask;
-  int a_slot[kMaxTasks], b_slot[kMaxTasks];
+  int a_slot[kMaxTasks], b_slot[kMaxTasks];  // of the output blocks, in TMEM order
   int a_blk[kMaxTasks], b_blk[kMaxTasks];
+  int nop;
+  int op_task[kMaxTasks];  // first output of each MMA
+  int op_n[kMaxTasks];     // its columns: 256 when it covers two outputs, else 128
 };
 
 struct Params {
@@ -86,7 +108,7 @@ struct Params {
 };
 
 __host__ __device__ inline size_t smem_bytes(int nload_max, int ring) {
-  return size_t(2 * ring) * nload_max * kSlotBytes + 1024 + 1024;
+  return size_t(2 * ring) * nload_max * kSlotBytes + 1024 + kControlBytes + kConvWarps * kFlushTile * sizeof(float);
 }
 
 // kind::tf32 / kind::f16(BF16) instruction descriptor: F32 accumulate, A and B MN-major.
@@ -117,14 +139,28 @@ __device__ __forceinline__ uint32_t pack_bf16(float lo_elem, float hi_elem) {
 
 // Split 8 scaled floats into BF16 hi and lo 16-byte chunks.
 __device__ __forceinline__ void split8(const float (&v)[8], uint4& hi, uint4& lo) {
-  float h[8], l[8];
+  uint32_t h[4], l[4];
 #pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    h[i] = __bfloat162float(__float2bfloat16_rn(v[i]));
-    l[i] = v[i] - h[i];
+  for (int i = 0; i < 4; ++i) {
+    const __nv_bfloat162 b = __floats2bfloat162_rn(v[2 * i], v[2 * i + 1]);
+    h[i] = *reinterpret_cast<const uint32_t*>(&b);
+    l[i] = pack_bf16(v[2 * i] - __low2float(b), v[2 * i + 1] - __high2float(b));
   }
-  hi = make_uint4(pack_bf16(h[0], h[1]), pack_bf16(h[2], h[3]), pack_bf16(h[4], h[5]), pack_bf16(h[6], h[7]));
-  lo = make_uint4(pack_bf16(l[0], l[1]), pack_bf16(l[2], l[3]), pack_bf16(l[4], l[5]), pack_bf16(l[6], l[7]));
+  hi = make_uint4(h[0], h[1], h[2], h[3]);
+  lo = make_uint4(l[0], l[1], l[2], l[3]);
+}
+
+// 32 lanes x 16 consecutive 32-bit columns.
+__device__ __forceinline__ void tmem_ld16(uint32_t addr, float (&v)[16]) {
+  uint32_t r[16];
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
+        "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+      : "r"(addr));
+  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+  for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[i]);
 }
 
 template <bool TF32>
@@ -147,6 +183,7 @@ __global__ void __launch_bounds__(kThreads, 1) gram_tc(const __grid_constant__ C
   uint64_t* acc_empty = acc_full + 1;
   uint64_t* drain = acc_empty + 1;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(drain + 1);
+  float* flush_tiles = reinterpret_cast<float*>(smem + 2 * p.ring * stage_bytes + kControlBytes);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const long long r0 = (long long)slice * p.slice_rows;
@@ -157,12 +194,12 @@ __global__ void __launch_bounds__(kThreads, 1) gram_tc(const __grid_constant__ C
   if (threadIdx.x == 0) {
     for (int s = 0; s < R; ++s) {
       mbar_init(&stg_full[s], 1);
-      mbar_init(&stg_empty[s], TF32 ? 1 : kConverters / 32);  // TF32: freed by the MMA commit
-      mbar_init(&op_full[s], kConverters / 32);
+      mbar_init(&stg_empty[s], TF32 ? 1 : kConvWarps);  // TF32: freed by the MMA commit
+      mbar_init(&op_full[s], kConvWarps);
       mbar_init(&op_empty[s], 1);
     }
     mbar_init(acc_full, 1);
-    mbar_init(acc_empty, 4);
+    mbar_init(acc_empty, kConvWarps);
     mbar_init(drain, 1);
     fence_mbar_init();
   }
@@ -187,20 +224,21 @@ __global__ void __launch_bounds__(kThreads, 1) gram_tc(const __grid_constant__ C
   if (warp == 0) {
     // ------------------------------------------------------------- producer --
     if (lane == 0) prefetch_tensormap(&map);
-    int k = 0;
-    bool ok = true;
-    for (; k < nstages && ok; ++k) {
-      const int s_ = k % R;
-      if (k >= R) ok = __all_sync(0xffffffffu, mbar_wait(&stg_empty[s_], ((k / R) - 1) & 1, p.err, kErrWaitEmpty));
-      if (!ok) break;
+    int k = 0, s_ = 0;
+    uint32_t parity = 1;  // of the phase that frees the stage: the first round finds it free
+    const int nload = u.nload;
+    const int box_col = lane < 4 * nload ? u.load[lane >> 2] * kBlock + 32 * (lane & 3) : 0;
+    for (; k < nstages; ++k) {
+      if (!__all_sync(0xffffffffu, mbar_wait_fast(&stg_empty[s_], parity, p.err, kErrWaitEmpty))) break;
       const int row = int(r0 + (long long)k * kRows);
-      if (lane == 0) mbar_arrive_expect_tx(&stg_full[s_], uint32_t(u.nload * kSlotBytes));
+      if (lane == 0) mbar_arrive_expect_tx(&stg_full[s_], uint32_t(nload * kSlotBytes));
       __syncwarp();
-      unsigned char* dst = staging + s_ * stage_bytes;
       // 4 boxes (32 columns) per staged block, one box per lane.
-      if (lane < 4 * u.nload) {
-        const int slot = lane >> 2, box = lane & 3;
-        tma_load_2d(dst + slot * kSlotBytes + box * 2048, &map, &stg_full[s_], u.load[slot] * kBlock + 32 * box, row);
+      if (lane < 4 * nload)
+        tma_load_2d(staging + s_ * stage_bytes + lane * 2048, &map, &stg_full[s_], box_col, row);
+      if (++s_ == R) {
+        s_ = 0;
+        parity ^= 1;
       }
     }
     // Drain: the last issued stages' copies have landed before the CTA exits.
@@ -212,39 +250,53 @@ __global__ void __launch_bounds__(kThreads, 1) gram_tc(const __grid_constant__ C
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA --
     if (lane == 0) {
-      const uint32_t idesc = idesc_mn(TF32, 128, 128);
-      int flushes = 0;
-      for (int k = 0; k < nstages; ++k) {
-        const int s_ = k % R;
-        const int in_seg = k % kStagesPerFlush;
-        if (in_seg == 0 && flushes > 0 && !mbar_wait(acc_empty, (flushes - 1) & 1, p.err, kErrWaitEmpty)) break;
-        if (!mbar_wait(&op_full[s_], (k / R) & 1, p.err, kErrWaitFull)) break;
-        tc_fence_after();
-        const uint32_t op = smem_u32(operands + s_ * stage_bytes);
-        for (int t = 0; t < u.ntask; ++t) {
-          const uint32_t d = tmem + uint32_t(kBlock * t);
-          if constexpr (TF32) {
+      // Everything about the unit's MMAs that does not change from stage to stage is
+      // held in registers: this one thread's time per stage sets the kernel's pace
+      // as soon as the converters keep up.
+      constexpr uint32_t kAHalf = TF32 ? kSlotBytes : kSlotBytes / 2;  // bytes of one staged operand
+      const int nop = u.nop;
+      uint32_t a_at[kMaxTasks], b_at[kMaxTasks], d_at[kMaxTasks], idesc[kMaxTasks];
 #pragma unroll
-            for (int q = 0; q < 2; ++q) {
-              const uint32_t a = op + u.a_slot[t] * kSlotBytes + q * 1024;
-              const uint32_t b = op + u.b_slot[t] * kSlotBytes + q * 1024;
-              mma_tf32(d, smem_desc(a, 2048, 512, kLayoutSw128Base32), smem_desc(b, 2048, 512, kLayoutSw128Base32),
-                       idesc, (in_seg > 0 || q > 0) ? 1u : 0u);
-            }
+      for (int i = 0; i < kMaxTasks; ++i) {
+        const int t = i < nop ? u.op_task[i] : 0;
+        a_at[i] = uint32_t(u.a_slot[t]) * kAHalf >> 4;
+        b_at[i] = uint32_t(u.b_slot[t]) * kAHalf >> 4;
+        d_at[i] = tmem + uint32_t(kBlock * t);
+        idesc[i] = idesc_mn(TF32, 128, i < nop ? u.op_n[i] : kBlock);
+      }
+      const uint64_t fixed = TF32 ? smem_desc(0, 2048, 512, kLayoutSw128Base32) : smem_desc(0, 2048, 1024, kLayoutSw128);
+      const uint32_t lo = uint32_t(p.nload_max) * (kSlotBytes / 2) >> 4;
+      const uint32_t first = smem_u32(operands) >> 4, step = uint32_t(stage_bytes) >> 4;
+      int flushes = 0, s_ = 0, in_seg = 0;
+      uint32_t parity = 0;
+      for (int k = 0; k < nstages; ++k) {
+        if (in_seg == 0 && flushes > 0 && !mbar_wait_fast(acc_empty, (flushes - 1) & 1, p.err, kErrWaitEmpty)) break;
+        if (!mbar_wait_fast(&op_full[s_], parity, p.err, kErrWaitFull)) break;
+        tc_fence_after();
+        const uint64_t op = fixed + (first + uint32_t(s_) * step);
+        const uint32_t more = in_seg > 0 ? 1u : 0u;
+#pragma unroll
+        for (int i = 0; i < kMaxTasks; ++i) {
+          if (i >= nop) break;
+          const uint64_t a = op + a_at[i], b = op + b_at[i];
+          if constexpr (TF32) {
+            mma_tf32(d_at[i], a, b, idesc[i], more);
+            mma_tf32(d_at[i], a + 64, b + 64, idesc[i], 1u);  // rows 8-15: 1024 bytes on
           } else {
-            const uint32_t hi = op, lo = op + uint32_t(p.nload_max) * (kSlotBytes / 2);
-            const uint32_t ah = hi + u.a_slot[t] * (kSlotBytes / 2), al = lo + u.a_slot[t] * (kSlotBytes / 2);
-            const uint32_t bh = hi + u.b_slot[t] * (kSlotBytes / 2), bl = lo + u.b_slot[t] * (kSlotBytes / 2);
-            mma_f16(d, smem_desc(ah, 2048, 1024, kLayoutSw128), smem_desc(bh, 2048, 1024, kLayoutSw128), idesc,
-                    in_seg > 0 ? 1u : 0u);
-            mma_f16(d, smem_desc(al, 2048, 1024, kLayoutSw128), smem_desc(bh, 2048, 1024, kLayoutSw128), idesc, 1u);
-            mma_f16(d, smem_desc(ah, 2048, 1024, kLayoutSw128), smem_desc(bl, 2048, 1024, kLayoutSw128), idesc, 1u);
+            mma_f16(d_at[i], a, b, idesc[i], more);
+            mma_f16(d_at[i], a + lo, b, idesc[i], 1u);
+            mma_f16(d_at[i], a, b + lo, idesc[i], 1u);
           }
         }
         mma_commit(TF32 ? &stg_empty[s_] : &op_empty[s_]);
-        if (in_seg == kStagesPerFlush - 1 || k == nstages - 1) {
+        if (++in_seg == kStagesPerFlush || k == nstages - 1) {
           mma_commit(acc_full);
           ++flushes;
+          in_seg = 0;
+        }
+        if (++s_ == R) {
+          s_ = 0;
+          parity ^= 1;
         }
       }
       mma_commit(drain);
@@ -253,50 +305,67 @@ __global__ void __launch_bounds__(kThreads, 1) gram_tc(const __grid_constant__ C
     __syncwarp();
   } else {
     // ------------------------------------------------ converters / epilogue --
-    const int ct = threadIdx.x - 64;  // 0 .. 191
-    const bool epilogue = warp >= 4;
-    const int quarter = warp & 3;
-    int flushes = 0;
+    const int ct = threadIdx.x - 64;  // 0 .. kConverters - 1
+    const int quarter = warp & 3, part = (warp - 2) >> 2;  // TMEM lanes, share of a quarter's columns
+    const int nload = u.nload;
+    int flushes = 0, s_ = 0, in_seg = 0;
+    uint32_t parity = 0;
     for (int k = 0; k < nstages; ++k) {
-      const int s_ = k % R;
-      if (!__all_sync(0xffffffffu, mbar_wait(&stg_full[s_], (k / R) & 1, p.err, kErrWaitFull))) break;
-      if (!TF32 && k >= R &&
-          !__all_sync(0xffffffffu, mbar_wait(&op_empty[s_], ((k / R) - 1) & 1, p.err, kErrWaitEmpty)))
-        break;
+      if (!__all_sync(0xffffffffu, mbar_wait_fast(&stg_full[s_], parity, p.err, kErrWaitFull))) break;
+      if (!TF32 && !__all_sync(0xffffffffu, mbar_wait_fast(&op_empty[s_], parity ^ 1, p.err, kErrWaitEmpty))) break;
       const unsigned char* src = staging + s_ * stage_bytes;
       unsigned char* dst = operands + s_ * stage_bytes;
       if constexpr (TF32) {
-        // In place (dst == src): an elementwise map over the staged bytes.
-        const int chunks = u.nload * (kSlotBytes / 16);
-        for (int i = ct; i < chunks; i += kConverters) {
-          float4 v = reinterpret_cast<const float4*>(src)[i];
-          v.x = round_tf32(v.x * prescale);
-          v.y = round_tf32(v.y * prescale);
-          v.z = round_tf32(v.z * prescale);
-          v.w = round_tf32(v.w * prescale);
-          reinterpret_cast<float4*>(dst)[i] = v;
+        // In place (dst == src): an elementwise map over the staged bytes, four
+        // loads in flight per thread.
+        const int chunks = nload * (kSlotBytes / 16);
+        for (int i0 = ct; i0 < chunks; i0 += 4 * kConverters) {
+          float4 v[4];
+#pragma unroll
+          for (int j = 0; j < 4; ++j)
+            if (i0 + j * kConverters < chunks) v[j] = reinterpret_cast<const float4*>(src)[i0 + j * kConverters];
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            v[j].x = round_tf32(v[j].x * prescale);
+            v[j].y = round_tf32(v[j].y * prescale);
+            v[j].z = round_tf32(v[j].z * prescale);
+            v[j].w = round_tf32(v[j].w * prescale);
+            if (i0 + j * kConverters < chunks) reinterpret_cast<float4*>(dst)[i0 + j * kConverters] = v[j];
+          }
         }
       } else {
-        // Item = (slot, row, 64-column atom, 16-byte output chunk of 8 BF16).
+        // Item = (slot, row, 64-column atom, 16-byte output chunk of 8 BF16); both of
+        // a thread's items are loaded before either is converted.
         unsigned char* hi = dst;
         unsigned char* lo = dst + size_t(p.nload_max) * (kSlotBytes / 2);
-        const int items = u.nload * kRows * 16;
-        for (int i = ct; i < items; i += kConverters) {
-          const int slot = i >> 8, rem = i & 255;
-          const int row = rem >> 4, atom = (rem >> 3) & 1, c = rem & 7;
-          const int sw = row & 7;
-          const int box = 2 * atom + (c >> 2);
-          const int c0 = 2 * (c & 3);
-          const unsigned char* rbase = src + slot * kSlotBytes + box * 2048 + (row >> 3) * 1024 + sw * 128;
-          const float4 x0 = *reinterpret_cast<const float4*>(rbase + ((c0 ^ sw) << 4));
-          const float4 x1 = *reinterpret_cast<const float4*>(rbase + (((c0 + 1) ^ sw) << 4));
-          const float v[8] = {x0.x * prescale, x0.y * prescale, x0.z * prescale, x0.w * prescale,
-                              x1.x * prescale, x1.y * prescale, x1.z * prescale, x1.w * prescale};
-          uint4 h, l;
-          split8(v, h, l);
-          const int off = slot * (kSlotBytes / 2) + atom * 2048 + (row >> 3) * 1024 + sw * 128 + ((c ^ sw) << 4);
-          *reinterpret_cast<uint4*>(hi + off) = h;
-          *reinterpret_cast<uint4*>(lo + off) = l;
+        const int items = nload * kRows * 16;
+        for (int i0 = ct; i0 < items; i0 += 2 * kConverters) {
+          float4 x[2][2];
+          int off[2];
+#pragma unroll
+          for (int j = 0; j < 2; ++j) {
+            const int i = min(i0 + j * kConverters, items - 1);
+            const int slot = i >> 8, rem = i & 255;
+            const int row = rem >> 4, atom = (rem >> 3) & 1, c = rem & 7;
+            const int sw = row & 7;
+            const int box = 2 * atom + (c >> 2);
+            const int c0 = 2 * (c & 3);
+            const unsigned char* rbase = src + slot * kSlotBytes + box * 2048 + (row >> 3) * 1024 + sw * 128;
+            x[j][0] = *reinterpret_cast<const float4*>(rbase + ((c0 ^ sw) << 4));
+            x[j][1] = *reinterpret_cast<const float4*>(rbase + (((c0 + 1) ^ sw) << 4));
+            off[j] = slot * (kSlotBytes / 2) + atom * 2048 + (row >> 3) * 1024 + sw * 128 + ((c ^ sw) << 4);
+          }
+#pragma unroll
+          for (int j = 0; j < 2; ++j) {
+            const float v[8] = {x[j][0].x * prescale, x[j][0].y * prescale, x[j][0].z * prescale, x[j][0].w * prescale,
+                                x[j][1].x * prescale, x[j][1].y * prescale, x[j][1].z * prescale, x[j][1].w * prescale};
+            uint4 h, l;
+            split8(v, h, l);
+            if (i0 + j * kConverters < items) {
+              *reinterpret_cast<uint4*>(hi + off[j]) = h;
+              *reinterpret_cast<uint4*>(lo + off[j]) = l;
+            }
+          }
         }
       }
       fence_async_smem();  // generic-proxy writes -> visible to the tensor core
@@ -305,31 +374,39 @@ __global__ void __launch_bounds__(kThreads, 1) gram_tc(const __grid_constant__ C
         if (!TF32) mbar_arrive(&stg_empty[s_]);
         mbar_arrive(&op_full[s_]);
       }
-      const bool flush_here = (k % kStagesPerFlush) == kStagesPerFlush - 1 || k == nstages - 1;
-      if (epilogue && flush_here) {
+      if (++s_ == R) {
+        s_ = 0;
+        parity ^= 1;
+      }
+      if (++in_seg == kStagesPerFlush || k == nstages - 1) {
+        in_seg = 0;
         if (!__all_sync(0xffffffffu, mbar_wait(acc_full, flushes & 1, p.err, kErrWaitFull))) break;
         tc_fence_after();
-        const int m_lane = 32 * quarter + lane;  // accumulator row within the block
-        const bool even = (lane & 1) == 0;
+        float* tile = flush_tiles + (warp - 2) * kFlushTile;
+        const int col = lane & 15;
         for (int t = 0; t < u.ntask; ++t) {
-          const int row_real = u.a_blk[t] * kBlock + m_lane;  // row of D
-          const int m = row_real >> 1;                         // frame of the row
-          for (int c0 = 0; c0 < kBlock; c0 += 32) {
-            float val[32];
-            tmem_ld32(tmem + (uint32_t(32 * quarter) << 16) + uint32_t(kBlock * t + c0), val);
+          // A block below the diagonal is stored as its conjugate transpose.
+          const bool lower = u.a_blk[t] > u.b_blk[t];
+          for (int c0 = 0; c0 < kBlock; c0 += 16) {
+            if ((t * (kBlock / 16) + c0 / 16) % (kConvWarps / 4) != part) continue;
+            float val[16];
+            tmem_ld16(tmem + (uint32_t(32 * quarter) << 16) + uint32_t(kBlock * t + c0), val);
 #pragma unroll
-            for (int i = 0; i < 16; ++i) {
-              const float o_re = __shfl_xor_sync(0xffffffffu, val[2 * i], 1);
-              const float o_im = __shfl_xor_sync(0xffffffffu, val[2 * i + 1], 1);
-              // Even row 2m holds (D[2m][2n], D[2m][2n+1]); its partner row 2m+1 the same columns.
-              const int n = (u.b_blk[t] * kBlock + c0) / 2 + i;
-              if (even && m < p.nt && n < p.nt) {
-                const double re = double(val[2 * i]) + double(o_im);
-                const double im = double(val[2 * i + 1]) - double(o_re);
-                atomicAdd(p.upper + 2 * (size_t(m) * p.nt + n), re * factor);
-                atomicAdd(p.upper + 2 * (size_t(m) * p.nt + n) + 1, im * factor);
-              }
+            for (int i = 0; i < 16; ++i) tile[lane * kTilePitch + i] = val[i];
+            __syncwarp();
+            // Sixteen lanes take the components of eight frame pairs (m, n), n along
+            // the lanes: re = D[2m][2n] + D[2m+1][2n+1], im = D[2m][2n+1] - D[2m+1][2n].
+            const int n = (u.b_blk[t] * kBlock + c0 + col) / 2;
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+              const int row = 2 * (2 * i + (lane >> 4));
+              const int m = (u.a_blk[t] * kBlock + 32 * quarter + row) / 2;
+              const double x = double(tile[row * kTilePitch + col]), y = double(tile[(row + 1) * kTilePitch + (col ^ 1)]);
+              const double v = col & 1 ? (lower ? y - x : x - y) : x + y;
+              if (m < p.nt && n < p.nt)
+                atomicAdd(p.upper + 2 * (lower ? size_t(n) * p.nt + m : size_t(m) * p.nt + n) + (col & 1), v * factor);
             }
+            __syncwarp();  // the tile is read before the next columns overwrite it
           }
         }
         tc_fence_before();
@@ -382,6 +459,52 @@ inline bool diagonal_path(int d, int nb, int n, const Unit* units, int* owner, b
       }
   }
   return false;
+}
+
+// Orders a unit's staged blocks so that as many pairs of outputs as possible share
+// one MMA of 256 columns, (a, b) and (a, c) with b and c staged side by side, and
+// lists its outputs (either triangle) and MMAs in that order.  An MMA of 128
+// columns reads its two operands for half the work of one with 256: the MMAs'
+// operand reads are most of the kernel's shared-memory traffic, which bounds it.
+inline void merge_outputs(Unit& un) {
+  bool need[kMaxBlocks][kMaxBlocks] = {};
+  for (int t = 0; t < un.ntask; ++t)
+    need[un.a_blk[t]][un.b_blk[t]] = need[un.b_blk[t]][un.a_blk[t]] = true;
+  static const int kOrders[6][3] = {{0, 1, 2}, {0, 2, 1}, {1, 0, 2}, {1, 2, 0}, {2, 0, 1}, {2, 1, 0}};
+  Unit best{};
+  for (const auto& order : kOrders) {
+    Unit c{};
+    c.nload = un.nload;
+    bool valid = true;
+    for (int j = 0; j < un.nload; ++j) {
+      valid = valid && order[j] < un.nload;
+      c.load[j] = un.load[order[j] < un.nload ? order[j] : 0];
+    }
+    if (!valid) continue;
+    bool open[kMaxBlocks][kMaxBlocks];
+    for (int a = 0; a < kMaxBlocks; ++a)
+      for (int b = 0; b < kMaxBlocks; ++b) open[a][b] = need[a][b];
+    auto add = [&](int i, int j, int outputs) {
+      c.op_task[c.nop] = c.ntask;
+      c.op_n[c.nop++] = outputs * kBlock;
+      for (int k = j; k < j + outputs; ++k) {
+        const int a = c.load[i], b = c.load[k];
+        c.a_slot[c.ntask] = i;
+        c.b_slot[c.ntask] = k;
+        c.a_blk[c.ntask] = a;
+        c.b_blk[c.ntask++] = b;
+        open[a][b] = open[b][a] = false;
+      }
+    };
+    for (int i = 0; i < c.nload; ++i)
+      for (int j = 0; j + 1 < c.nload; ++j)
+        if (open[c.load[i]][c.load[j]] && open[c.load[i]][c.load[j + 1]]) add(i, j, 2);
+    for (int i = 0; i < c.nload; ++i)
+      for (int j = 0; j < c.nload; ++j)
+        if (open[c.load[i]][c.load[j]]) add(i, j, 1);
+    if (!best.nop || c.nop < best.nop) best = c;
+  }
+  un = best;
 }
 
 // Pack the upper 128-column blocks (b <= c) of an nb-block Gram into units of
@@ -454,6 +577,7 @@ inline int plan_units(int nb, Unit* units, int* nload_max) {
     if (!rest) return 0;
     unit_add(*rest, d, d);
   }
+  for (int u = 0; u < count; ++u) merge_outputs(units[u]);
   *nload_max = 0;
   for (int u = 0; u < count; ++u)
     if (units[u].nload > *nload_max) *nload_max = units[u].nload;
