@@ -353,6 +353,15 @@ rcabeam_status rcabeam_voxel_order_workspace_bytes(size_t nv, size_t* bytes);
 rcabeam_status rcabeam_voxel_order_device(const float* scan, size_t nv, unsigned* order, void* workspace,
                                           size_t workspace_bytes);
 
+/* Blocking copy between pageable host memory and the device (upload: host to
+ * device) by up to eight host threads through caller-provided pinned staging
+ * (extension; rcabeam_host_staging_bytes gives the useful size, at least two 2 MiB
+ * buffers).  The copy runs on streams of its own: work that still uses `device`
+ * must have finished, and staging is free again on return. */
+rcabeam_status rcabeam_host_staging_bytes(size_t bytes, size_t* staging);
+rcabeam_status rcabeam_host_copy(void* host, void* device, size_t bytes, int upload, void* staging,
+                                 size_t staging_bytes);
+
 /* Failure-path self-test of the bounded waits (extension; no counterpart in the
  * reference): one CTA of four warps waits, limit_ns at most (<= 2 s), on an
  * mbarrier that nothing arrives on, with the same wait routine as the

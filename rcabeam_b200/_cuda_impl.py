@@ -21,6 +21,8 @@ from rcabeam_b200 import _lib
 _COMPLEX64 = (np.complex64, torch.complex64)
 # Device scratch for the St-SW correlation series of one voxel tile.
 _STSW_SCRATCH_BYTES = 256 << 20
+# Host arrays from this size on cross through pinned staging and several host threads.
+_STAGED_COPY_BYTES = 4 << 20
 
 
 def _ptr(t: torch.Tensor | None) -> int | None:
@@ -33,12 +35,39 @@ def _device() -> torch.device:
     return torch.device("cuda", torch.cuda.current_device())
 
 
+def _host_copy(host: np.ndarray, device: torch.Tensor, upload: bool) -> None:
+    """Blocking copy of a contiguous host array to or from a device tensor of the same bytes.
+
+    The pinned staging (at most 32 MiB) comes from torch's caching host allocator, so repeated
+    calls reuse it and it is returned to that cache.
+    """
+    size = ctypes.c_size_t(0)
+    _lib.check(_lib.lib().rcabeam_host_staging_bytes(host.nbytes, ctypes.byref(size)), "host_staging_bytes")
+    staging = torch.empty(int(size.value), dtype=torch.uint8, pin_memory=True)
+    # The copy has streams of its own; the memory may still be in use on the current one.
+    torch.cuda.current_stream(device.device).synchronize()
+    _lib.call("rcabeam_host_copy", host.ctypes.data, device.data_ptr(), host.nbytes, int(upload), staging.data_ptr(),
+              staging.numel())
+
+
+def _download(device: torch.Tensor, host: np.ndarray) -> None:
+    """Device tensor into a host array of the same shape (the device's work is complete)."""
+    if host.flags.c_contiguous and host.flags.writeable and host.nbytes >= _STAGED_COPY_BYTES:
+        _host_copy(host, device, False)
+    else:
+        np.copyto(host, device.cpu().numpy())
+
+
 def _to_device(a, dtype: torch.dtype) -> torch.Tensor:
     if isinstance(a, torch.Tensor):
         if not a.is_cuda:
             return a.to(_device(), dtype=dtype, non_blocking=False).contiguous()
         return a.to(dtype=dtype).contiguous()
     arr = np.ascontiguousarray(a)
+    if arr.nbytes >= _STAGED_COPY_BYTES and dtype == torch.complex64 and arr.dtype == np.complex64:
+        out = torch.empty(arr.shape, dtype=dtype, device=_device())
+        _host_copy(arr, out, True)
+        return out
     if not arr.flags.writeable:
         arr = arr.copy()
     return torch.from_numpy(arr).to(_device(), dtype=dtype)
@@ -164,9 +193,9 @@ def ensemble_from_channels(rc, cr, scan, xe, ye, angles, starts, pd, signal, wei
     if _lib.device_error():
         raise _lib.RcabeamCudaError("a reconstruction kernel timed out waiting on its staging pipeline")
     if host_pd:
-        np.copyto(np.asarray(pd).reshape(nv, 2), d_pd.cpu().numpy())
+        _download(d_pd, np.asarray(pd).reshape(nv, 2))
     if host_sig:
-        np.copyto(np.asarray(signal).reshape(nv * planes, nt), d_sig.cpu().numpy())
+        _download(d_sig, np.asarray(signal).reshape(nv * planes, nt))
     return upload
 
 

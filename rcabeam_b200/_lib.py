@@ -55,6 +55,8 @@ SIGNATURES: dict[str, list] = {
     "rcabeam_simulate_scene_device": [P, Z, P, P, P, P, Z, Z, Z, Z, I, D, D, D, D, D, D],
     "rcabeam_voxel_order_workspace_bytes": [Z, ctypes.POINTER(c_size_t)],
     "rcabeam_voxel_order_device": [P, Z, P, P, Z],
+    "rcabeam_host_staging_bytes": [Z, ctypes.POINTER(c_size_t)],
+    "rcabeam_host_copy": [P, P, Z, I, P, Z],
     "rcabeam_wait_selftest_device": [ctypes.c_ulonglong, I, P],
     "rcabeam_device_error": [ctypes.POINTER(c_int)],
 }

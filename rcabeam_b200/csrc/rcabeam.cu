@@ -23,6 +23,7 @@
 #include "das_tc.cuh"
 #include "gram_f64.cuh"
 #include "gram_tc.cuh"
+#include "host_copy.cuh"
 #include "pack.cuh"
 #include "scene.cuh"
 
@@ -1016,6 +1017,24 @@ rcabeam_status rcabeam_ensemble_static_device(const void* rc, const void* cr, co
                                               float c, float fs, float fd, float fn, int method) {
   return ensemble_static(rc, cr, scan, xe, ye, angles, starts, pd, signal, ns, nc, na, nt, nv, c, fs, fd, fn,
                          method);
+}
+
+rcabeam_status rcabeam_host_staging_bytes(size_t bytes, size_t* staging) {
+  if (!staging) return RCABEAM_ERROR_ARGUMENT;
+  const size_t chunks = (bytes + host::kChunk - 1) / host::kChunk;
+  *staging = std::min<size_t>(chunks, host::kMaxThreads) * 2 * host::kChunk;
+  return RCABEAM_SUCCESS;
+}
+
+rcabeam_status rcabeam_host_copy(void* host, void* device, size_t bytes, int upload, void* staging,
+                                 size_t staging_bytes) {
+  if (!host || !device || !bytes || !staging || staging_bytes < 2 * host::kChunk) return RCABEAM_ERROR_ARGUMENT;
+  try {
+    return host::copy(host, device, bytes, upload != 0, staging, staging_bytes) ? RCABEAM_SUCCESS
+                                                                                : RCABEAM_ERROR_CUDA;
+  } catch (...) {  // out of host memory: nothing may leave a C entry point
+    return RCABEAM_ERROR_CUDA;
+  }
 }
 
 rcabeam_status rcabeam_wait_selftest_device(unsigned long long limit_ns, int code, int* gave_up) {

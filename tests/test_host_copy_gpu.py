@@ -1,0 +1,49 @@
+"""Staged host copies (rcabeam_host_copy): chunk and thread remainders, read-only sources, concurrent callers."""
+
+from __future__ import annotations
+
+import threading
+
+import numpy as np
+import pytest
+import torch
+
+from rcabeam_b200 import _cuda_impl
+
+pytestmark = pytest.mark.gpu
+CHUNK = 2 << 20
+
+
+@pytest.fixture(autouse=True)
+def _cuda():
+    if not torch.cuda.is_available():
+        pytest.skip("needs CUDA")
+
+
+@pytest.mark.parametrize("nbytes", [8, CHUNK - 8, CHUNK, CHUNK + 8, 16 * CHUNK, 16 * CHUNK + 8, 37 * CHUNK - 16])
+def test_round_trip_is_exact(nbytes):
+    host = np.random.default_rng(nbytes).integers(0, 255, nbytes, dtype=np.uint8)
+    host.flags.writeable = False
+    device = torch.empty(nbytes, dtype=torch.uint8, device="cuda")
+    _cuda_impl._host_copy(host, device, True)
+    assert np.array_equal(device.cpu().numpy(), host)
+    back = np.zeros(nbytes, np.uint8)
+    _cuda_impl._host_copy(back, device, False)
+    assert np.array_equal(back, host)
+
+
+def test_concurrent_uploads_from_two_threads():
+    arrays = [np.random.default_rng(i).standard_normal((1 << 20) + i).astype(np.complex64) for i in range(2)]
+    out = [None, None]
+
+    def work(i):
+        for _ in range(3):
+            out[i] = _cuda_impl._to_device(arrays[i], torch.complex64)
+
+    threads = [threading.Thread(target=work, args=(i,)) for i in range(2)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    for a, d in zip(arrays, out):
+        assert np.array_equal(d.cpu().numpy(), a)
