@@ -1,6 +1,5 @@
-// St-SW (method 4) of the frame-batched path and the per-frame entry points of
-// the reference's single-frame API (core.cu).  One warp owns one voxel; lanes
-// own frames.
+// The pair sums of St-SW (method 4) and the per-frame entry points of the
+// reference's single-frame API (core.cu).
 #pragma once
 
 #include "common.cuh"
@@ -9,10 +8,6 @@
 namespace rcb {
 namespace generic {
 
-// One register frame per lane: these warp-per-voxel kernels are bound by the
-// latency of their per-frame gathers, so resident warps matter more than the
-// taps each 32-frame block re-forms (St-SW, k = 2: 205 ms at 4 frames, 97 ms at 1).
-constexpr int kRegFrames = 1;
 constexpr int kWarps = 4;
 
 struct Voxel {
@@ -33,37 +28,6 @@ __device__ __forceinline__ Tap tap_of(const Voxel& q, int config, const float* e
   return make_tap(__dadd_rn(ttx, trx), double(starts[a]), fs, fd, ns, act);
 }
 
-// Interpolated, rotated sample of a packed (c, a, s, t) complex64 ensemble.
-__device__ __forceinline__ float2 packed_sample(const float2* iq, const Tap& t, int ch, int a, int frame, int ns,
-                                                int na, int nt) {
-  if (t.i0 < 0 || frame >= nt) return make_float2(0.f, 0.f);
-  size_t idx = ((size_t(ch) * na + a) * ns + size_t(t.i0)) * nt + frame;
-  size_t nxt = t.i0 == ns - 1 ? idx : idx + nt;
-  float2 va = iq[idx], vb = iq[nxt];
-  float2 val = make_float2(fmaf(t.w, vb.x - va.x, va.x), fmaf(t.w, vb.y - va.y, va.y));
-  return cmul(val, t.phase);
-}
-
-// Transmit delays of a voxel for one angle (RC transmits along y, CR along x),
-// formed once per angle with the float64 operations of tap_of.
-struct AngleTx {
-  double rc, cr, start;
-};
-__device__ __forceinline__ AngleTx angle_tx(const das::Args& p, const Voxel& q, int a) {
-  const double th = double(p.angles[a]), cs = cos(th), sn = sin(th);
-  return AngleTx{transmit_delay(q.y, q.z, cs, sn, p.c), transmit_delay(q.x, q.z, cs, sn, p.c), double(p.starts[a])};
-}
-
-// Tap of channel c0 + lane for one aperture (empty beyond nc): tap_of's float64
-// operations with the angle's transmit delay precomputed (identical taps).
-__device__ __forceinline__ Tap lane_tap_tx(const das::Args& p, const Voxel& q, int config, int c0, const AngleTx& tx) {
-  const int ch = c0 + int(threadIdx.x & 31);
-  if (ch >= p.nc) return Tap{-1, 0.f, make_float2(0.f, 0.f)};
-  bool act;
-  const double trx = receive_delay(config ? q.y : q.x, q.z, double((config ? p.ye : p.xe)[ch]), p.c, p.fn, &act);
-  return make_tap(__dadd_rn(config ? tx.cr : tx.rc, trx), tx.start, p.fs, p.fd, p.ns, act);
-}
-
 // ------------------------------------------------------------ St-SW --
 // St-SW (method 4; reference stsw.py:10-107, ensemble.cu:457-627).  Angles of
 // each aperture fall into K interleaved subsets (a % K).  Per frame: the
@@ -73,103 +37,10 @@ __device__ __forceinline__ Tap lane_tap_tx(const das::Args& p, const Voxel& q, i
 // weight |sum over (i1 < i2, j1 != j2) of sum_t c1 conj(c2) / sqrt(E1 E2)| with
 // E the series energies; the power is the XDoppler |mean_t r conj(q)|.
 //
-// Pass 1 (one warp per voxel, lanes over frames): per-angle channel sums in
-// angle-major order with the taps broadcast as for RC-FMAS, Welford updates of
-// the subset statistics (no E|x|^2 - |E x|^2 cancellation), the series written
-// to the caller's workspace (v K^2 + i K + j) nt + t and r conj(q) summed into
-// pd[2v], pd[2v + 1].
-template <int K, int RF>
-__global__ void __launch_bounds__(kWarps * 32) stsw_series(das::Args p, float2* series) {
-  const size_t v = size_t(blockIdx.x) * kWarps + (threadIdx.x >> 5);
-  if (v >= size_t(p.nv)) return;
-  const int lane = threadIdx.x & 31;
-  const int fbase = blockIdx.y * 32 * RF + lane;
-  const Voxel q = load_voxel(p.scan, v);
-  const float2* rc = static_cast<const float2*>(p.rc);
-  const float2* cr = static_cast<const float2*>(p.cr);
-  __shared__ __align__(16) Tap taps[kWarps][2][32];
-  Tap* tap_rc = taps[threadIdx.x >> 5][0];
-  Tap* tap_cr = taps[threadIdx.x >> 5][1];
-  float2 r[RF] = {}, s[RF] = {};
-  float2 mr[K][RF] = {}, mq[K][RF] = {};
-  float vr[K][RF] = {}, vq[K][RF] = {};
-  for (int a = 0; a < p.na; ++a) {
-    float2 ar[RF] = {}, aq[RF] = {};
-    const AngleTx tx = angle_tx(p, q, a);  // the voxel's transmit delays, once per angle
-    for (int c0 = 0; c0 < p.nc; c0 += 32) {
-      // Each lane forms one channel's taps; the warp then reads them back from
-      // shared memory (one broadcast 16-byte load per tap instead of four shuffles).
-      __syncwarp();  // the previous chunk's reads are done
-      tap_rc[lane] = lane_tap_tx(p, q, 0, c0, tx);
-      tap_cr[lane] = lane_tap_tx(p, q, 1, c0, tx);
-      __syncwarp();
-      const int count = min(32, p.nc - c0);
-      for (int j = 0; j < count; ++j) {
-        const int ch = c0 + j;
-        const Tap tr = tap_rc[j], tq = tap_cr[j];
-#pragma unroll
-        for (int f = 0; f < RF; ++f) {
-          const int frame = fbase + 32 * f;
-          ar[f] = cadd(ar[f], packed_sample(rc, tr, ch, a, frame, p.ns, p.na, p.nt));
-          aq[f] = cadd(aq[f], packed_sample(cr, tq, ch, a, frame, p.ns, p.na, p.nt));
-        }
-      }
-    }
-    // Welford update of subset a % K, whose (a / K + 1)-th angle this is.
-    const int subset = a % K;
-    const float inv = 1.0f / float(a / K + 1);
-#pragma unroll
-    for (int f = 0; f < RF; ++f) {
-      r[f] = cadd(r[f], ar[f]);
-      s[f] = cadd(s[f], aq[f]);
-#pragma unroll
-      for (int i = 0; i < K; ++i) {
-        if (i != subset) continue;
-        const float2 dr = make_float2(ar[f].x - mr[i][f].x, ar[f].y - mr[i][f].y);
-        const float2 dq = make_float2(aq[f].x - mq[i][f].x, aq[f].y - mq[i][f].y);
-        mr[i][f] = make_float2(fmaf(dr.x, inv, mr[i][f].x), fmaf(dr.y, inv, mr[i][f].y));
-        mq[i][f] = make_float2(fmaf(dq.x, inv, mq[i][f].x), fmaf(dq.y, inv, mq[i][f].y));
-        vr[i][f] += dr.x * (ar[f].x - mr[i][f].x) + dr.y * (ar[f].y - mr[i][f].y);
-        vq[i][f] += dq.x * (aq[f].x - mq[i][f].x) + dq.y * (aq[f].y - mq[i][f].y);
-      }
-    }
-  }
-  float cross_re = 0.f, cross_im = 0.f;
-#pragma unroll
-  for (int f = 0; f < RF; ++f) {
-    const int frame = fbase + 32 * f;
-    if (frame >= p.nt) continue;
-    const float2 x = cmul(r[f], cconj(s[f]));
-    cross_re += x.x;
-    cross_im += x.y;
-#pragma unroll
-    for (int i = 0; i < K; ++i) {
-      // Subset i holds the angles i, i + K, ... < na.
-      const float count = float((p.na - 1 - i) / K + 1);
-#pragma unroll
-      for (int j = 0; j < K; ++j) {
-        const float countq = float((p.na - 1 - j) / K + 1);
-        const float2 num = cmul(mr[i][f], cconj(mq[j][f]));
-        const float den = cabs2(mr[i][f]) + cabs2(mq[j][f]) + (vr[i][f] / count + vq[j][f] / countq) * 0.5f -
-                          hypotf(num.x, num.y);
-        float2 value = den > 0.f ? make_float2(num.x / den, num.y / den) : make_float2(0.f, 0.f);
-        if (!isfinite(value.x) || !isfinite(value.y)) value = make_float2(0.f, 0.f);
-        series[(v * (K * K) + size_t(i * K + j)) * size_t(p.nt) + size_t(frame)] = value;
-      }
-    }
-  }
-#pragma unroll
-  for (int off = 16; off > 0; off >>= 1) {
-    cross_re += __shfl_xor_sync(0xffffffffu, cross_re, off);
-    cross_im += __shfl_xor_sync(0xffffffffu, cross_im, off);
-  }
-  if (lane == 0) {
-    atomicAdd(p.pd + 2 * v, cross_re / float(p.nt));
-    atomicAdd(p.pd + 2 * v + 1, cross_im / float(p.nt));
-  }
-}
-
-// Pass 2 (one warp per voxel): series energies over frames, then the pair sum
+// The series come from the staged kernel (das_rows.cuh), whose angles run subset by
+// subset; it also sums r conj(q) into pd[2v], pd[2v + 1].
+//
+// stsw_finish (one warp per voxel): series energies over frames, then the pair sum
 // with running row / column sums of the normalized series (for row i, the
 // earlier rows' total minus their column j pairs with c[i][j]), the raw weight
 // |acc| and the XDoppler magnitude in pd[2v].

@@ -1,6 +1,6 @@
 // Frame-batched RCA delay-and-sum on the CUDA cores (float32 arithmetic, exact
-// geometry): OPW, XDoppler, separate apertures, RC-FMAS and DMAS-CCF-ACF from one
-// staged pipeline.  The reference does the same arithmetic per sample from a
+// geometry): OPW, XDoppler, separate apertures, RC-FMAS, DMAS-CCF-ACF and the
+// subset statistics of St-SW from one staged pipeline.  The reference does the same arithmetic per sample from a
 // per-call geometry table (ensemble.cu:143-454).
 //
 // Work: an item is a tile of 128 voxels (consecutive in a spatially compact
@@ -50,7 +50,10 @@ constexpr int kMaxBuilders = 4;
 constexpr int kMaxGroups = 8;              // frame groups of an item
 constexpr int kBoxRows = 8;                // sample rows of one TMA box
 
-enum Mode : int { kOpw = 0, kXdoppler = 1, kFmas = 2, kDmas = 3, kApertures = 5 };
+// St-SW (method 4) with K angle subsets is kStsw + K.
+enum Mode : int { kOpw = 0, kXdoppler = 1, kFmas = 2, kDmas = 3, kApertures = 5, kStsw = 8 };
+template <int MODE>
+constexpr int kSubsets = MODE > kStsw ? MODE - kStsw : 0;
 // Stage tags: the run a step belongs to and whether another window of the same
 // step follows; or the end of an item.
 constexpr int kTagEnd = -1, kTagMore = 1 << 30, kTagMask = kTagMore - 1;
@@ -70,6 +73,7 @@ struct Args {
   double c, fs, fd, fn;
   int* err;
   const double* offsets;  // [2][nc] receive-delay offsets in seconds (RC, CR), or nullptr
+  float2* series;         // St-SW: (nv, K^2, nt) correlation series
 };
 
 // Packed (slab, sample, frame) channels of both apertures as TMA tensors.
@@ -519,12 +523,13 @@ struct Builder {
     }
   }
 
-  // Both apertures, angle by angle; tag = aperture * na + angle.
-  __device__ __forceinline__ void walk_angles() {
+  // Both apertures, angle by angle (subset by subset: angles s, s + subsets, ...);
+  // tag = aperture * na + angle.
+  __device__ __forceinline__ void walk_angles(int subsets) {
     for (int cfg = 0; cfg < 2; ++cfg) {
       fill_table(cfg);
       const float* el = cfg ? p.ye : p.xe;
-      for (int a = 0; a < p.na; ++a) {
+      for (int i = 0, a = 0; i < p.na; ++i) {
         for (int ch = 0; ch < p.nc && ok; ++ch) {
           if (!reachable(cfg, ch)) continue;
           if (turn-- > 0) continue;
@@ -536,6 +541,8 @@ struct Builder {
           for (int j = 0; j < 4; ++j) receive(cfg, lane + 32 * j, e, extra, &rx[j], &rxc[j]);
           emit(cfg, ch, a, cfg * p.na + a, rx, rxc);
         }
+        a += subsets;
+        if (a >= p.na) a = a % subsets + 1;  // the next subset's first angle
       }
     }
   }
@@ -543,9 +550,11 @@ struct Builder {
   template <int MODE>
   __device__ __forceinline__ void walk() {
     if constexpr (MODE == kFmas) {
-      walk_angles();
+      walk_angles(1);
+    } else if constexpr (kSubsets<MODE> > 0) {
+      walk_angles(kSubsets<MODE>);
     } else if constexpr (MODE == kDmas) {
-      walk_angles();
+      walk_angles(1);
       walk_channels(2 * p.na);
     } else {
       walk_channels(0);
@@ -656,7 +665,11 @@ __device__ __forceinline__ void add_step(float4 (&acc)[PAIRS], const float4& tap
 
 // Floats per voxel and frame that a thread keeps in shared memory (its own).
 template <int MODE>
-constexpr int kStash = MODE == kOpw ? 0 : MODE == kFmas ? 4 : MODE == kDmas ? 5 : 2;
+constexpr int kStash = MODE == kOpw ? 0 : MODE == kFmas || MODE > kStsw ? 4 : MODE == kDmas ? 5 : 2;
+
+// Methods whose power is the mean of a complex product.
+template <int MODE>
+constexpr bool kCross = MODE == kXdoppler || MODE > kStsw;
 
 // Threads of a CTA: 16 consumer warps and 3 builders at 96 registers fill an SM;
 // OPW of few frames takes 80 registers and shares the SM with other CTAs.
@@ -680,7 +693,7 @@ struct Consumer {
   const Shared& sh;
   const Ring ring;
   int first, slot, group, thread, count;
-  int state;  // DMAS: 0 RC angles, 1 CR angles, 2 channels
+  int state;  // DMAS: 0 RC angles, 1 CR angles, 2 channels; St-SW: aperture * K + subset
   float4 acc[PAIRS];
 
   __device__ __forceinline__ Consumer(const Args& p_, const Shape& sp_, const Layout& lt_, const Shared& sh_,
@@ -734,12 +747,47 @@ struct Consumer {
     }
   }
 
+  // St-SW: float f of a voxel-frame's subset statistics (aperture, subset: mean,
+  // mean squared deviation) is kept where its correlation series goes later, in
+  // the caller's workspace of 2 K^2 floats; those beyond (K = 2 has 12) in slot 3.
+  static constexpr int K = kSubsets<MODE>;
+  __device__ __forceinline__ float& statistic(unsigned v, int f, int k) const {
+    if (K == 2 && f == 8) return stash(3, k);
+    float2& q = p.series[(size_t(v) * (K * K) + size_t(f / 2)) * size_t(p.nt) + size_t(first + k)];
+    return f & 1 ? q.y : q.x;
+  }
+
+  // Ends the current subset (slots 0-2) of `angles` angles.  The last one of K = 2
+  // stays in its slots.
+  __device__ __forceinline__ void close_subset(int index, int angles) {
+    const unsigned v = sh.vox[slot];
+    const int frames = v == UINT_MAX || group >= sp.groups ? 0 : min(2 * sp.pairs, p.nt - first);
+    for (int k = 0; k < 2 * sp.pairs; ++k) {
+      stash(2, k) = stash(2, k) / float(angles);
+      if (K == 2 && index == 2 * K - 1) continue;
+      if (k < frames)
+        for (int f = 0; f < 3; ++f) statistic(v, 3 * index + f, k) = stash(f, k);
+      for (int f = 0; f < 3; ++f) stash(f, k) = 0.f;
+    }
+  }
+
+  // Angles of subset i: i, i + K, ... < na.
+  __device__ __forceinline__ int subset_angles(int i) const { return (p.na - 1 - i) / K + 1; }
+
   // Ends a run of steps of one tag.
   __device__ __forceinline__ void fold(int tag) {
     if constexpr (MODE == kXdoppler || MODE == kApertures) {
       if (tag != 0) return;
     }
     if constexpr (MODE == kDmas) advance(tag < p.na ? 0 : tag < 2 * p.na ? 1 : 2);
+    float inv = 1.f;
+    if constexpr (K > 0) {
+      const int a = tag % p.na, index = tag / p.na * K + a % K;
+      for (; state < index; ++state) close_subset(state, subset_angles(state % K));
+      // The angle's place in its subset; angles that no voxel of the tile sees are
+      // zero sums that still count.
+      inv = 1.0f / float(a / K + 1);
+    }
 #pragma unroll
     for (int k = 0; k < kFrames; ++k) {
       if (k % 4 == 0 && k >= 2 * sp.pairs) break;
@@ -750,6 +798,12 @@ struct Consumer {
       } else if constexpr (MODE == kFmas) {
         const int s = tag < p.na ? 0 : 2;
         store(s, k, cadd(load(s, k), csroot(v)));
+      } else if constexpr (K > 0) {
+        // Welford's update (no E|x|^2 - |E x|^2 cancellation).
+        const float2 m = load(0, k), d = make_float2(v.x - m.x, v.y - m.y);
+        const float2 now = make_float2(fmaf(d.x, inv, m.x), fmaf(d.y, inv, m.y));
+        store(0, k, now);
+        stash(2, k) += d.x * (v.x - now.x) + d.y * (v.y - now.y);
       } else if constexpr (MODE == kDmas) {
         if (state == 2) {
           store(1, k, cadd(load(1, k), csroot(v)));
@@ -808,6 +862,8 @@ struct Consumer {
     if constexpr (MODE != kOpw)
       if (open >= 0) fold(open);
     if constexpr (MODE == kDmas) advance(2);
+    if constexpr (K > 0)
+      for (; state < 2 * K; ++state) close_subset(state, subset_angles(state % K));
     return true;
   }
 
@@ -836,6 +892,10 @@ struct Consumer {
         const float2 val = cmul(load(0, k), load(2, k));
         if (p.signal) p.signal[at] = val;
         pr += cabs2(val);
+      } else if constexpr (K > 0) {
+        const float2 val = write_series(v, k);
+        pr += val.x;
+        pi += val.y;
       } else {
         const float mag = stash(3, k), act = sh.active[slot];
         const float dm = cabs2(load(1, k)) - mag;
@@ -847,7 +907,44 @@ struct Consumer {
       }
     }
     sh.power[group * kTileVoxels + slot] = pr;
-    if constexpr (MODE == kXdoppler) sh.power[(kMaxGroups + group) * kTileVoxels + slot] = pi;
+    if constexpr (kCross<MODE>) sh.power[(kMaxGroups + group) * kTileVoxels + slot] = pi;
+  }
+
+  // St-SW: the K x K correlation series of one frame from its subset statistics
+  // (reference stsw.py:45-66); returns r conj(q) of the aperture sums.
+  __device__ __forceinline__ float2 write_series(unsigned v, int k) {
+    float2 mean[2][K > 0 ? K : 1], sum[2];
+    float spread[2][K > 0 ? K : 1];
+#pragma unroll
+    for (int ap = 0; ap < 2; ++ap) {
+      sum[ap] = make_float2(0.f, 0.f);
+#pragma unroll
+      for (int i = 0; i < K; ++i) {
+        const int index = ap * K + i;
+        if (K == 2 && index == 2 * K - 1) {
+          mean[ap][i] = load(0, k);
+          spread[ap][i] = stash(2, k);
+        } else {
+          mean[ap][i] = make_float2(statistic(v, 3 * index, k), statistic(v, 3 * index + 1, k));
+          spread[ap][i] = statistic(v, 3 * index + 2, k);
+        }
+        const float n = float(subset_angles(i));
+        sum[ap] = make_float2(fmaf(n, mean[ap][i].x, sum[ap].x), fmaf(n, mean[ap][i].y, sum[ap].y));
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < K; ++i) {
+#pragma unroll
+      for (int j = 0; j < K; ++j) {
+        const float2 num = cmul(mean[0][i], cconj(mean[1][j]));
+        const float den = cabs2(mean[0][i]) + cabs2(mean[1][j]) + (spread[0][i] + spread[1][j]) * 0.5f -
+                          hypotf(num.x, num.y);
+        float2 value = den > 0.f ? make_float2(num.x / den, num.y / den) : make_float2(0.f, 0.f);
+        if (!isfinite(value.x) || !isfinite(value.y)) value = make_float2(0.f, 0.f);
+        p.series[(size_t(v) * (K * K) + size_t(i * K + j)) * size_t(p.nt) + size_t(first + k)] = value;
+      }
+    }
+    return cmul(sum[0], cconj(sum[1]));
   }
 };
 
@@ -892,10 +989,10 @@ __device__ __forceinline__ bool run_item(const Args& p, const Shape& sp, const L
       float re = 0.f, im = 0.f;
       for (int g = 0; g < sp.groups; ++g) {
         re += sh.power[g * kTileVoxels + i];
-        if constexpr (MODE == kXdoppler) im += sh.power[(kMaxGroups + g) * kTileVoxels + i];
+        if constexpr (kCross<MODE>) im += sh.power[(kMaxGroups + g) * kTileVoxels + i];
       }
       atomicAdd(p.pd + 2 * size_t(v), re * inv_nt);
-      if constexpr (MODE == kXdoppler) atomicAdd(p.pd + 2 * size_t(v) + 1, im * inv_nt);
+      if constexpr (kCross<MODE>) atomicAdd(p.pd + 2 * size_t(v) + 1, im * inv_nt);
     }
   }
   return ok;

@@ -171,6 +171,8 @@ static const unsigned* voxel_order(const float* scan, size_t nv, void* workspace
 }
 
 // ---------------------------------------------------------- dispatch --
+static unsigned blocks_for(size_t n, unsigned threads) { return unsigned((n + threads - 1) / threads); }
+
 static int sm_count() {
   int dev = 0, sms = 148;
   cudaGetDevice(&dev);
@@ -495,27 +497,21 @@ static rcabeam_status ensemble_impl(const void* rc, const void* cr, const float*
   a.fd = double(fd);
   a.fn = double(fn);
   a.err = device_error_ptr();
+  // The caller owns 2 * nv * (nc + na) float4 of scratch (reference rcabeam.h:196).
+  a.order = voxel_order(scan, nv, geometry_workspace, 2 * nv * (nc + na) * 16);
   if (method == 4) {
     // St-SW: series into the caller's workspace (nv k^2 nt complex64), then
     // energies, pair sums, raw weights and the XDoppler magnitude.
-    constexpr int kStswFrames = generic::kRegFrames;
-    const unsigned blocks = unsigned((nv + generic::kWarps - 1) / generic::kWarps);
-    dim3 grid(blocks, unsigned((nt + 32 * kStswFrames - 1) / (32 * kStswFrames)));
-    float2* series = static_cast<float2*>(workspace);
-    if (k == 2) {
-      generic::stsw_series<2, kStswFrames><<<grid, generic::kWarps * 32>>>(a, series);
-      generic::stsw_finish<2><<<blocks, generic::kWarps * 32>>>(pd, weights, series, nv, int(nt));
-    } else if (k == 3) {
-      generic::stsw_series<3, kStswFrames><<<grid, generic::kWarps * 32>>>(a, series);
-      generic::stsw_finish<3><<<blocks, generic::kWarps * 32>>>(pd, weights, series, nv, int(nt));
-    } else {
-      generic::stsw_series<4, kStswFrames><<<grid, generic::kWarps * 32>>>(a, series);
-      generic::stsw_finish<4><<<blocks, generic::kWarps * 32>>>(pd, weights, series, nv, int(nt));
-    }
+    a.series = static_cast<float2*>(workspace);
+    const rcabeam_status st = k == 2   ? run_rows<das::kStsw + 2, false>(a)
+                              : k == 3 ? run_rows<das::kStsw + 3, false>(a)
+                                       : run_rows<das::kStsw + 4, false>(a);
+    if (st != RCABEAM_SUCCESS) return st;
+    const unsigned blocks = blocks_for(nv, generic::kWarps);
+    auto finish = k == 2 ? generic::stsw_finish<2> : k == 3 ? generic::stsw_finish<3> : generic::stsw_finish<4>;
+    finish<<<blocks, generic::kWarps * 32>>>(pd, weights, a.series, nv, int(nt));
     return launch_status();
   }
-  // The caller owns 2 * nv * (nc + na) float4 of scratch (reference rcabeam.h:196).
-  a.order = voxel_order(scan, nv, geometry_workspace, 2 * nv * (nc + na) * 16);
   const void* planes[2] = {rc, cr};
   if (HALF && tc_eligible(planes, 2, nt) && nv <= size_t(INT32_MAX) - tc::kVox && tc_smem_bytes(false, nt, na, 2)) {
     tc::Args t{};
@@ -573,8 +569,6 @@ static bool bad_frame_args(const void* iq, const float* scan, const float* el, c
   return !iq || !scan || !el || !angles || !starts || !out || ns < 2 || !nc || !na || !nv ||
          (config != 0 && config != 1) || ns > INT32_MAX || nc > INT32_MAX || na > INT32_MAX;
 }
-
-static unsigned blocks_for(size_t n, unsigned threads) { return unsigned((n + threads - 1) / threads); }
 
 // One cuSOLVER handle per device, bound to the legacy default stream.
 static cusolverDnHandle_t solver_handle() {
