@@ -46,7 +46,7 @@ template <int MODE>
 __device__ __forceinline__ bool item_of(const Ensemble& e, const das::Args& args, const das::Shape& sp,
                                         const Queue& q, const das::Shared& sh, int tile, int chunk, uint32_t& phase) {
   const CUtensorMap* maps = e.maps.map;
-  if constexpr (MODE == das::kOpw) {
+  if constexpr (MODE != das::kDmas) {
     if (e.width > 8)
       return sp.boxes ? das::run_item<MODE, 13, false, true>(args, sp, q.layout, sh, maps, tile, chunk, phase)
                       : das::run_item<MODE, 13, false, false>(args, sp, q.layout, sh, maps, tile, chunk, phase);

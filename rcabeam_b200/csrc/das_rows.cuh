@@ -1,18 +1,21 @@
 // Frame-batched RCA delay-and-sum on the CUDA cores (float32 arithmetic, exact
 // geometry): OPW, XDoppler, separate apertures, RC-FMAS, DMAS-CCF-ACF and the
-// subset statistics of St-SW from one staged pipeline.  The reference does the same arithmetic per sample from a
-// per-call geometry table (ensemble.cu:143-454).
+// subset statistics of St-SW from one staged pipeline.  The reference does the same
+// arithmetic per sample from a per-call geometry table (ensemble.cu:143-454).
 //
 // Work: an item is a tile of 128 voxels (consecutive in a spatially compact
 // order) x a chunk of up to 104 frames; a CTA runs one.  Its steps are the
 // (aperture, channel, angle) triples; for each, the tile's interpolation taps fall
 // in a short window of consecutive sample rows.
-//   * Builder warps (3, steps dealt round robin) form a step's taps -- receive
-//     delays once per channel, transmit delays from a per-tile table, both as
-//     fixed-point sample positions that are simply added -- and start the
+//   * Builder warps (3 as a rule, steps dealt round robin) form a step's taps --
+//     receive delays once per channel, transmit delays from a per-tile table, both
+//     as fixed-point sample positions that are simply added -- and start the
 //     window's copy into a ring stage: TMA boxes of 8 rows, or bulk copies of the
 //     rows where odd frame counts or unaligned buffers rule a tensor map out.
 //     Only the rows that taps need are copied.
+//   * Where the walk changes channel with every step, a helper warp per builder
+//     forms its receive delays one step ahead (48 x 96 x 48 voxels, 384 x 128 x 7 x
+//     64, RC-FMAS: 37.6 ms without, 30.7 with).
 //   * Consumer warps own 32 voxels x up to 26 frames each: a lane one voxel, its
 //     frames' sums in registers.  Per step a lane reads its tap once and then both
 //     rows of each frame pair with 16-byte shared-memory loads at immediate
@@ -98,6 +101,7 @@ struct Shape {
 // Shared memory and warps of one launch.
 struct Layout {
   int builders;     // builder warps
+  int helpers;      // warps that form receive delays for them: one each, or none
   int stages;       // ring stages: two per builder
   int stage_bytes;  // taps and rows of one of them
   int zero_bytes;   // a row of zeros: what voxels outside a step read
@@ -118,6 +122,8 @@ struct Shared {
   float* stash;
   uint64_t* full;
   uint64_t* empty;
+  uint64_t* rx_full;      // [2][kMaxBuilders] helpers' receive delays ready, taken
+  uint64_t* rx_empty;
   int2* tag;              // run of the stage's step; voxel blocks with a tap in it (bit per block)
   unsigned* vox;          // voxel ids of the tile
   float* pos;             // [3][128] x, z, y
@@ -126,7 +132,7 @@ struct Shared {
   float* bounds;          // tile minimum and maximum of x and of y, maximum of z, rows a step can span
   double* angle;          // [na][3] cos, sin, start
   double* limit;          // [128] f-number half aperture at the voxel's depth
-  long long* rx;          // [2][kMaxBuilders][128] receive delays of two blocks of channels
+  long long* rx;          // [2][kMaxBuilders][128] receive delays: two blocks of channels, or two steps per builder
   unsigned* rxc;
   long long* tx;          // [na][128] transmit delay minus start, 2^-32 samples
   unsigned* txc;          // [na][128] transmit phase, 2^-32 cycles
@@ -140,7 +146,7 @@ struct Ring {
   int stages, bytes, rows;
 };
 constexpr int kRxEntries = 2 * kMaxBuilders * kTileVoxels;
-constexpr int kFixedBytes = kMaxStages * 24 + kTileVoxels * 4 * (1 + 3 + 2 * kMaxGroups + 1) + 64 + kTileVoxels * 8 + kRxEntries * 12;
+constexpr int kFixedBytes = kMaxStages * 24 + 4 * kMaxBuilders * 8 + kTileVoxels * 4 * (1 + 3 + 2 * kMaxGroups + 1) + 64 + kTileVoxels * 8 + kRxEntries * 12;
 
 __device__ __forceinline__ Shared carve(unsigned char* smem, const Layout& l) {
   Shared s;
@@ -158,7 +164,9 @@ __device__ __forceinline__ Shared carve(unsigned char* smem, const Layout& l) {
   s.rx = reinterpret_cast<long long*>(s.limit + kTileVoxels);
   s.full = reinterpret_cast<uint64_t*>(s.rx + kRxEntries);
   s.empty = s.full + kMaxStages;
-  s.tag = reinterpret_cast<int2*>(s.empty + kMaxStages);
+  s.rx_full = s.empty + kMaxStages;
+  s.rx_empty = s.rx_full + 2 * kMaxBuilders;
+  s.tag = reinterpret_cast<int2*>(s.rx_empty + 2 * kMaxBuilders);
   s.vox = reinterpret_cast<unsigned*>(s.tag + kMaxStages);
   s.pos = reinterpret_cast<float*>(s.vox + kTileVoxels);
   s.power = s.pos + 3 * kTileVoxels;
@@ -265,8 +273,8 @@ struct Builder {
   double ks, kc;    // samples and demodulation cycles per metre
 
   __device__ __forceinline__ Builder(const Args& p_, const Shape& sp_, const Layout& lt_, const Shared& sh_,
-                                     const Ring& ring_, const CUtensorMap* maps_, int f0, uint32_t phase_)
-      : p(p_), sp(sp_), lt(lt_), sh(sh_), ring(ring_), maps(maps_), frame0(f0), warp(threadIdx.x >> 5),
+                                     const Ring& ring_, const CUtensorMap* maps_, int f0, int warp_, uint32_t phase_)
+      : p(p_), sp(sp_), lt(lt_), sh(sh_), ring(ring_), maps(maps_), frame0(f0), warp(warp_),
         lane(threadIdx.x & 31), phase(phase_), ok(true), ks(p_.fs / p_.c), kc(p_.fd / p_.c) {
     turn = stage = warp;  // every item starts at stage 0
   }
@@ -275,15 +283,53 @@ struct Builder {
     asm volatile("bar.sync 1, %0;" ::"r"(lt.builders * 32) : "memory");
   }
 
-  // Receive delay and phase of tile slot i.
-  __device__ __forceinline__ void receive(int cfg, int i, double e, double extra, long long* delay,
-                                          unsigned* cyc) const {
-    const double v = double(sh.pos[(cfg ? 2 : 0) * kTileVoxels + i]), z = double(sh.pos[kTileVoxels + i]);
-    const double d = __dadd_rn(v, -e);
-    const double r = path_root(fma(d, d, z * z));
-    const bool inside = p.fn <= 0.0 || fabs(d) <= sh.limit[i];
-    *delay = inside && sh.vox[i] != UINT_MAX ? fixed32(fma(r, ks, extra * p.fs)) : kNever;
-    *cyc = cycles32(fma(r, kc, extra * p.fd));
+  // Receive delays and phases of this lane's voxels for one channel.
+  __device__ __forceinline__ void receive(int cfg, int ch, long long (&rx)[4], unsigned (&rxc)[4]) const {
+    const double e = double((cfg ? p.ye : p.xe)[ch]), extra = p.offsets ? p.offsets[cfg * p.nc + ch] : 0.0;
+    double s[4], cyc[4], most = 0.0;
+    bool out[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const int i = lane + 32 * j;
+      const double z = double(sh.pos[kTileVoxels + i]);
+      const double d = __dadd_rn(double(sh.pos[(cfg ? 2 : 0) * kTileVoxels + i]), -e);
+      const double r = path_root(fma(d, d, z * z));
+      out[j] = sh.vox[i] == UINT_MAX || (p.fn > 0.0 && !(fabs(d) <= sh.limit[i]));
+      s[j] = fma(r, ks, extra * p.fs);
+      cyc[j] = fma(r, kc, extra * p.fd);
+      most = fmax(most, fabs(s[j]) + fabs(cyc[j]));
+      if (isnan(r)) most = INFINITY;
+    }
+    // One range check for all (fixed32, cycles32).
+    if (__all_sync(0xffffffffu, most < 524288.0)) {
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        rx[j] = __double_as_longlong(s[j] + 1572864.0) - 0x4138000000000000ll;
+        rxc[j] = unsigned(__double_as_longlong(cyc[j] + 1572864.0));
+      }
+    } else {
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        rx[j] = fixed32(s[j]);
+        rxc[j] = cycles32(cyc[j]);
+      }
+    }
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+      if (out[j]) rx[j] = kNever;
+  }
+
+  // The two slots of receive delays between a helper and its builder.
+  __device__ __forceinline__ int rx_at(int s) const { return (s * kMaxBuilders + warp) * kTileVoxels + lane; }
+  __device__ __forceinline__ bool rx_wait(uint64_t* bars, int s, uint32_t flip, int code) {
+    ok = ok && __all_sync(0xffffffffu, mbar_wait_fast(&bars[s * kMaxBuilders + warp], ((phase >> (30 + s)) & 1) ^ flip,
+                                                      p.err, code));
+    phase ^= 1u << (30 + s);
+    return ok;
+  }
+  __device__ __forceinline__ void rx_arrive(uint64_t* bars, int s) const {
+    __syncwarp();
+    if (lane == 0) mbar_arrive(&bars[s * kMaxBuilders + warp]);
   }
 
   // Transmit delay (minus the angle's start) and phase of tile slot i.
@@ -488,16 +534,16 @@ struct Builder {
   __device__ __forceinline__ void walk_channels(int first) {
     for (int cfg = 0; cfg < 2; ++cfg) {
       fill_table(cfg);
-      const float* el = cfg ? p.ye : p.xe;
       int half = 0;
       for (int c0 = 0; c0 < p.nc; c0 += lt.builders, half ^= 1) {
-        const int mine = c0 + warp;
-        if (mine < p.nc) {
-          const double e = double(el[mine]), extra = p.offsets ? p.offsets[cfg * p.nc + mine] : 0.0;
+        if (c0 + warp < p.nc) {
+          long long rx[4];
+          unsigned rxc[4];
+          receive(cfg, c0 + warp, rx, rxc);
 #pragma unroll
           for (int j = 0; j < 4; ++j) {
-            const int i = lane + 32 * j, at = (half * kMaxBuilders + warp) * kTileVoxels + i;
-            receive(cfg, i, e, extra, sh.rx + at, sh.rxc + at);
+            sh.rx[rx_at(half) + 32 * j] = rx[j];
+            sh.rxc[rx_at(half) + 32 * j] = rxc[j];
           }
         }
         sync_builders();
@@ -524,22 +570,40 @@ struct Builder {
   }
 
   // Both apertures, angle by angle (subset by subset: angles s, s + subsets, ...);
-  // tag = aperture * na + angle.
+  // tag = aperture * na + angle.  The channel changes with every step, so a helper
+  // warp forms the receive delays of its builder's next step meanwhile.
+  template <bool HELPER>
   __device__ __forceinline__ void walk_angles(int subsets) {
+    int s = 0;
     for (int cfg = 0; cfg < 2; ++cfg) {
-      fill_table(cfg);
-      const float* el = cfg ? p.ye : p.xe;
+      if constexpr (!HELPER) fill_table(cfg);
       for (int i = 0, a = 0; i < p.na; ++i) {
         for (int ch = 0; ch < p.nc && ok; ++ch) {
           if (!reachable(cfg, ch)) continue;
           if (turn-- > 0) continue;
           turn = lt.builders - 1;
-          const double e = double(el[ch]), extra = p.offsets ? p.offsets[cfg * p.nc + ch] : 0.0;
           long long rx[4];
           unsigned rxc[4];
+          if constexpr (HELPER) {
+            if (!rx_wait(sh.rx_empty, s, 1, kErrWaitEmpty)) continue;
+            receive(cfg, ch, rx, rxc);
 #pragma unroll
-          for (int j = 0; j < 4; ++j) receive(cfg, lane + 32 * j, e, extra, &rx[j], &rxc[j]);
-          emit(cfg, ch, a, cfg * p.na + a, rx, rxc);
+            for (int j = 0; j < 4; ++j) {
+              sh.rx[rx_at(s) + 32 * j] = rx[j];
+              sh.rxc[rx_at(s) + 32 * j] = rxc[j];
+            }
+            rx_arrive(sh.rx_full, s);
+          } else {
+            if (!rx_wait(sh.rx_full, s, 0, kErrWaitFull)) continue;
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+              rx[j] = sh.rx[rx_at(s) + 32 * j];
+              rxc[j] = sh.rxc[rx_at(s) + 32 * j];
+            }
+            rx_arrive(sh.rx_empty, s);
+            emit(cfg, ch, a, cfg * p.na + a, rx, rxc);
+          }
+          s ^= 1;
         }
         a += subsets;
         if (a >= p.na) a = a % subsets + 1;  // the next subset's first angle
@@ -550,11 +614,11 @@ struct Builder {
   template <int MODE>
   __device__ __forceinline__ void walk() {
     if constexpr (MODE == kFmas) {
-      walk_angles(1);
+      walk_angles<false>(1);
     } else if constexpr (kSubsets<MODE> > 0) {
-      walk_angles(kSubsets<MODE>);
+      walk_angles<false>(kSubsets<MODE>);
     } else if constexpr (MODE == kDmas) {
-      walk_angles(1);
+      walk_angles<false>(1);
       walk_channels(2 * p.na);
     } else {
       walk_channels(0);
@@ -663,6 +727,10 @@ __device__ __forceinline__ void add_step(float4 (&acc)[PAIRS], const float4& tap
   }
 }
 
+// Methods that walk their angles one after another.
+template <int MODE>
+constexpr bool kAngleMajor = MODE == kFmas || MODE == kDmas || MODE > kStsw;
+
 // Floats per voxel and frame that a thread keeps in shared memory (its own).
 template <int MODE>
 constexpr int kStash = MODE == kOpw ? 0 : MODE == kFmas || MODE > kStsw ? 4 : MODE == kDmas ? 5 : 2;
@@ -675,7 +743,7 @@ constexpr bool kCross = MODE == kXdoppler || MODE > kStsw;
 // OPW of few frames takes 80 registers and shares the SM with other CTAs.
 template <int MODE>
 __host__ __device__ constexpr int max_threads(int pairs) {
-  return MODE == kOpw && pairs <= 8 ? 384 : 608;
+  return MODE == kDmas ? 512 : MODE == kOpw && pairs <= 8 ? 384 : 608;
 }
 template <int MODE>
 __host__ __device__ constexpr int min_ctas(int pairs) {
@@ -698,8 +766,8 @@ struct Consumer {
 
   __device__ __forceinline__ Consumer(const Args& p_, const Shape& sp_, const Layout& lt_, const Shared& sh_,
                                       const Ring& ring_, int f0)
-      : p(p_), sp(sp_), lt(lt_), sh(sh_), ring(ring_), thread(int(threadIdx.x) - 32 * lt_.builders),
-        count(lt_.threads - 32 * lt_.builders), state(0) {
+      : p(p_), sp(sp_), lt(lt_), sh(sh_), ring(ring_), thread(int(threadIdx.x) - 32 * (lt_.builders + lt_.helpers)),
+        count(lt_.threads - 32 * (lt_.builders + lt_.helpers)), state(0) {
     slot = thread % kTileVoxels;
     group = thread / kTileVoxels;
     first = f0 + 2 * sp.pairs * group;
@@ -723,52 +791,149 @@ struct Consumer {
     stash(s + 1, k) = v.y;
   }
 
+  // What ends a run of steps is called, not inlined: in the step loop its addresses
+  // and temporaries spilled the loop's state, a local store per step that every
+  // release of a stage then waited for (37 x 51 x 35 voxels, 400 x 96 x 9 x 90: St-SW, k = 3, 36.4 ms
+  // inlined, 18.2 called; 48 x 96 x 48, 384 x 128 x 7 x 64: RC-FMAS 30.7 -> 24.5,
+  // DMAS 83 -> 68).  `q` is the thread's first float
+  // of slot 0, its frames `step` and slots `slots` floats apart.
+  struct Sums {
+    float4 q[PAIRS];
+    __device__ __forceinline__ float2 value(int k) const {
+      return k & 1 ? make_float2(q[k / 2].z, q[k / 2].w) : make_float2(q[k / 2].x, q[k / 2].y);
+    }
+  };
+  __device__ __forceinline__ Sums sums() const {
+    Sums s;
+#pragma unroll
+    for (int k = 0; k < PAIRS; ++k) s.q[k] = acc[k];
+    return s;
+  }
+
+  // XDoppler, apertures: the first aperture's sums, kept in slots 0 and 1.
+  static __device__ __noinline__ void keep(const Sums sums, float* q, int step, int slots, int frames) {
+#pragma unroll
+    for (int k = 0; k < kFrames; ++k, q += step) {
+      if (k >= frames) return;
+      const float2 v = sums.value(k);
+      q[0] = v.x;
+      q[slots] = v.y;
+    }
+  }
+
+  // RC-FMAS, one angle: the signed square root.
+  static __device__ __noinline__ void add_root(const Sums sums, float* q, int step, int slots, int frames) {
+#pragma unroll
+    for (int k = 0; k < kFrames; ++k, q += step) {
+      if (k >= frames) return;
+      const float2 r = csroot(sums.value(k));
+      q[0] += r.x;
+      q[slots] += r.y;
+    }
+  }
+  // DMAS, one angle: sum and energy.
+  static __device__ __noinline__ void add_moments(const Sums sums, float* q, int step, int slots, int frames) {
+#pragma unroll
+    for (int k = 0; k < kFrames; ++k, q += step) {
+      if (k >= frames) return;
+      const float2 v = sums.value(k);
+      q[0] += v.x;
+      q[slots] += v.y;
+      q[2 * slots] += cabs2(v);
+    }
+  }
+  // DMAS, one channel: signed square root (slots 1, 2) and magnitude (slot 3).
+  static __device__ __noinline__ void add_roots(const Sums sums, float* q, int step, int slots, int frames) {
+#pragma unroll
+    for (int k = 0; k < kFrames; ++k, q += step) {
+      if (k >= frames) return;
+      const float2 v = sums.value(k), r = csroot(v);
+      q[slots] += r.x;
+      q[2 * slots] += r.y;
+      q[3 * slots] += hypotf(v.x, v.y);
+    }
+  }
   // DMAS: closes the sums of state 0 (slots 0, 1: r; 2: energy) into |mean|^2
   // and variance, those of state 1 (slots 2, 3: q; 4: energy) with them into
   // the angular coherence (slot 0), and clears the next state's slots.
-  __device__ __forceinline__ void advance(int to) {
-    const float inv = 1.0f / float(p.na);
-    for (; state < to; ++state) {
-      const int s0 = state == 0 ? 0 : 2;
-      for (int k = 0; k < 2 * sp.pairs; ++k) {
-        const float n = cabs2(load(s0, k)) * inv * inv;
-        const float v = fmaxf(stash(s0 + 2, k) * inv - n, 0.f);
-        if (state == 0) {
-          store(0, k, make_float2(n, v));
-          stash(2, k) = 0.f;
-        } else {
-          const float2 r = load(0, k);
-          const float num = sqrtf(r.x) * sqrtf(n), den = r.x + n + (r.y + v) / 2 - num;
-          stash(0, k) = den > 0.f ? num / den : 0.f;
-          store(1, k, make_float2(0.f, 0.f));
-          stash(3, k) = 0.f;
-        }
+  static __device__ __noinline__ void close_state(float* q, int step, int slots, int frames, int state, float inv) {
+    for (int k = 0; k < frames; ++k, q += step) {
+      const float* from = q + (state == 0 ? 0 : 2 * slots);
+      const float n = cabs2(make_float2(from[0], from[slots])) * inv * inv;
+      const float v = fmaxf(from[2 * slots] * inv - n, 0.f);
+      if (state == 0) {
+        q[0] = n;
+        q[slots] = v;
+        q[2 * slots] = 0.f;
+      } else {
+        const float rn = q[0], rv = q[slots];
+        const float num = sqrtf(rn) * sqrtf(n), den = rn + n + (rv + v) / 2 - num;
+        q[0] = den > 0.f ? num / den : 0.f;
+        q[slots] = q[2 * slots] = q[3 * slots] = 0.f;
       }
     }
   }
+  __device__ __forceinline__ void advance(int to) {
+    for (; state < to; ++state)
+      close_state(sh.stash + thread, count, 2 * sp.pairs * count, 2 * sp.pairs, state, 1.0f / float(p.na));
+  }
 
-  // St-SW: float f of a voxel-frame's subset statistics (aperture, subset: mean,
-  // mean squared deviation) is kept where its correlation series goes later, in
-  // the caller's workspace of 2 K^2 floats; those beyond (K = 2 has 12) in slot 3.
+  // St-SW: a voxel-frame's subset statistics (aperture, subset: mean, mean squared
+  // deviation), floats 3 index + (0, 1, 2), are kept in pairs where its correlation
+  // series goes later, in the caller's workspace of K^2 float2; K = 2, which has 12
+  // floats, leaves the last subset in slots 0-2 and the deviation before it in slot
+  // 3.  The deviation of an even subset waits in slot 3 for its pair: each 32-byte
+  // sector is then written once and in full.
   static constexpr int K = kSubsets<MODE>;
-  __device__ __forceinline__ float& statistic(unsigned v, int f, int k) const {
-    if (K == 2 && f == 8) return stash(3, k);
-    float2& q = p.series[(size_t(v) * (K * K) + size_t(f / 2)) * size_t(p.nt) + size_t(first + k)];
+  __device__ __forceinline__ float2& statistics(unsigned v, int pair, int k) const {
+    return p.series[(size_t(v) * (K * K) + size_t(pair)) * size_t(p.nt) + size_t(first + k)];
+  }
+  __device__ __forceinline__ float statistic(unsigned v, int f, int k) const {
+    if (K == 2 && f >= 8) return stash(f == 8 ? 3 : f - 9, k);
+    const float2 q = statistics(v, f / 2, k);
     return f & 1 ? q.y : q.x;
   }
 
-  // Ends the current subset (slots 0-2) of `angles` angles.  The last one of K = 2
-  // stays in its slots.
-  __device__ __forceinline__ void close_subset(int index, int angles) {
-    const unsigned v = sh.vox[slot];
-    const int frames = v == UINT_MAX || group >= sp.groups ? 0 : min(2 * sp.pairs, p.nt - first);
-    for (int k = 0; k < 2 * sp.pairs; ++k) {
-      stash(2, k) = stash(2, k) / float(angles);
-      if (K == 2 && index == 2 * K - 1) continue;
-      if (k < frames)
-        for (int f = 0; f < 3; ++f) statistic(v, 3 * index + f, k) = stash(f, k);
-      for (int f = 0; f < 3; ++f) stash(f, k) = 0.f;
+  // One angle: Welford's update of slots 0-2 (no E|x|^2 - |E x|^2 cancellation).
+  static __device__ __noinline__ void add_angle(const Sums sums, float* q, int step, int slots, int frames,
+                                                float inv) {
+#pragma unroll
+    for (int k = 0; k < kFrames; ++k, q += step) {
+      if (k >= frames) return;
+      const float2 v = sums.value(k);
+      const float2 m = make_float2(q[0], q[slots]), d = make_float2(v.x - m.x, v.y - m.y);
+      const float2 now = make_float2(fmaf(d.x, inv, m.x), fmaf(d.y, inv, m.y));
+      q[0] = now.x;
+      q[slots] = now.y;
+      q[2 * slots] += d.x * (v.x - now.x) + d.y * (v.y - now.y);
     }
+  }
+  // Ends subset `index` (slots 0-2) of `angles` angles; `to` is the voxel's first
+  // series value of the thread's frames, of which `live` exist.
+  static __device__ __noinline__ void end_subset(float* q, int step, int slots, int frames, int index, int angles,
+                                                 float2* to, int nt, int live) {
+    for (int k = 0; k < frames; ++k, q += step) {
+      const float2 mean = make_float2(q[0], q[slots]);
+      const float spread = q[2 * slots] / float(angles);
+      if (K == 2 && index == 2 * K - 1) {
+        q[2 * slots] = spread;
+        continue;
+      }
+      if (index % 2 == 0) {
+        if (k < live) to[size_t(3 * index / 2) * nt + k] = mean;
+        q[3 * slots] = spread;
+      } else if (k < live) {
+        to[size_t((3 * index - 1) / 2) * nt + k] = make_float2(q[3 * slots], mean.x);
+        to[size_t((3 * index + 1) / 2) * nt + k] = make_float2(mean.y, spread);
+      }
+      q[0] = q[slots] = q[2 * slots] = 0.f;
+    }
+  }
+  __device__ __forceinline__ void close_subset(int index, int angles) const {
+    const unsigned v = sh.vox[slot];
+    const int live = v == UINT_MAX || group >= sp.groups ? 0 : min(2 * sp.pairs, p.nt - first);
+    end_subset(sh.stash + thread, count, 2 * sp.pairs * count, 2 * sp.pairs, index, angles,
+               live > 0 ? &statistics(v, 0, 0) : nullptr, p.nt, live);
   }
 
   // Angles of subset i: i, i + K, ... < na.
@@ -776,44 +941,27 @@ struct Consumer {
 
   // Ends a run of steps of one tag.
   __device__ __forceinline__ void fold(int tag) {
+    // Keeps the products below out of the step loop's registers.
+    if constexpr (MODE == kDmas || K > 0) asm volatile("" : "+r"(count), "+r"(thread));
+    float* q = sh.stash + thread;
+    const int frames = 2 * sp.pairs, slots = frames * count;
     if constexpr (MODE == kXdoppler || MODE == kApertures) {
       if (tag != 0) return;
-    }
-    if constexpr (MODE == kDmas) advance(tag < p.na ? 0 : tag < 2 * p.na ? 1 : 2);
-    float inv = 1.f;
-    if constexpr (K > 0) {
+      keep(sums(), q, count, slots, frames);
+    } else if constexpr (MODE == kFmas) {
+      add_root(sums(), q + (tag < p.na ? 0 : 2 * slots), count, slots, frames);
+    } else if constexpr (MODE == kDmas) {
+      advance(tag < p.na ? 0 : tag < 2 * p.na ? 1 : 2);
+      if (state == 2)
+        add_roots(sums(), q, count, slots, frames);
+      else
+        add_moments(sums(), q + (state == 0 ? 0 : 2 * slots), count, slots, frames);
+    } else if constexpr (K > 0) {
       const int a = tag % p.na, index = tag / p.na * K + a % K;
       for (; state < index; ++state) close_subset(state, subset_angles(state % K));
       // The angle's place in its subset; angles that no voxel of the tile sees are
       // zero sums that still count.
-      inv = 1.0f / float(a / K + 1);
-    }
-#pragma unroll
-    for (int k = 0; k < kFrames; ++k) {
-      if (k % 4 == 0 && k >= 2 * sp.pairs) break;
-      if (k >= 2 * sp.pairs) continue;
-      const float2 v = value(k);
-      if constexpr (MODE == kXdoppler || MODE == kApertures) {
-        store(0, k, v);
-      } else if constexpr (MODE == kFmas) {
-        const int s = tag < p.na ? 0 : 2;
-        store(s, k, cadd(load(s, k), csroot(v)));
-      } else if constexpr (K > 0) {
-        // Welford's update (no E|x|^2 - |E x|^2 cancellation).
-        const float2 m = load(0, k), d = make_float2(v.x - m.x, v.y - m.y);
-        const float2 now = make_float2(fmaf(d.x, inv, m.x), fmaf(d.y, inv, m.y));
-        store(0, k, now);
-        stash(2, k) += d.x * (v.x - now.x) + d.y * (v.y - now.y);
-      } else if constexpr (MODE == kDmas) {
-        if (state == 2) {
-          store(1, k, cadd(load(1, k), csroot(v)));
-          stash(3, k) += hypotf(v.x, v.y);
-        } else {
-          const int s = state == 0 ? 0 : 2;
-          store(s, k, cadd(load(s, k), v));
-          stash(s + 2, k) += cabs2(v);
-        }
-      }
+      add_angle(sums(), q, count, slots, frames, 1.0f / float(a / K + 1));
     }
     clear();
   }
@@ -921,13 +1069,8 @@ struct Consumer {
 #pragma unroll
       for (int i = 0; i < K; ++i) {
         const int index = ap * K + i;
-        if (K == 2 && index == 2 * K - 1) {
-          mean[ap][i] = load(0, k);
-          spread[ap][i] = stash(2, k);
-        } else {
-          mean[ap][i] = make_float2(statistic(v, 3 * index, k), statistic(v, 3 * index + 1, k));
-          spread[ap][i] = statistic(v, 3 * index + 2, k);
-        }
+        mean[ap][i] = make_float2(statistic(v, 3 * index, k), statistic(v, 3 * index + 1, k));
+        spread[ap][i] = statistic(v, 3 * index + 2, k);
         const float n = float(subset_angles(i));
         sum[ap] = make_float2(fmaf(n, mean[ap][i].x, sum[ap].x), fmaf(n, mean[ap][i].y, sum[ap].y));
       }
@@ -952,7 +1095,11 @@ __device__ __forceinline__ void init_shared(const Shared& sh, const Layout& lt) 
   if (threadIdx.x == 0) {
     for (int s = 0; s < lt.stages; ++s) {
       mbar_init(&sh.full[s], 1);
-      mbar_init(&sh.empty[s], lt.threads / 32 - lt.builders);
+      mbar_init(&sh.empty[s], lt.threads / 32 - lt.builders - lt.helpers);
+    }
+    for (int s = 0; s < 2 * kMaxBuilders; ++s) {
+      mbar_init(&sh.rx_full[s], 1);
+      mbar_init(&sh.rx_empty[s], 1);
     }
     fence_mbar_init();
   }
@@ -970,9 +1117,17 @@ __device__ __forceinline__ bool run_item(const Args& p, const Shape& sp, const L
                   deep ? sp.rows_deep : sp.rows};
   const int frame0 = chunk * sp.frames, warp = threadIdx.x >> 5;
   bool ok;
-  if (warp < lt.builders) {
-    Builder<HALF, BOXES> b(p, sp, lt, sh, ring, maps, frame0, phase);
-    b.template walk<MODE>();
+  if (warp < lt.builders + lt.helpers) {
+    const bool helper = kAngleMajor<MODE> && warp >= lt.builders;
+    Builder<HALF, BOXES> b(p, sp, lt, sh, ring, maps, frame0, helper ? warp - lt.builders : warp, phase);
+    if constexpr (kAngleMajor<MODE>) {
+      if (helper)
+        b.template walk_angles<true>(kSubsets<MODE> > 0 ? kSubsets<MODE> : 1);
+      else
+        b.template walk<MODE>();
+    } else {
+      b.template walk<MODE>();
+    }
     phase = b.phase;
     ok = b.ok;
   } else {

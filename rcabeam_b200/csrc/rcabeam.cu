@@ -206,6 +206,13 @@ struct RowsPlan {
 // results in shared memory).  13 pairs per thread keep a tap's cost small beside
 // its 26 frames; up to 32 frames run 8 pairs, whose kernel leaves room for
 // several CTAs per SM.
+// Sample rows that `bytes` of a stage hold beside the taps.
+static int stage_rows(const das::Shape& sp, int elem, int bytes) {
+  const int slack = sp.frames * elem + 64;  // threads past the last frame read on
+  const int n = std::max(bytes - das::kTapBytes - slack, 0) / sp.pitch;
+  return sp.boxes ? n / das::kBoxRows * das::kBoxRows : n;
+}
+
 template <int MODE>
 static RowsPlan plan_items(const das::Args& a, bool half, int sms, int most) {
   constexpr int kStash = das::kStash<MODE>;
@@ -218,7 +225,10 @@ static RowsPlan plan_items(const das::Args& a, bool half, int sms, int most) {
   // Few tiles: shorter items, so that every SM has one.
   while ((long long)tiles * chunks < sms && (a.nt + chunks - 1) / chunks > 16) ++chunks;
   const int per = (a.nt + chunks - 1) / chunks;
-  r.width = kStash == 0 && per > 32 ? 13 : 8;
+  // 26 frames a thread where they pad a shorter chunk less than 16 do (50 frames: 52
+  // against 64).
+  const bool wide = MODE == das::kXdoppler && (per + 25) / 26 * 26 < (per + 15) / 16 * 16;
+  r.width = (kStash == 0 || wide) && per > 32 ? 13 : 8;
   sp.groups = (per + 2 * r.width - 1) / (2 * r.width);
   sp.pairs = (per + 2 * sp.groups - 1) / (2 * sp.groups);
   sp.frames = 2 * sp.pairs * sp.groups;
@@ -240,8 +250,12 @@ static RowsPlan plan_items(const das::Args& a, bool half, int sms, int most) {
     sp.pitch = sp.contiguous ? a.nt * elem : das::align16(sp.frames * elem) + 16 + a.nt % (16 / elem) * elem;
   const int consumers = das::kBlocks * sp.groups;
   const int row_slack = sp.frames * elem + 64;  // threads past the last frame read on
-  lt.builders = 3;
-  lt.threads = 32 * (lt.builders + consumers);
+  // DMAS keeps so much beside the ring that at 48 frames two builders' stages hold
+  // coarse grids' windows whole and three builders' do not (37 x 51 x 35 voxels, 90 frames:
+  // 54 against 87 ms).
+  lt.builders = MODE == das::kDmas && sp.groups > 2 ? 2 : 3;
+  lt.helpers = das::kAngleMajor<MODE> ? lt.builders : 0;
+  lt.threads = 32 * (lt.builders + lt.helpers + consumers);
   lt.angles = a.na;
   lt.zero_bytes = das::align16(2 * sp.pitch + row_slack);
   lt.stash_bytes = kStash * 2 * sp.pairs * 4 * 32 * consumers;
@@ -252,16 +266,12 @@ static RowsPlan plan_items(const das::Args& a, bool half, int sms, int most) {
   auto fit = [&](int cap, int least) {
     const int fixed = das::kFixedBytes + 24 * a.na + lt.zero_bytes + lt.stash_bytes + lt.table_bytes;
     if (cap <= fixed) return false;
-    auto rows_of = [&](int bytes) {
-      const int n = (bytes - das::kTapBytes - row_slack) / sp.pitch;
-      return sp.boxes ? n / das::kBoxRows * das::kBoxRows : n;
-    };
     // More rows than a compact tile needs would only cost a CTA its neighbours.
     const long long enough = (das::kTapBytes + row_slack + 96ll * sp.pitch + 255) / 256 * 128;
     lt.stages = 2 * lt.builders;
     lt.stage_bytes = int(std::min<long long>((cap - fixed) / lt.stages / 128 * 128, enough));
-    sp.rows = rows_of(2 * lt.stage_bytes);
-    sp.rows_deep = std::max(rows_of(lt.stage_bytes), 0);
+    sp.rows = stage_rows(sp, elem, 2 * lt.stage_bytes);
+    sp.rows_deep = stage_rows(sp, elem, lt.stage_bytes);
     lt.smem = fixed + lt.stages * lt.stage_bytes;
     return sp.rows >= least;
   };
@@ -301,7 +311,7 @@ static rcabeam_status run_rows(const das::Args& a, cudaStream_t stream = 0) {
     return r.width == 13 ? launch_rows<MODE, 13, true, false>(a, r, n, stream)
                          : launch_rows<MODE, 8, true, false>(a, r, n, stream);
   } else {
-    if constexpr (MODE == das::kOpw) {
+    if constexpr (MODE == das::kOpw || MODE == das::kXdoppler) {
       if (r.width == 13)
         return r.shape.boxes ? launch_rows<MODE, 13, false, true>(a, r, n, stream)
                              : launch_rows<MODE, 13, false, false>(a, r, n, stream);
@@ -1420,10 +1430,12 @@ bool batch_plan(size_t n, const rcabeam_batch_ensemble* list, std::vector<batch:
                 long long* total_items, das::Layout* layout) {
   if (!n || !list || n > (1u << 20)) return false;
   long long items = 0, tiles_xd = 0;
-  if (out) out->resize(n);
   das::Layout lt{};
   int consumers = 0, stash_unit = 0;
   bool fits = true;
+  std::vector<batch::Ensemble> own;
+  if (!out) out = &own;
+  out->resize(n);
   for (size_t i = 0; i < n; ++i) {
     const rcabeam_batch_ensemble& d = list[i];
     if (!d.rc || !d.cr || !d.scan || !d.xe || !d.ye || !d.angles || !d.starts || !d.pd || d.ns < 2 || !d.nc ||
@@ -1458,7 +1470,7 @@ bool batch_plan(size_t n, const rcabeam_batch_ensemble* list, std::vector<batch:
     a.err = device_error_ptr();
     // 64: the planned split; 16 or 32: items of at most that many frames.
     const RowsPlan r = batch_item_plan(a, d.method, fpc == 64 ? INT32_MAX : fpc);
-    fits = fits && r.layout.smem && (i == 0 || r.layout.builders == lt.builders);
+    fits = fits && r.layout.smem;
     e.method = d.method;
     e.shape = r.shape;
     e.maps = r.maps;
@@ -1468,15 +1480,16 @@ bool batch_plan(size_t n, const rcabeam_batch_ensemble* list, std::vector<batch:
     e.tile_base = tiles_xd;
     items += (long long)e.tiles * e.shape.chunks;
     if (d.method == 1) tiles_xd += e.tiles;
-    const int warps = r.layout.threads / 32 - r.layout.builders;
+    const int warps = r.layout.threads / 32 - r.layout.builders - r.layout.helpers;
     consumers = std::max(consumers, warps);
     stash_unit = std::max(stash_unit, r.layout.stash_bytes / (32 * warps));
-    lt.builders = r.layout.builders;
+    lt.builders = i == 0 ? r.layout.builders : std::min(lt.builders, r.layout.builders);
+    lt.helpers = r.layout.helpers > 0 ? lt.builders : 0;
     lt.stage_bytes = std::max(lt.stage_bytes, r.layout.stage_bytes);
     lt.zero_bytes = std::max(lt.zero_bytes, r.layout.zero_bytes);
     lt.angles = std::max(lt.angles, r.layout.angles);
     lt.table_bytes = std::max(lt.table_bytes, r.layout.table_bytes);
-    if (out) (*out)[i] = e;
+    (*out)[i] = e;
   }
   L->ens = 0;
   L->next = L->ens + align256(n * sizeof(batch::Ensemble));
@@ -1484,16 +1497,24 @@ bool batch_plan(size_t n, const rcabeam_batch_ensemble* list, std::vector<batch:
   L->tile_done = L->done + align256(n * 4);
   L->total = L->tile_done + align256(size_t(tiles_xd > 0 ? tiles_xd : 1) * 4);
   *total_items = items;
-  if (layout) {
-    // A launch's ring stages are the largest any ensemble plans for itself.
-    lt.threads = 32 * (lt.builders + consumers);
-    lt.stages = 2 * lt.builders;
-    lt.stash_bytes = stash_unit * 32 * consumers;
-    lt.smem = das::kFixedBytes + 24 * lt.angles + lt.zero_bytes + lt.stash_bytes + lt.table_bytes +
-              lt.stages * lt.stage_bytes;
-    if (!fits || lt.smem > 227 * 1024) lt.smem = 0;
-    *layout = lt;
+  // A launch's ring stages are the largest any ensemble plans for itself, or what
+  // is left of an SM's shared memory (less the kernel's own) beside the largest
+  // tables and stashes.
+  lt.threads = 32 * (lt.builders + lt.helpers + consumers);
+  lt.stages = 2 * lt.builders;
+  lt.stash_bytes = stash_unit * 32 * consumers;
+  const int fixed = das::kFixedBytes + 24 * lt.angles + lt.zero_bytes + lt.stash_bytes + lt.table_bytes;
+  const int room = std::max(226 * 1024 - fixed, 0) / lt.stages / 128 * 128;
+  if (room < lt.stage_bytes) {
+    lt.stage_bytes = room;
+    for (batch::Ensemble& e : *out) {
+      e.shape.rows = stage_rows(e.shape, 8, 2 * room);
+      e.shape.rows_deep = stage_rows(e.shape, 8, room);
+      fits = fits && e.shape.rows >= 40;
+    }
   }
+  lt.smem = fits ? fixed + lt.stages * lt.stage_bytes : 0;
+  if (layout) *layout = lt;
   return true;
 }
 

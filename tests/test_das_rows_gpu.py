@@ -11,7 +11,8 @@ import pytest
 import torch
 
 from oracle import methods
-from rcabeam_b200 import _cuda_impl, _lib
+from rcabeam_b200 import _cuda_impl, _lib, batching
+from rcabeam_b200.sim import RCAGeometry
 from tests._cases import rel_l2
 
 pytestmark = pytest.mark.gpu
@@ -96,3 +97,31 @@ def test_staged_splits_match_oracle(frames, kind, nv, na, fn, shift):
     assert rel_l2(pd, np.mean(np.abs(fmas) ** 2, axis=-1)) <= 1e-4
     pd, _ = run(3)
     assert rel_l2(pd, methods.dmas_ccf_acf_power(rc, cr, *geom)) <= 1e-4
+
+
+@pytest.mark.parametrize("method,specs", [
+    ("xdoppler", [(50, 3), (16, 48), (64, 2)]),  # a long angle table beside wide stages: they shrink
+    ("dmas", [(48, 2), (20, 9), (7, 40)]),       # items with two and with three builder warps
+])
+def test_queue_of_uneven_layouts(method, specs):
+    """Ensembles whose own rings differ share one launch (1e-5 as in test_batch_gpu.py)."""
+    rng = np.random.default_rng(len(specs))
+    ns, nc = 160, 8
+    el = (np.arange(nc) - (nc - 1) / 2) * 0.2e-3
+    geom = RCAGeometry(el, el, c=C, fs=FS, f_demod=FD, fnumber=None)
+    ensembles = []
+    for frames, na in specs:
+        shape = (ns, nc, na, frames)
+        packed = [torch.from_numpy((rng.normal(size=shape) + 1j * rng.normal(size=shape)).astype(np.complex64))
+                  .permute(1, 2, 0, 3).contiguous().cuda() for _ in range(2)]
+        grid = (np.linspace(-1.2e-3, 1.2e-3, 9), np.linspace(3e-3, 6e-3, 13), np.linspace(-1e-3, 1e-3, 7))
+        e = batching.Ensemble(packed[0], packed[1], shape, grid, geom, np.deg2rad(np.linspace(-8, 8, na)), 3e-6, method)
+        e.build(torch.device("cuda"))
+        ensembles.append(e)
+    batching.sequential(ensembles)
+    want = [e.power().cpu().numpy().copy() for e in ensembles]
+    batching.BatchQueue(ensembles, ctas_per_sm=1).run()
+    torch.cuda.synchronize()
+    for e, w in zip(ensembles, want):
+        assert np.abs(w).max() > 0
+        assert rel_l2(e.power().cpu().numpy(), w) <= 1e-5
