@@ -132,7 +132,10 @@ __device__ __forceinline__ void voxel_pos(const Geometry& g, int l, double& x, d
 // up.  A region of interest lists far fewer voxels than the GPU has threads (1332
 // for a 1 mm sphere): one thread each left eleven CTAs walking all channels one
 // after another (3.35 ms per 8-frame chunk at 2 x 128 channels and 7 angles, angles'
-// sines formed per tap); with a warp each the same chunk takes 0.19 ms.
+// sines formed per tap); with a warp each the same chunk takes 0.19 ms.  A channel's
+// angles are summed in R, the channels in float64: the delay and sound-speed
+// gradients are float64 sums over all of a region's samples, and what they lose is
+// mostly the rounding of the IQ formed here.
 template <typename R, int LANES>
 __global__ void __launch_bounds__(128) forward(Geometry g, const typename Cx<R>::type* __restrict__ rc,
                                                const typename Cx<R>::type* __restrict__ cr,
@@ -146,15 +149,18 @@ __global__ void __launch_bounds__(128) forward(Geometry g, const typename Cx<R>:
   const int l = live ? int(id / LANES) : g.nvl - 1;
   double x, z, y;
   voxel_pos(g, l, x, z, y);
-  R re[kChunk], im[kChunk];
+  double re[kChunk], im[kChunk];
 #pragma unroll
-  for (int t = 0; t < kChunk; ++t) re[t] = im[t] = R(0);
+  for (int t = 0; t < kChunk; ++t) re[t] = im[t] = 0.0;
   for (int pair = sub; pair < 2 * g.nc; pair += LANES) {
     const int ap = pair >= g.nc, ch = pair - ap * g.nc;
     const C* X = ap ? cr : rc;
     const double u = ap ? x : y;
     const Receive rx = receive_of(g, ap ? y : x, z, ap, ch);
     if (!rx.active) continue;
+    R sr[kChunk], si[kChunk];
+#pragma unroll
+    for (int k = 0; k < kChunk; ++k) sr[k] = si[k] = R(0);
     for (int a = 0; a < g.na; ++a) {
       const Tap64 t = tap(g, table, rx, u, z, a);
       if (!t.ok) continue;
@@ -167,10 +173,15 @@ __global__ void __launch_bounds__(128) forward(Geometry g, const typename Cx<R>:
         if (k < g.frames) {
           const C x0 = X[b0 + k], x1 = X[b1 + k];
           const R vr = f0w * x0.x + f * x1.x, vi = f0w * x0.y + f * x1.y;
-          re[k] += vr * ph.x - vi * ph.y;
-          im[k] += vr * ph.y + vi * ph.x;
+          sr[k] += vr * ph.x - vi * ph.y;
+          si[k] += vr * ph.y + vi * ph.x;
         }
       }
+    }
+#pragma unroll
+    for (int k = 0; k < kChunk; ++k) {
+      re[k] += double(sr[k]);
+      im[k] += double(si[k]);
     }
   }
 #pragma unroll
@@ -186,8 +197,8 @@ __global__ void __launch_bounds__(128) forward(Geometry g, const typename Cx<R>:
 #pragma unroll
   for (int k = 0; k < kChunk; ++k) {
     if (k < g.frames) {
-      if (iq) iq[size_t(l) * g.frames + k] = C{re[k], im[k]};
-      p += double(re[k]) * double(re[k]) + double(im[k]) * double(im[k]);
+      if (iq) iq[size_t(l) * g.frames + k] = C{R(re[k]), R(im[k])};
+      p += re[k] * re[k] + im[k] * im[k];
     }
   }
   if (power) power[l] += p / double(g.nt);
