@@ -50,7 +50,7 @@ namespace das {
 constexpr int kTileVoxels = 128;
 constexpr int kBlocks = kTileVoxels / 32;  // consumer warps per frame group
 constexpr int kMaxBuilders = 4;
-constexpr int kMaxGroups = 8;              // frame groups of an item
+constexpr int kMaxGroups = 4;              // frame groups of an item (plan_items: 104 frames in 26s, 64 in 16s)
 constexpr int kBoxRows = 8;                // sample rows of one TMA box
 
 // St-SW (method 4) with K angle subsets is kStsw + K.
@@ -127,7 +127,7 @@ struct Shared {
   int2* tag;              // run of the stage's step; voxel blocks with a tap in it (bit per block)
   unsigned* vox;          // voxel ids of the tile
   float* pos;             // [3][128] x, z, y
-  float* power;           // [2][groups][128] sums over a group's frames
+  double* power;          // [2][groups][128] sums over a group's frames
   float* active;          // [128] channels inside the aperture (DMAS)
   float* bounds;          // tile minimum and maximum of x and of y, maximum of z, rows a step can span
   double* angle;          // [na][3] cos, sin, start
@@ -146,7 +146,7 @@ struct Ring {
   int stages, bytes, rows;
 };
 constexpr int kRxEntries = 2 * kMaxBuilders * kTileVoxels;
-constexpr int kFixedBytes = kMaxStages * 24 + 4 * kMaxBuilders * 8 + kTileVoxels * 4 * (1 + 3 + 2 * kMaxGroups + 1) + 64 + kTileVoxels * 8 + kRxEntries * 12;
+constexpr int kFixedBytes = kMaxStages * 24 + 4 * kMaxBuilders * 8 + kTileVoxels * (4 * (1 + 3 + 1) + 8 * 2 * kMaxGroups) + 64 + kTileVoxels * 8 + kRxEntries * 12;
 
 __device__ __forceinline__ Shared carve(unsigned char* smem, const Layout& l) {
   Shared s;
@@ -169,8 +169,8 @@ __device__ __forceinline__ Shared carve(unsigned char* smem, const Layout& l) {
   s.tag = reinterpret_cast<int2*>(s.rx_empty + 2 * kMaxBuilders);
   s.vox = reinterpret_cast<unsigned*>(s.tag + kMaxStages);
   s.pos = reinterpret_cast<float*>(s.vox + kTileVoxels);
-  s.power = s.pos + 3 * kTileVoxels;
-  s.active = s.power + 2 * kMaxGroups * kTileVoxels;
+  s.power = reinterpret_cast<double*>(s.pos + 3 * kTileVoxels);
+  s.active = reinterpret_cast<float*>(s.power + 2 * kMaxGroups * kTileVoxels);
   s.bounds = s.active + kTileVoxels;
   s.rxc = reinterpret_cast<unsigned*>(s.bounds + 16);
   return s;
@@ -1015,11 +1015,20 @@ struct Consumer {
     return true;
   }
 
+  // |x|^2 in float64.
+  static __device__ __forceinline__ double power_of(float2 x) {
+    return fma(double(x.x), double(x.x), double(x.y) * double(x.y));
+  }
+
+  // The frames' values and, in float64, their power.  A thread adds up to 26 frames
+  // one after another: in float32 that showed in the power maps (48 x 96 x 48 voxels,
+  // 384 x 128 x 7 x 64, RC-FMAS: 1.4e-7 from float64, 5.9e-8 with these sums; 40 x 70 x
+  // 36, 300 x 96 x 9 x 75, OPW of filtered channels: 1.69e-7 and 1.3e-7).
   __device__ __forceinline__ void write() {
     if (group >= sp.groups) return;
     const unsigned v = sh.vox[slot];
     const int frames = v == UINT_MAX ? 0 : min(2 * sp.pairs, p.nt - first);
-    float pr = 0.f, pi = 0.f;
+    double pr = 0.0, pi = 0.0;
 #pragma unroll
     for (int k = 0; k < kFrames; ++k) {
       if (k >= frames) continue;
@@ -1027,23 +1036,23 @@ struct Consumer {
       const size_t at = size_t(v) * p.nt + first + k;
       if constexpr (MODE == kOpw) {
         if (p.signal) p.signal[at] = x;
-        pr += cabs2(x);
+        pr += power_of(x);
       } else if constexpr (MODE == kApertures) {
         p.signal[at + size_t(v) * p.nt] = load(0, k);
         p.signal[at + size_t(v) * p.nt + p.nt] = x;
       } else if constexpr (MODE == kXdoppler) {
         const float2 val = cmul(load(0, k), cconj(x));
         if (p.signal) p.signal[at] = val;
-        pr += val.x;
-        pi += val.y;
+        pr += double(val.x);
+        pi += double(val.y);
       } else if constexpr (MODE == kFmas) {
         const float2 val = cmul(load(0, k), load(2, k));
         if (p.signal) p.signal[at] = val;
-        pr += cabs2(val);
+        pr += power_of(val);
       } else if constexpr (K > 0) {
         const float2 val = write_series(v, k);
-        pr += val.x;
-        pi += val.y;
+        pr += double(val.x);
+        pi += double(val.y);
       } else {
         const float mag = stash(3, k), act = sh.active[slot];
         const float dm = cabs2(load(1, k)) - mag;
@@ -1051,7 +1060,7 @@ struct Consumer {
         float pw = dm * wc * stash(0, k);
         if (!isfinite(pw)) pw = 0.f;
         if (p.signal) p.signal[at] = make_float2(pw, 0.f);
-        pr += pw;
+        pr += double(pw);
       }
     }
     sh.power[group * kTileVoxels + slot] = pr;
@@ -1137,17 +1146,16 @@ __device__ __forceinline__ bool run_item(const Args& p, const Shape& sp, const L
   }
   ok = __syncthreads_and(ok);
   if constexpr (MODE != kApertures) {
-    const float inv_nt = 1.0f / float(p.nt);
     for (int i = threadIdx.x; ok && i < kTileVoxels; i += blockDim.x) {
       const unsigned v = sh.vox[i];
       if (v == UINT_MAX) continue;
-      float re = 0.f, im = 0.f;
+      double re = 0.0, im = 0.0;
       for (int g = 0; g < sp.groups; ++g) {
         re += sh.power[g * kTileVoxels + i];
         if constexpr (kCross<MODE>) im += sh.power[(kMaxGroups + g) * kTileVoxels + i];
       }
-      atomicAdd(p.pd + 2 * size_t(v), re * inv_nt);
-      if constexpr (kCross<MODE>) atomicAdd(p.pd + 2 * size_t(v) + 1, im * inv_nt);
+      atomicAdd(p.pd + 2 * size_t(v), float(re / double(p.nt)));
+      if constexpr (kCross<MODE>) atomicAdd(p.pd + 2 * size_t(v) + 1, float(im / double(p.nt)));
     }
   }
   return ok;

@@ -38,7 +38,7 @@ def _voxels(kind: str, nv: int, rng) -> np.ndarray:
     return scan.astype(np.float32)
 
 
-def _reconstruct(rc, cr, scan, xe, ye, angles, starts, fn, method, shift):
+def _reconstruct(rc, cr, scan, xe, ye, angles, starts, fn, method, shift, fd=FD):
     ns, nc, na, nt = rc.shape
     dev = lambda a: torch.from_numpy(np.ascontiguousarray(a)).cuda()  # noqa: E731
     packed = []
@@ -54,7 +54,7 @@ def _reconstruct(rc, cr, scan, xe, ye, angles, starts, fn, method, shift):
     work = torch.empty(_cuda_impl.workspace_bytes(nv, nc, na), dtype=torch.uint8, device="cuda")
     t = [dev(a) for a in (scan, xe, ye, angles, starts)]
     _lib.call("rcabeam_ensemble_device", packed[0].data_ptr(), packed[1].data_ptr(), *(a.data_ptr() for a in t),
-              pd.data_ptr(), signal.data_ptr(), None, None, work.data_ptr(), ns, nc, na, nt, nv, C, FS, FD,
+              pd.data_ptr(), signal.data_ptr(), None, None, work.data_ptr(), ns, nc, na, nt, nv, C, FS, fd,
               -1.0 if fn is None else fn, method, 2)
     return pd[:, 0].cpu().numpy(), signal.cpu().numpy().reshape(nv, planes, nt)
 
@@ -125,3 +125,21 @@ def test_queue_of_uneven_layouts(method, specs):
     for e, w in zip(ensembles, want):
         assert np.abs(w).max() > 0
         assert rel_l2(e.power().cpu().numpy(), w) <= 1e-5
+
+
+@pytest.mark.parametrize("method", [0, 1])
+@pytest.mark.parametrize("frames", [26, 78])
+def test_power_sums_keep_small_frames(method, frames):
+    """One strong frame among ones, every product exact: the power is the float64 mean
+    rounded once to float32 (2^-24; XDoppler's hypotf adds up to 3 ulp); a float32 sum
+    loses all the other frames (1.5e-6)."""
+    value = np.ones(frames, np.complex64)
+    value[0] = 2.0**12
+    rc = np.broadcast_to(value, (64, 1, 1, frames)).copy()
+    cr = rc if method == 1 else np.zeros_like(rc)
+    scan = np.array([[0.0, 3e-3, 0.0]], np.float32)
+    zero = np.zeros(1, np.float32)
+    start = np.array([2 * 3e-3 / C - 1e-6], np.float32)
+    pd, _ = _reconstruct(rc, cr, scan, zero, zero, zero, start, None, method, 0, fd=0.0)
+    want = (2.0**24 + frames - 1) / frames
+    assert abs(float(pd[0]) - want) <= (2.0**-24 if method == 0 else 7 * 2.0**-24) * want
