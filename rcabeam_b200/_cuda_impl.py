@@ -23,6 +23,7 @@ _COMPLEX64 = (np.complex64, torch.complex64)
 _STSW_SCRATCH_BYTES = 256 << 20
 # Host arrays from this size on cross through pinned staging and several host threads.
 _STAGED_COPY_BYTES = 4 << 20
+_NUMPY_TYPE = {torch.float32: np.float32, torch.complex64: np.complex64}
 
 
 def _ptr(t: torch.Tensor | None) -> int | None:
@@ -51,8 +52,9 @@ def _host_copy(host: np.ndarray, device: torch.Tensor, upload: bool) -> None:
 
 
 def _download(device: torch.Tensor, host: np.ndarray) -> None:
-    """Device tensor into a host array of the same shape (the device's work is complete)."""
-    if host.flags.c_contiguous and host.flags.writeable and host.nbytes >= _STAGED_COPY_BYTES:
+    """Device tensor into a host array of the same shape (the device's work is complete); types convert."""
+    same = host.dtype == _NUMPY_TYPE.get(device.dtype) and host.size == device.numel() and device.is_contiguous()
+    if same and host.flags.c_contiguous and host.flags.writeable and host.nbytes >= _STAGED_COPY_BYTES:
         _host_copy(host, device, False)
     else:
         np.copyto(host, device.cpu().numpy())

@@ -154,3 +154,23 @@ def test_depth_axis():
     assert np.all(np.diff(axis) <= 1540 / (2 * 15e6) + 1e-15)
     with pytest.raises(ValueError):
         rb.depth_axis(2.0, 1.0, 1e6)
+
+
+@pytest.mark.parametrize("elements", [1 << 10, 1 << 20])
+@pytest.mark.parametrize("source,target", [("float32", "<f8"), ("float32", ">f4"), ("complex64", "<c16"),
+                                           ("float32", "<f4"), ("complex64", "<c8")])
+def test_downloads_convert_types(monkeypatch, elements, source, target):
+    """Raw bytes cross only into an array of the tensor's own type; any other type is converted."""
+    import torch
+
+    from rcabeam_b200 import _cuda_impl
+
+    def staged(host, device, upload):
+        assert not upload and host.dtype == np.dtype(source) and host.nbytes == device.numel() * device.element_size()
+        np.copyto(host, device.numpy())
+
+    monkeypatch.setattr(_cuda_impl, "_host_copy", staged)
+    device = torch.arange(elements, dtype=torch.float32).to(getattr(torch, source)).reshape(-1, 2)
+    host = np.zeros(device.shape, target)
+    _cuda_impl._download(device, host)
+    assert np.array_equal(host, device.numpy())

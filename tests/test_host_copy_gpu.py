@@ -47,3 +47,22 @@ def test_concurrent_uploads_from_two_threads():
         t.join()
     for a, d in zip(arrays, out):
         assert np.array_equal(d.cpu().numpy(), a)
+
+
+@pytest.mark.parametrize("voxels", [1000, 300_000])
+def test_wider_host_outputs_are_converted(voxels):
+    rng = np.random.default_rng(voxels)
+    rc, cr = ((rng.normal(size=(64, 2, 1, 2)) + 1j * rng.normal(size=(64, 2, 1, 2))).astype(np.complex64)
+              for _ in range(2))
+    scan = rng.uniform([-1e-3, 3e-3, -1e-3], [1e-3, 4e-3, 1e-3], (voxels, 3)).astype(np.float32)
+    el, zero = np.array([-1e-4, 1e-4], np.float32), np.zeros(1, np.float32)
+    start = np.array([2 * 3e-3 / 1540 - 0.3e-6], np.float32)
+    results = []
+    for real, cplx in ((np.float32, np.complex64), (np.float64, np.complex128)):
+        pd, signal = np.zeros((voxels, 2), real), np.zeros((voxels, 2), cplx)
+        _cuda_impl.ensemble_from_channels(rc, cr, scan, el, el, zero, start, pd, signal, None, 1540.0, 20e6, 5e6, -1.0,
+                                          0, 2, False)
+        results.append((pd, signal))
+    (pd, signal), (pd64, signal64) = results
+    assert np.abs(signal).max() > 0
+    assert np.array_equal(pd64, pd) and np.array_equal(signal64, signal)
