@@ -52,6 +52,7 @@ constexpr int kBlocks = kTileVoxels / 32;  // consumer warps per frame group
 constexpr int kMaxBuilders = 4;
 constexpr int kMaxGroups = 4;              // frame groups of an item (plan_items: 104 frames in 26s, 64 in 16s)
 constexpr int kBoxRows = 8;                // sample rows of one TMA box
+constexpr int kMaxBoxes = 32;              // boxes of one window: each lane issues at most one
 
 // St-SW (method 4) with K angle subsets is kStsw + K.
 enum Mode : int { kOpw = 0, kXdoppler = 1, kFmas = 2, kDmas = 3, kApertures = 5, kStsw = 8 };

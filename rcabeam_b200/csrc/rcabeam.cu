@@ -210,7 +210,7 @@ struct RowsPlan {
 static int stage_rows(const das::Shape& sp, int elem, int bytes) {
   const int slack = sp.frames * elem + 64;  // threads past the last frame read on
   const int n = std::max(bytes - das::kTapBytes - slack, 0) / sp.pitch;
-  return sp.boxes ? n / das::kBoxRows * das::kBoxRows : n;
+  return sp.boxes ? std::min(n / das::kBoxRows, das::kMaxBoxes) * das::kBoxRows : n;
 }
 
 template <int MODE>
@@ -1508,8 +1508,8 @@ bool batch_plan(size_t n, const rcabeam_batch_ensemble* list, std::vector<batch:
   if (room < lt.stage_bytes) {
     lt.stage_bytes = room;
     for (batch::Ensemble& e : *out) {
-      e.shape.rows = stage_rows(e.shape, 8, 2 * room);
-      e.shape.rows_deep = stage_rows(e.shape, 8, room);
+      e.shape.rows = std::min(e.shape.rows, stage_rows(e.shape, 8, 2 * room));
+      e.shape.rows_deep = std::min(e.shape.rows_deep, stage_rows(e.shape, 8, room));
       fits = fits && e.shape.rows >= 40;
     }
   }

@@ -127,6 +127,32 @@ def test_queue_of_uneven_layouts(method, specs):
         assert rel_l2(e.power().cpu().numpy(), w) <= 1e-5
 
 
+@pytest.mark.parametrize("method,frames", [("opw", (100, 16)), ("xdoppler", (64, 16))])
+def test_queue_of_long_windows(method, frames):
+    """A step's window of more than 256 sample rows, 32 boxes, beside an ensemble whose
+    ring gives the short one far wider stages (1e-5 as in test_batch_gpu.py)."""
+    rng = np.random.default_rng(frames[0])
+    ns, nc, na = 800, 6, 5
+    el = (np.arange(nc) - (nc - 1) / 2) * 0.2e-3
+    geom = RCAGeometry(el, el, c=C, fs=FS, f_demod=FD, fnumber=None)
+    grid = (np.linspace(-1e-3, 1e-3, 3), np.linspace(3e-3, 30e-3, 20), np.linspace(-1e-3, 1e-3, 2))  # one tile
+    ensembles = []
+    for nt in frames:
+        packed = [torch.from_numpy((rng.normal(size=(nc, na, ns, nt)) + 1j * rng.normal(size=(nc, na, ns, nt)))
+                                   .astype(np.complex64)).cuda() for _ in range(2)]
+        e = batching.Ensemble(packed[0], packed[1], (ns, nc, na, nt), grid, geom, np.deg2rad(np.linspace(-8, 8, na)),
+                              3e-6, method)
+        e.build(torch.device("cuda"))
+        ensembles.append(e)
+    batching.sequential(ensembles)
+    want = [e.power().cpu().numpy().copy() for e in ensembles]
+    batching.BatchQueue(ensembles, ctas_per_sm=1).run()
+    torch.cuda.synchronize()
+    for e, w in zip(ensembles, want):
+        assert np.abs(w).min() > 0
+        assert rel_l2(e.power().cpu().numpy(), w) <= 1e-5
+
+
 @pytest.mark.parametrize("method", [0, 1])
 @pytest.mark.parametrize("frames", [26, 78])
 def test_power_sums_keep_small_frames(method, frames):
