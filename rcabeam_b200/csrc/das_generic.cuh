@@ -1,5 +1,6 @@
-// The pair sums of St-SW (method 4) and the per-frame entry points of the
-// reference's single-frame API (core.cu).
+// RC-FMAS, DMAS-CCF-ACF and St-SW of few voxels with one warp per voxel, the pair
+// sums of St-SW (method 4) and the per-frame entry points of the reference's
+// single-frame API (core.cu).
 #pragma once
 
 #include "common.cuh"
@@ -28,6 +29,195 @@ __device__ __forceinline__ Tap tap_of(const Voxel& q, int config, const float* e
   return make_tap(__dadd_rn(ttx, trx), double(starts[a]), fs, fd, ns, act);
 }
 
+// ---------------------------------------------------- one warp per voxel --
+// The nonlinear methods of few voxels: a warp owns one voxel, a lane one frame (grid.y
+// counts blocks of 32).  The staged kernel (das_rows.cuh) walks all channels and angles
+// of 128 voxels in one CTA; with few tiles most SMs have none, and the walk's latency is
+// the call's time.  Here the same steps run on as many warps as there are voxels, bound
+// by the latency of the per-frame gathers until the SMs are full (about 4000 warps):
+// 128 channels, 11 angles, 64 frames, 1000 voxels over 10 mm: RC-FMAS 4.84 -> 1.08 ms,
+// DMAS 37.6 -> 2.3, St-SW (k = 3) 5.27 -> 1.06; within 2 mm, where a tile's windows are
+// short, 1.35 -> 1.05, 3.37 -> 1.95 and 1.51 -> 1.07.  rcabeam.cu (few_voxels) draws the line.
+struct WarpTaps {
+  Tap rc[32], cr[32];
+};
+
+// Interpolated, rotated sample of a packed (c, a, s, t) complex64 ensemble.
+__device__ __forceinline__ float2 packed_sample(const void* iq, const Tap& t, int ch, int a, int frame,
+                                                const das::Args& p) {
+  if (t.i0 < 0 || frame >= p.nt) return make_float2(0.f, 0.f);
+  const float2* at =
+      static_cast<const float2*>(iq) + ((size_t(ch) * p.na + a) * p.ns + size_t(t.i0)) * p.nt + frame;
+  const float2 va = at[0], vb = at[t.i0 == p.ns - 1 ? 0 : p.nt];
+  return cmul(make_float2(fmaf(t.w, vb.x - va.x, va.x), fmaf(t.w, vb.y - va.y, va.y)), t.phase);
+}
+
+// Sums of both apertures over the channels of angle a.  A lane forms one channel's
+// taps, which the warp then reads back from shared memory.
+__device__ __forceinline__ void angle_sums(const das::Args& p, const Voxel& q, int a, int frame, WarpTaps& taps,
+                                           float2& r, float2& s) {
+  const int lane = threadIdx.x & 31;
+  const double th = double(p.angles[a]), cs = cos(th), sn = sin(th), start = double(p.starts[a]);
+  const double tx_rc = transmit_delay(q.y, q.z, cs, sn, p.c), tx_cr = transmit_delay(q.x, q.z, cs, sn, p.c);
+  r = s = make_float2(0.f, 0.f);
+  for (int c0 = 0; c0 < p.nc; c0 += 32) {
+    const int count = min(32, p.nc - c0);
+    __syncwarp();  // the previous taps have been read
+    if (lane < count) {
+      bool active;
+      const double rx_rc = receive_delay(q.x, q.z, double(p.xe[c0 + lane]), p.c, p.fn, &active);
+      taps.rc[lane] = make_tap(__dadd_rn(tx_rc, rx_rc), start, p.fs, p.fd, p.ns, active);
+      const double rx_cr = receive_delay(q.y, q.z, double(p.ye[c0 + lane]), p.c, p.fn, &active);
+      taps.cr[lane] = make_tap(__dadd_rn(tx_cr, rx_cr), start, p.fs, p.fd, p.ns, active);
+    }
+    __syncwarp();
+    for (int j = 0; j < count; ++j) {
+      r = cadd(r, packed_sample(p.rc, taps.rc[j], c0 + j, a, frame, p));
+      s = cadd(s, packed_sample(p.cr, taps.cr[j], c0 + j, a, frame, p));
+    }
+  }
+}
+
+// Sums of both apertures over the angles of channel ch.
+__device__ __forceinline__ void channel_sums(const das::Args& p, const Voxel& q, int ch, int frame, WarpTaps& taps,
+                                             float2& r, float2& s) {
+  const int lane = threadIdx.x & 31;
+  r = s = make_float2(0.f, 0.f);
+  for (int a0 = 0; a0 < p.na; a0 += 32) {
+    const int count = min(32, p.na - a0);
+    __syncwarp();
+    if (lane < count) {
+      taps.rc[lane] = tap_of(q, 0, p.xe, ch, p.angles, p.starts, a0 + lane, p.c, p.fs, p.fd, p.fn, p.ns);
+      taps.cr[lane] = tap_of(q, 1, p.ye, ch, p.angles, p.starts, a0 + lane, p.c, p.fs, p.fd, p.fn, p.ns);
+    }
+    __syncwarp();
+    for (int j = 0; j < count; ++j) {
+      r = cadd(r, packed_sample(p.rc, taps.rc[j], ch, a0 + j, frame, p));
+      s = cadd(s, packed_sample(p.cr, taps.cr[j], ch, a0 + j, frame, p));
+    }
+  }
+}
+
+// Power of one frame by RC-FMAS: signed square roots of the channel sums, added over angles.
+__device__ __forceinline__ double fmas_frame(const das::Args& p, const Voxel& q, size_t v, int frame, WarpTaps& taps) {
+  float2 r = make_float2(0.f, 0.f), s = r;
+  for (int a = 0; a < p.na; ++a) {
+    float2 ar, as;
+    angle_sums(p, q, a, frame, taps, ar, as);
+    r = cadd(r, csroot(ar));
+    s = cadd(s, csroot(as));
+  }
+  const float2 value = cmul(r, s);
+  if (p.signal && frame < p.nt) p.signal[v * p.nt + frame] = value;
+  return das::power_of(value);
+}
+
+// Power of one frame by DMAS-CCF-ACF (reference ensemble.cu:143-232): channel sums
+// for the DMAS and coherence terms, then angle sums for the angular coherence.
+__device__ __forceinline__ double dmas_frame(const das::Args& p, const Voxel& q, size_t v, int frame, WarpTaps& taps) {
+  float2 root = make_float2(0.f, 0.f), r = root, s = root;
+  float magnitude = 0.f, active = 0.f, er = 0.f, es = 0.f;
+  for (int ch = 0; ch < p.nc; ++ch) {
+    float2 cr, cs;
+    channel_sums(p, q, ch, frame, taps, cr, cs);
+    root = cadd(root, cadd(csroot(cr), csroot(cs)));
+    magnitude += hypotf(cr.x, cr.y) + hypotf(cs.x, cs.y);
+    bool act_r, act_s;
+    receive_delay(q.x, q.z, double(p.xe[ch]), p.c, p.fn, &act_r);
+    receive_delay(q.y, q.z, double(p.ye[ch]), p.c, p.fn, &act_s);
+    active += float(act_r) + float(act_s);
+  }
+  for (int a = 0; a < p.na; ++a) {
+    float2 ar, as;
+    angle_sums(p, q, a, frame, taps, ar, as);
+    r = cadd(r, ar);
+    s = cadd(s, as);
+    er += cabs2(ar);
+    es += cabs2(as);
+  }
+  const float inv = 1.0f / float(p.na);
+  const float dm = cabs2(root) - magnitude;
+  const float wc = (active > 0.f && magnitude > 0.f) ? fmaxf(dm, 0.f) / active / magnitude : 0.f;
+  const float nr = cabs2(r) * inv * inv, ns = cabs2(s) * inv * inv;
+  const float var = fmaxf(er * inv - nr, 0.f) + fmaxf(es * inv - ns, 0.f);
+  const float num = sqrtf(nr) * sqrtf(ns), den = nr + ns + var / 2 - num;
+  float power = den > 0.f ? dm * wc * (num / den) : 0.f;
+  if (!isfinite(power)) power = 0.f;
+  if (p.signal && frame < p.nt) p.signal[v * p.nt + frame] = make_float2(power, 0.f);
+  return double(power);
+}
+
+// St-SW, one frame: the K x K correlation series (below) and r conj(q) of the aperture sums.
+template <int K>
+__device__ __forceinline__ float2 stsw_frame(const das::Args& p, const Voxel& q, size_t v, int frame, WarpTaps& taps) {
+  float2 r = make_float2(0.f, 0.f), s = r, mr[K] = {}, ms[K] = {};
+  float vr[K] = {}, vs[K] = {};
+  for (int a = 0; a < p.na; ++a) {
+    float2 ar, as;
+    angle_sums(p, q, a, frame, taps, ar, as);
+    r = cadd(r, ar);
+    s = cadd(s, as);
+    // Welford update of subset a % K, whose (a / K + 1)-th angle this is.
+    const float inv = 1.0f / float(a / K + 1);
+#pragma unroll
+    for (int i = 0; i < K; ++i) {
+      if (i != a % K) continue;
+      const float2 dr = make_float2(ar.x - mr[i].x, ar.y - mr[i].y), ds = make_float2(as.x - ms[i].x, as.y - ms[i].y);
+      mr[i] = make_float2(fmaf(dr.x, inv, mr[i].x), fmaf(dr.y, inv, mr[i].y));
+      ms[i] = make_float2(fmaf(ds.x, inv, ms[i].x), fmaf(ds.y, inv, ms[i].y));
+      vr[i] += dr.x * (ar.x - mr[i].x) + dr.y * (ar.y - mr[i].y);
+      vs[i] += ds.x * (as.x - ms[i].x) + ds.y * (as.y - ms[i].y);
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < K; ++i) {
+    const float ni = float((p.na - 1 - i) / K + 1);  // angles i, i + K, ... < na
+#pragma unroll
+    for (int j = 0; j < K; ++j) {
+      const float nj = float((p.na - 1 - j) / K + 1);
+      const float2 value = das::correlation(mr[i], vr[i] / ni, ms[j], vs[j] / nj);
+      if (frame < p.nt) p.series[(v * (K * K) + size_t(i * K + j)) * size_t(p.nt) + size_t(frame)] = value;
+    }
+  }
+  return cmul(r, cconj(s));
+}
+
+__device__ __forceinline__ double warp_sum(double x) {
+#pragma unroll
+  for (int off = 16; off > 0; off >>= 1) x += __shfl_xor_sync(0xffffffffu, x, off);
+  return x;
+}
+
+// MODE as in das_rows.cuh: kFmas, kDmas or kStsw + K.  Ten CTAs of St-SW per SM (48
+// registers) hide more of the gathers than nine (8192 voxels, 64 frames, 128 channels, 11
+// angles: 4.41 -> 3.33 ms; twelve, with spills, 3.55).
+template <int MODE>
+__global__ void __launch_bounds__(kWarps * 32, MODE > das::kStsw ? 10 : 1) ensemble_warps(const __grid_constant__ das::Args p) {
+  __shared__ __align__(16) WarpTaps all[kWarps];
+  const size_t v = size_t(blockIdx.x) * kWarps + (threadIdx.x >> 5);
+  if (v >= size_t(p.nv)) return;
+  WarpTaps& taps = all[threadIdx.x >> 5];
+  const int lane = threadIdx.x & 31, frame = int(blockIdx.y) * 32 + lane;
+  const Voxel q = load_voxel(p.scan, v);
+  double re = 0.0, im = 0.0;
+  if constexpr (MODE == das::kFmas) {
+    re = fmas_frame(p, q, v, frame, taps);
+  } else if constexpr (MODE == das::kDmas) {
+    re = dmas_frame(p, q, v, frame, taps);
+  } else {
+    const float2 cross = stsw_frame<das::kSubsets<MODE>>(p, q, v, frame, taps);
+    re = double(cross.x);
+    im = double(cross.y);
+  }
+  // Frames past the end are sums of nothing: zeros.
+  re = warp_sum(re);
+  if constexpr (das::kCross<MODE>) im = warp_sum(im);
+  if (lane == 0) {
+    atomicAdd(p.pd + 2 * v, float(re / double(p.nt)));
+    if constexpr (das::kCross<MODE>) atomicAdd(p.pd + 2 * v + 1, float(im / double(p.nt)));
+  }
+}
+
 // ------------------------------------------------------------ St-SW --
 // St-SW (method 4; reference stsw.py:10-107, ensemble.cu:457-627).  Angles of
 // each aperture fall into K interleaved subsets (a % K).  Per frame: the
@@ -38,7 +228,7 @@ __device__ __forceinline__ Tap tap_of(const Voxel& q, int config, const float* e
 // E the series energies; the power is the XDoppler |mean_t r conj(q)|.
 //
 // The series come from the staged kernel (das_rows.cuh), whose angles run subset by
-// subset; it also sums r conj(q) into pd[2v], pd[2v + 1].
+// subset, or from ensemble_warps; both also sum r conj(q) into pd[2v], pd[2v + 1].
 //
 // stsw_finish (one warp per voxel): series energies over frames, then the pair sum
 // with running row / column sums of the normalized series (for row i, the

@@ -751,6 +751,20 @@ __host__ __device__ constexpr int min_ctas(int pairs) {
   return MODE == kOpw && pairs <= 8 ? 2 : 1;
 }
 
+// |x|^2 in float64.
+__device__ __forceinline__ double power_of(float2 x) {
+  return fma(double(x.x), double(x.x), double(x.y) * double(x.y));
+}
+
+// Correlation of two subsets from their means and mean squared deviations (reference
+// stsw.py:45-66); zero where it has no value.
+__device__ __forceinline__ float2 correlation(float2 r, float spread_r, float2 q, float spread_q) {
+  const float2 num = cmul(r, cconj(q));
+  const float den = cabs2(r) + cabs2(q) + (spread_r + spread_q) * 0.5f - hypotf(num.x, num.y);
+  const float2 value = den > 0.f ? make_float2(num.x / den, num.y / den) : make_float2(0.f, 0.f);
+  return isfinite(value.x) && isfinite(value.y) ? value : make_float2(0.f, 0.f);
+}
+
 // A consumer thread owns one voxel (a warp 32 of them) and one group of frames.
 template <int MODE, int PAIRS, bool HALF, bool BOXES>
 struct Consumer {
@@ -1016,11 +1030,6 @@ struct Consumer {
     return true;
   }
 
-  // |x|^2 in float64.
-  static __device__ __forceinline__ double power_of(float2 x) {
-    return fma(double(x.x), double(x.x), double(x.y) * double(x.y));
-  }
-
   // The frames' values and, in float64, their power.  A thread adds up to 26 frames
   // one after another: in float32 that showed in the power maps (48 x 96 x 48 voxels,
   // 384 x 128 x 7 x 64, RC-FMAS: 1.4e-7 from float64, 5.9e-8 with these sums; 40 x 70 x
@@ -1089,11 +1098,7 @@ struct Consumer {
     for (int i = 0; i < K; ++i) {
 #pragma unroll
       for (int j = 0; j < K; ++j) {
-        const float2 num = cmul(mean[0][i], cconj(mean[1][j]));
-        const float den = cabs2(mean[0][i]) + cabs2(mean[1][j]) + (spread[0][i] + spread[1][j]) * 0.5f -
-                          hypotf(num.x, num.y);
-        float2 value = den > 0.f ? make_float2(num.x / den, num.y / den) : make_float2(0.f, 0.f);
-        if (!isfinite(value.x) || !isfinite(value.y)) value = make_float2(0.f, 0.f);
+        const float2 value = correlation(mean[0][i], spread[0][i], mean[1][j], spread[1][j]);
         p.series[(size_t(v) * (K * K) + size_t(i * K + j)) * size_t(p.nt) + size_t(first + k)] = value;
       }
     }

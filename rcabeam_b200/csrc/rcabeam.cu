@@ -321,12 +321,40 @@ static rcabeam_status run_rows(const das::Args& a, cudaStream_t stream = 0) {
   }
 }
 
+// Whether a call of a nonlinear method has too few voxel tiles for the staged kernel
+// and runs a warp per voxel (das_generic.cuh).  The staged kernel's time is its items'
+// latency, and long with windows of tens of rows (few voxels over a wide aperture): a
+// warp per voxel is as fast there up to 16000-32000 warps, in compact grids up to 4000-8000
+// while the items fit one wave and to 16000 in two (64 channels, 5 angles, RC-FMAS, staged
+// against warps, ms: 8000 voxels over 10 mm x 2 frames 0.59 / 0.40, within 2 mm 0.35 /
+// 0.40; 16000 x 2 0.58 / 0.73 and 0.35 / 0.74; 8000 x 64 1.03 / 0.79 and 0.82 / 0.73; 16000 x
+// 64 1.15 / 1.39 and 0.78 / 1.29).
+static bool few_voxels(int method, size_t nv, size_t nt) {
+  if (method < 2 || method > 4) return false;
+  const size_t warps = nv * ((nt + 31) / 32), tiles = (nv + das::kTileVoxels - 1) / das::kTileVoxels;
+  return warps <= 8192 || (warps <= 16384 && tiles * ((nt + 15) / 16) > size_t(sm_count()));
+}
+
+template <int MODE>
+static rcabeam_status run_warps(const das::Args& a, cudaStream_t stream = 0) {
+  const dim3 grid(blocks_for(size_t(a.nv), generic::kWarps), blocks_for(size_t(a.nt), 32));
+  generic::ensemble_warps<MODE><<<grid, generic::kWarps * 32, 0, stream>>>(a);
+  return launch_status();
+}
+
+// Subset statistics and series of St-SW with K subsets (a.series).
+template <int K>
+static rcabeam_status run_stsw(const das::Args& a) {
+  return few_voxels(4, size_t(a.nv), size_t(a.nt)) ? run_warps<das::kStsw + K>(a) : run_rows<das::kStsw + K, false>(a);
+}
+
 // Methods 0-3 and 5 of the float32 path on `stream`.
 static rcabeam_status run_method(const das::Args& a, int method, cudaStream_t stream = 0) {
+  const bool few = few_voxels(method, size_t(a.nv), size_t(a.nt));
   switch (method) {
     case 0: return run_rows<das::kOpw, false>(a, stream);
-    case 2: return run_rows<das::kFmas, false>(a, stream);
-    case 3: return run_rows<das::kDmas, false>(a, stream);
+    case 2: return few ? run_warps<das::kFmas>(a, stream) : run_rows<das::kFmas, false>(a, stream);
+    case 3: return few ? run_warps<das::kDmas>(a, stream) : run_rows<das::kDmas, false>(a, stream);
     case 5: return run_rows<das::kApertures, false>(a, stream);
     default: break;
   }
@@ -508,14 +536,12 @@ static rcabeam_status ensemble_impl(const void* rc, const void* cr, const float*
   a.fn = double(fn);
   a.err = device_error_ptr();
   // The caller owns 2 * nv * (nc + na) float4 of scratch (reference rcabeam.h:196).
-  a.order = voxel_order(scan, nv, geometry_workspace, 2 * nv * (nc + na) * 16);
+  if (!few_voxels(method, nv, nt)) a.order = voxel_order(scan, nv, geometry_workspace, 2 * nv * (nc + na) * 16);
   if (method == 4) {
     // St-SW: series into the caller's workspace (nv k^2 nt complex64), then
     // energies, pair sums, raw weights and the XDoppler magnitude.
     a.series = static_cast<float2*>(workspace);
-    const rcabeam_status st = k == 2   ? run_rows<das::kStsw + 2, false>(a)
-                              : k == 3 ? run_rows<das::kStsw + 3, false>(a)
-                                       : run_rows<das::kStsw + 4, false>(a);
+    const rcabeam_status st = k == 2 ? run_stsw<2>(a) : k == 3 ? run_stsw<3>(a) : run_stsw<4>(a);
     if (st != RCABEAM_SUCCESS) return st;
     const unsigned blocks = blocks_for(nv, generic::kWarps);
     auto finish = k == 2 ? generic::stsw_finish<2> : k == 3 ? generic::stsw_finish<3> : generic::stsw_finish<4>;
@@ -818,8 +844,10 @@ static rcabeam_status ensemble_static(const void* rc, const void* cr, const floa
   a.err = device_error_ptr();
   // The sort rewrites keys, values and the bounding box (cleared inside) on every call.
   // Calls too small to need an order run in identity order; a failed sort is an error.
-  a.order = voxel_order(scan, nv, scratch, kStaticScratchBytes);
-  if (!a.order && order_bytes(nv, nullptr)) return RCABEAM_ERROR_CUDA;
+  if (!few_voxels(method, nv, nt)) {
+    a.order = voxel_order(scan, nv, scratch, kStaticScratchBytes);
+    if (!a.order && order_bytes(nv, nullptr)) return RCABEAM_ERROR_CUDA;
+  }
   return run_method(a, method);
 }
 

@@ -38,7 +38,7 @@ def _voxels(kind: str, nv: int, rng) -> np.ndarray:
     return scan.astype(np.float32)
 
 
-def _reconstruct(rc, cr, scan, xe, ye, angles, starts, fn, method, shift, fd=FD):
+def _reconstruct(rc, cr, scan, xe, ye, angles, starts, fn, method, shift, fd=FD, k=2):
     ns, nc, na, nt = rc.shape
     dev = lambda a: torch.from_numpy(np.ascontiguousarray(a)).cuda()  # noqa: E731
     packed = []
@@ -51,11 +51,17 @@ def _reconstruct(rc, cr, scan, xe, ye, angles, starts, fn, method, shift, fd=FD)
     pd = torch.empty((nv, 2), dtype=torch.float32, device="cuda")
     planes = 2 if method == 5 else 1
     signal = torch.full((nv * planes, nt), float("nan"), dtype=torch.complex64, device="cuda")
+    weights = series = None
+    if method == 4:
+        weights, signal = torch.empty(nv, dtype=torch.float32, device="cuda"), None
+        series = torch.empty(nv * k * k * nt, dtype=torch.complex64, device="cuda")
     work = torch.empty(_cuda_impl.workspace_bytes(nv, nc, na), dtype=torch.uint8, device="cuda")
     t = [dev(a) for a in (scan, xe, ye, angles, starts)]
     _lib.call("rcabeam_ensemble_device", packed[0].data_ptr(), packed[1].data_ptr(), *(a.data_ptr() for a in t),
-              pd.data_ptr(), signal.data_ptr(), None, None, work.data_ptr(), ns, nc, na, nt, nv, C, FS, fd,
-              -1.0 if fn is None else fn, method, 2)
+              pd.data_ptr(), *(None if a is None else a.data_ptr() for a in (signal, weights, series)), work.data_ptr(),
+              ns, nc, na, nt, nv, C, FS, fd, -1.0 if fn is None else fn, method, k)
+    if method == 4:
+        return pd[:, 0].cpu().numpy(), weights.cpu().numpy()
     return pd[:, 0].cpu().numpy(), signal.cpu().numpy().reshape(nv, planes, nt)
 
 
@@ -97,6 +103,33 @@ def test_staged_splits_match_oracle(frames, kind, nv, na, fn, shift):
     assert rel_l2(pd, np.mean(np.abs(fmas) ** 2, axis=-1)) <= 1e-4
     pd, _ = run(3)
     assert rel_l2(pd, methods.dmas_ccf_acf_power(rc, cr, *geom)) <= 1e-4
+
+
+@pytest.mark.parametrize("method,k", [(2, 2), (3, 2), (4, 2), (4, 3), (4, 4)])
+@pytest.mark.parametrize("frames,kind,nv,na,fn,shift", [
+    (1, "dense", 127, 4, None, 0), (17, "coarse", 300, 5, 1.0, 1), (26, "dense", 1, 4, 1.0, 1),
+    (33, "apart", 257, 35, None, 0), (48, "coarse", 130, 5, 1.0, 0), (49, "dense", 150, 4, None, 1),
+    (97, "coarse", 129, 6, None, 0),
+])
+def test_nonlinear_routes_agree(method, k, frames, kind, nv, na, fn, shift):
+    """A few voxels (a warp each) and the same voxels repeated until the call takes the
+    staged kernel, on tiles of one voxel's repetitions and on mixed ones (1e-4: products of sums)."""
+    rng = np.random.default_rng(frames + nv)
+    ns, nc = 200, 37  # more channels than a warp has lanes, angles too with 35
+    scan = _voxels(kind, nv, rng)
+    xe = np.linspace(-4e-3, 4e-3, nc).astype(np.float32)
+    angles = np.linspace(-0.17, 0.16, na).astype(np.float32)
+    starts = np.full(na, 2 * 3e-3 / C - 0.4e-6, np.float32)
+    shape = (ns, nc, na, frames)
+    rc, cr = ((rng.normal(size=shape) + 1j * rng.normal(size=shape)).astype(np.complex64) for _ in range(2))
+    repeats = 16384 // (nv * -(-frames // 32)) + 1
+    args = (xe, xe + np.float32(1e-4), angles, starts, fn, method, shift)
+    pd, extra = _reconstruct(rc, cr, scan, *args, k=k)
+    pd_staged, extra_staged = _reconstruct(rc, cr, np.tile(scan, (repeats, 1)), *args, k=k)
+    assert np.abs(pd).max() > 0
+    for copy in (slice(0, nv), slice(len(pd_staged) - nv, None)):
+        assert rel_l2(pd_staged[copy], pd) <= 1e-4
+        assert rel_l2(extra_staged[copy], extra) <= 1e-4
 
 
 @pytest.mark.parametrize("method,specs", [
