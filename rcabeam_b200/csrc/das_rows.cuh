@@ -218,8 +218,8 @@ __device__ __forceinline__ void expect_tx(uint64_t* bar, uint32_t bytes) {
 
 // A copy of [start, start + len) of the buffer [lo, hi) puts byte `start` at
 // dst + (start & 15).  widen() gives the 16-byte bounds [a, b) of the bulk copy,
-// which stay inside the buffer; what they leave out (an unaligned first or last
-// sample of the whole ensemble) stage_copy() stores by hand, E bytes at a time.
+// which stay inside the buffer; what they leave out (an unaligned first sample of the
+// whole ensemble, or last one of a slab) stage_copy() stores by hand, E bytes at a time.
 __device__ __forceinline__ uint32_t widen(uintptr_t start, uintptr_t len, uintptr_t lo, uintptr_t hi, uintptr_t* a,
                                           uintptr_t* b) {
   *a = start & ~uintptr_t(15);
@@ -393,6 +393,8 @@ struct Builder {
       if (past_end) count = p.ns - base;
       uintptr_t a, b;
       if (sp.contiguous) {
+        // Not a byte of the next slab: its place is the row of zeros stored below.
+        if (past_end) hi = row0 + uintptr_t(count) * stride;
         if (lane == 0) {
           expect_tx(bar, widen(row0, count * stride, lo, hi, &a, &b));
           stage_copy<E>(data, row0, count * stride, a, b, bar);

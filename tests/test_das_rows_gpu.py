@@ -38,7 +38,8 @@ def _voxels(kind: str, nv: int, rng) -> np.ndarray:
     return scan.astype(np.float32)
 
 
-def _reconstruct(rc, cr, scan, xe, ye, angles, starts, fn, method, shift, fd=FD, k=2):
+def _reconstruct(rc, cr, scan, xe, ye, angles, starts, fn, method, shift, c=C, fs=FS, fd=FD,
+                 k=2):
     ns, nc, na, nt = rc.shape
     dev = lambda a: torch.from_numpy(np.ascontiguousarray(a)).cuda()  # noqa: E731
     packed = []
@@ -59,7 +60,7 @@ def _reconstruct(rc, cr, scan, xe, ye, angles, starts, fn, method, shift, fd=FD,
     t = [dev(a) for a in (scan, xe, ye, angles, starts)]
     _lib.call("rcabeam_ensemble_device", packed[0].data_ptr(), packed[1].data_ptr(), *(a.data_ptr() for a in t),
               pd.data_ptr(), *(None if a is None else a.data_ptr() for a in (signal, weights, series)), work.data_ptr(),
-              ns, nc, na, nt, nv, C, FS, fd, -1.0 if fn is None else fn, method, k)
+              ns, nc, na, nt, nv, c, fs, fd, -1.0 if fn is None else fn, method, k)
     if method == 4:
         return pd[:, 0].cpu().numpy(), weights.cpu().numpy()
     return pd[:, 0].cpu().numpy(), signal.cpu().numpy().reshape(nv, planes, nt)
@@ -184,6 +185,21 @@ def test_queue_of_long_windows(method, frames):
     for e, w in zip(ensembles, want):
         assert np.abs(w).min() > 0
         assert rel_l2(e.power().cpu().numpy(), w) <= 1e-5
+
+
+@pytest.mark.parametrize("frames,shift", [(15, 0), (15, 1), (33, 0), (16, 1)])
+def test_last_sample_keeps_the_next_slab_out(frames, shift):
+    """A tap on a slab's last sample weighs the row behind it by zero: that row is zeros, not
+    the next slab's samples (NaN here, of an angle whose window no voxel reaches)."""
+    ns = 65
+    rc = np.ones((ns, 1, 2, frames), np.complex64)
+    rc[:, :, 1] = np.nan
+    scan = np.array([[0.0, 2.0**-8, 0.0]], np.float32)  # delay 2^-17 s: sample 128 - 64, the last
+    zero = np.zeros(1, np.float32)
+    starts = np.array([64 * 2.0**-24, 1.0], np.float32)
+    pd, iq = _reconstruct(rc, np.zeros_like(rc), scan, zero, zero, np.zeros(2, np.float32), starts, None, 0, shift,
+                          c=2.0**10, fs=2.0**24, fd=0.0)
+    assert np.array_equal(iq[0, 0], np.ones(frames, np.complex64)) and pd[0] == 1.0
 
 
 @pytest.mark.parametrize("method", [0, 1])
