@@ -239,6 +239,7 @@ __device__ __forceinline__ void stage_copy(unsigned char* dst, uintptr_t start, 
     *reinterpret_cast<W*>(origin + q) = *reinterpret_cast<const W*>(q);
   for (uintptr_t q = b > start ? b : start; q < start + len; q += E)
     if (q >= a) *reinterpret_cast<W*>(origin + q) = *reinterpret_cast<const W*>(q);
+  if (start < a || b < start + len) fence_async_smem();  // a later window's copy may cover these bytes
 }
 
 // Sample position in float64, in the operation order of the float64 oracle:
@@ -419,6 +420,7 @@ struct Builder {
         unsigned char* past = data + unsigned(row0 & 15) + count * sp.pitch;
         const int words = (sp.contiguous ? p.nt : sp.frames) * (E / 4);
         for (int i = lane; i < words; i += 32) reinterpret_cast<unsigned*>(past)[i] = 0u;
+        fence_async_smem();  // a later window's copy covers these bytes
       }
     }
   }
@@ -1136,6 +1138,7 @@ __device__ __forceinline__ bool run_item(const Args& p, const Shape& sp, const L
   bool ok;
   if (warp < lt.builders + lt.helpers) {
     const bool helper = kAngleMajor<MODE> && warp >= lt.builders;
+    fence_async_smem();  // with another ring, copies fall where the item before kept taps
     Builder<HALF, BOXES> b(p, sp, lt, sh, ring, maps, frame0, helper ? warp - lt.builders : warp, phase);
     if constexpr (kAngleMajor<MODE>) {
       if (helper)
