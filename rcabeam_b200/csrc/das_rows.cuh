@@ -535,11 +535,13 @@ struct Builder {
   }
 
   // Both apertures, channel by channel; tag = first + aperture * nc + channel.
-  // Each builder forms the receive delays of one channel of a block for all.
+  // Each builder forms the receive delays of one channel of a block for all, in one of
+  // two slots in turn (over both apertures: the barrier of the block between two uses of
+  // a slot is what ends its reads).
   __device__ __forceinline__ void walk_channels(int first) {
+    int half = 0;
     for (int cfg = 0; cfg < 2; ++cfg) {
       fill_table(cfg);
-      int half = 0;
       for (int c0 = 0; c0 < p.nc; c0 += lt.builders, half ^= 1) {
         if (c0 + warp < p.nc) {
           long long rx[4];
