@@ -173,6 +173,14 @@ static const unsigned* voxel_order(const float* scan, size_t nv, void* workspace
 // ---------------------------------------------------------- dispatch --
 static unsigned blocks_for(size_t n, unsigned threads) { return unsigned((n + threads - 1) / threads); }
 
+// Lets a kernel ask for all shared memory that its `fixed` static bytes leave.  Every
+// call sets the same limit: one set to its own need could come between another
+// thread's larger limit and launch, which would then fail.
+template <typename K>
+static bool open_smem(K* kern, int fixed = 0) {
+  return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024 - fixed) == cudaSuccess;
+}
+
 static int sm_count() {
   int dev = 0, sms = 148;
   cudaGetDevice(&dev);
@@ -294,8 +302,7 @@ static RowsPlan plan_rows(const das::Args& a, bool half, int sms, int max_frames
 template <int MODE, int PAIRS, bool HALF, bool BOXES>
 static rcabeam_status launch_rows(const das::Args& a, const RowsPlan& r, unsigned items, cudaStream_t stream) {
   auto kern = das::das_rows<MODE, PAIRS, HALF, BOXES>;
-  if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, r.layout.smem) != cudaSuccess)
-    return RCABEAM_ERROR_CUDA;
+  if (!open_smem(kern)) return RCABEAM_ERROR_CUDA;
   kern<<<items, r.layout.threads, r.layout.smem, stream>>>(r.maps, a, r.shape, r.layout);
   return launch_status();
 }
@@ -477,8 +484,7 @@ static rcabeam_status run_tc(tc::Args a) {
               : stages == 4 ? tc::opw_tc<BF16X3, 4>
               : stages == 3 ? tc::opw_tc<BF16X3, 3>
                             : tc::opw_tc<BF16X3, 2>;
-  if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)) != cudaSuccess)
-    return RCABEAM_ERROR_CUDA;
+  if (!open_smem(kern)) return RCABEAM_ERROR_CUDA;
   a.partial = tc_partials_address();
   a.slot_clock = tc_slot_clock_address();
   if (!a.partial || !a.slot_clock) return RCABEAM_ERROR_CUDA;
@@ -639,9 +645,7 @@ static bool launch_async(const void* iq, void* out, double* power, size_t rows, 
   auto kern = clutter::project_rows_async<IN, MAXF>;
   const size_t smem = clutter::async_smem_bytes(k, nt, sizeof(IN));
   if (smem > 110 * 1024) return false;  // keep two CTAs per SM
-  if (smem > 48 * 1024 &&
-      cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)) != cudaSuccess)
-    return false;
+  if (smem > 48 * 1024 && !open_smem(kern)) return false;
   int dev = 0, sms = 148, per_sm = 2;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
@@ -659,7 +663,7 @@ static void launch_reg(const void* iq, void* out, double* power, size_t rows, si
                        int mode, unsigned* flags) {
   auto kern = clutter::project_rows_reg<F, K, H>;
   const size_t smem = clutter::reg_smem_bytes(nt);
-  if (smem > 48 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
+  if (smem > 48 * 1024) open_smem(kern);
   int dev = 0, sms = 148, per_sm = 3;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
@@ -676,7 +680,7 @@ static void launch_dmma(const void* iq, void* out, double* power, size_t rows, s
                         size_t k, unsigned* flags) {
   auto kern = clutter::project_power_dmma<8>;
   const size_t smem = clutter::dmma_smem_bytes(int((nt + 3) / 4));
-  if (smem > 48 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
+  if (smem > 48 * 1024) open_smem(kern);
   int dev = 0, sms = 148, per_sm = 2;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
@@ -766,8 +770,7 @@ static rcabeam_status gram_f64_launch(const void* iq, size_t rows, size_t nt, co
   const int stage = gramf64::stage_rows(int(nt));
   const size_t smem = size_t(2) * stage * prm.pitch * sizeof(double);
   auto kern = stage == 16 ? gramf64::gram_dmma<IN, 16> : gramf64::gram_dmma<IN, 8>;
-  if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)) != cudaSuccess)
-    return RCABEAM_ERROR_CUDA;
+  if (!open_smem(kern)) return RCABEAM_ERROR_CUDA;
   kern<<<unsigned(prm.units) * unsigned(prm.slices), gramf64::kThreads, smem>>>(static_cast<const IN*>(iq), prm);
   return launch_status();
 }
@@ -925,8 +928,7 @@ static rcabeam_status gram_tc_launch(const void* iq, size_t rows, size_t nt, con
     ++prm.ring;
   const size_t smem = std::max(gramtc::smem_bytes(prm.nload_max, prm.ring), size_t(120) << 10);
   auto kern = tf32 ? gramtc::gram_tc<true> : gramtc::gram_tc<false>;
-  if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)) != cudaSuccess)
-    return RCABEAM_ERROR_CUDA;
+  if (!open_smem(kern)) return RCABEAM_ERROR_CUDA;
   kern<<<unsigned(prm.nunits * prm.slices), gramtc::kThreads, smem>>>(map, prm);
   return launch_status();
 }
@@ -1023,9 +1025,7 @@ rcabeam_status rcabeam_ritz_matrix_device(const void* iq, size_t rows, size_t nt
   if (cudaMemsetAsync(h, 0, m * m * 2 * sizeof(double), 0) != cudaSuccess) return RCABEAM_ERROR_CUDA;
   const size_t smem = size_t(clutter::kRitzMax) * clutter::ritz_stride(int(nt)) * 16 +
                       size_t(clutter::kRefineRows) * clutter::kRitzMax * 16 + size_t(clutter::kRefineRows) * nt * 8;
-  if (cudaFuncSetAttribute(clutter::ritz_matrix, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)) !=
-      cudaSuccess)
-    return RCABEAM_ERROR_CUDA;
+  if (!open_smem(clutter::ritz_matrix)) return RCABEAM_ERROR_CUDA;
   int dev = 0, sms = 148;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
@@ -1621,8 +1621,7 @@ rcabeam_status rcabeam_batch_run_device(size_t n, const rcabeam_batch_ensemble* 
   const Kernel kern = list[0].method == 3   ? batch::run<das::kDmas>
                       : list[0].method == 1 ? batch::run<das::kXdoppler>
                                             : batch::run<das::kOpw>;
-  if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, layout.smem) != cudaSuccess)
-    return RCABEAM_ERROR_CUDA;
+  if (!open_smem(kern, 1024)) return RCABEAM_ERROR_CUDA;
   int resident = 1;
   if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, kern, layout.threads, layout.smem) != cudaSuccess)
     return RCABEAM_ERROR_CUDA;
@@ -1646,8 +1645,7 @@ rcabeam_status rcabeam_simulate_scene_device(const float* scatterers, size_t n, 
   if (chunk < 1) chunk = 1;
   if (chunk > nt) chunk = nt;
   const size_t smem = ns * chunk * sizeof(float2);
-  if (cudaFuncSetAttribute(scene::simulate, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)) != cudaSuccess)
-    return RCABEAM_ERROR_CUDA;
+  if (!open_smem(scene::simulate, 1024)) return RCABEAM_ERROR_CUDA;
   scene::Args a{};
   a.scatterers = scatterers;
   a.n = n;

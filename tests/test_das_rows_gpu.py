@@ -6,6 +6,8 @@ sums 1e-4)."""
 
 from __future__ import annotations
 
+import threading
+
 import numpy as np
 import pytest
 import torch
@@ -219,3 +221,32 @@ def test_power_sums_keep_small_frames(method, frames):
     want = (2.0**24 + frames - 1) / frames
     bound = -(-frames // 16) + (6 if method == 1 else 0)
     assert abs(float(pd[0]) - want) <= bound * 2.0**-24 * want
+
+
+def test_two_threads_of_different_sizes():
+    """Launches of one kernel that need different amounts of shared memory do not fail each other."""
+    errors = []
+
+    def work(frames):
+        rng = np.random.default_rng(frames)
+        shape = (8, 1, 1, frames)
+        rc = torch.from_numpy(rng.normal(size=shape).astype(np.complex64).transpose(1, 2, 0, 3).copy()).cuda()
+        zero = torch.zeros(3, dtype=torch.float32, device="cuda")
+        scan = torch.tensor([[0.0, 3e-3, 0.0]], device="cuda")
+        pd = torch.empty(2, dtype=torch.float32, device="cuda")
+        work = torch.empty(_cuda_impl.workspace_bytes(1, 1, 1), dtype=torch.uint8, device="cuda")
+        try:
+            for _ in range(2000):
+                _lib.call("rcabeam_ensemble_device", rc.data_ptr(), rc.data_ptr(), scan.data_ptr(), zero.data_ptr(),
+                          zero.data_ptr(), zero.data_ptr(), zero.data_ptr(), pd.data_ptr(), None, None, None,
+                          work.data_ptr(), 8, 1, 1, frames, 1, C, FS, FD, -1.0, 0, 2)
+        except _lib.RcabeamCudaError as e:
+            errors.append(e)
+
+    threads = [threading.Thread(target=work, args=(frames,)) for frames in (2, 16)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    torch.cuda.synchronize()
+    assert not errors
