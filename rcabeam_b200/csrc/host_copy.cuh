@@ -10,7 +10,6 @@
 
 #include <algorithm>
 #include <cstring>
-#include <system_error>
 #include <thread>
 #include <vector>
 
@@ -84,8 +83,9 @@ inline bool copy(void* host, void* device, size_t bytes, bool upload, void* pinn
   size_t started = 1;
   try {
     for (; started < n; ++started) threads.emplace_back(share, started);
-  } catch (const std::system_error&) {
-    // No more threads: the calling thread takes the remaining shares.
+  } catch (...) {
+    // No more threads, or no memory for one: the calling thread takes the remaining
+    // shares.  Nothing may leave here while threads run: their destructors would abort.
   }
   share(0);
   for (size_t i = started; i < n; ++i) share(i);
