@@ -21,8 +21,14 @@ from rcabeam_b200 import _lib
 _COMPLEX64 = (np.complex64, torch.complex64)
 # Device scratch for the St-SW correlation series of one voxel tile.
 _STSW_SCRATCH_BYTES = 256 << 20
-# Host arrays from this size on cross through pinned staging and several host threads.
-_STAGED_COPY_BYTES = 4 << 20
+# Host arrays from these sizes on cross through pinned staging and several host threads,
+# whose start costs about 0.4 ms.  Plain copies against staged ones, ms (16 host cores, 60 MiB
+# of cache; source out of / in the CPU's cache): up 4 MiB 0.45 / 0.66 and 0.29 / 0.48,
+# 12 MiB 1.19 / 1.13 and 0.67 / 1.11, 20 MiB 1.97 / 1.47 and 1.15 / 1.52, 32 MiB 3.09 / 1.71 and
+# 1.81 / 1.63; down into touched / fresh pages: 4 MiB 0.80 / 0.72 and 0.68 / 0.81, 8 MiB
+# 1.44 / 0.95 and 1.39 / 0.98, 32 MiB 3.9 / 1.9 and 17 / 2.2.
+_STAGED_UPLOAD_BYTES = 20 << 20
+_STAGED_DOWNLOAD_BYTES = 6 << 20
 _NUMPY_TYPE = {torch.float32: np.float32, torch.complex64: np.complex64}
 
 
@@ -54,7 +60,7 @@ def _host_copy(host: np.ndarray, device: torch.Tensor, upload: bool) -> None:
 def _download(device: torch.Tensor, host: np.ndarray) -> None:
     """Device tensor into a host array of the same shape (the device's work is complete); types convert."""
     same = host.dtype == _NUMPY_TYPE.get(device.dtype) and host.size == device.numel() and device.is_contiguous()
-    if same and host.flags.c_contiguous and host.flags.writeable and host.nbytes >= _STAGED_COPY_BYTES:
+    if same and host.flags.c_contiguous and host.flags.writeable and host.nbytes >= _STAGED_DOWNLOAD_BYTES:
         _host_copy(host, device, False)
     else:
         np.copyto(host, device.cpu().numpy())
@@ -66,7 +72,7 @@ def _to_device(a, dtype: torch.dtype) -> torch.Tensor:
             return a.to(_device(), dtype=dtype, non_blocking=False).contiguous()
         return a.to(dtype=dtype).contiguous()
     arr = np.ascontiguousarray(a)
-    if arr.nbytes >= _STAGED_COPY_BYTES and dtype == torch.complex64 and arr.dtype == np.complex64:
+    if arr.nbytes >= _STAGED_UPLOAD_BYTES and dtype == torch.complex64 and arr.dtype == np.complex64:
         out = torch.empty(arr.shape, dtype=dtype, device=_device())
         _host_copy(arr, out, True)
         return out

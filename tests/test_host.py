@@ -156,7 +156,7 @@ def test_depth_axis():
         rb.depth_axis(2.0, 1.0, 1e6)
 
 
-@pytest.mark.parametrize("elements", [1 << 10, 1 << 20])
+@pytest.mark.parametrize("elements", [1 << 10, 1 << 20, 1 << 22])
 @pytest.mark.parametrize("source,target", [("float32", "<f8"), ("float32", ">f4"), ("complex64", "<c16"),
                                            ("float32", "<f4"), ("complex64", "<c8")])
 def test_downloads_convert_types(monkeypatch, elements, source, target):

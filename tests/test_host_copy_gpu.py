@@ -49,7 +49,7 @@ def test_concurrent_uploads_from_two_threads():
         assert np.array_equal(d.cpu().numpy(), a)
 
 
-@pytest.mark.parametrize("voxels", [1000, 300_000])
+@pytest.mark.parametrize("voxels", [1000, 300_000, 700_000])
 def test_wider_host_outputs_are_converted(voxels):
     rng = np.random.default_rng(voxels)
     rc, cr = ((rng.normal(size=(64, 2, 1, 2)) + 1j * rng.normal(size=(64, 2, 1, 2))).astype(np.complex64)
@@ -66,3 +66,22 @@ def test_wider_host_outputs_are_converted(voxels):
     (pd, signal), (pd64, signal64) = results
     assert np.abs(signal).max() > 0
     assert np.array_equal(pd64, pd) and np.array_equal(signal64, signal)
+
+
+def test_concurrent_staged_copies():
+    hosts = [np.random.default_rng(i).integers(0, 255, 9 * CHUNK + 8 * i, dtype=np.uint8) for i in range(2)]
+    back = [np.zeros_like(h) for h in hosts]
+
+    def work(i):
+        device = torch.empty(hosts[i].nbytes, dtype=torch.uint8, device="cuda")
+        for _ in range(3):
+            _cuda_impl._host_copy(hosts[i], device, True)
+            _cuda_impl._host_copy(back[i], device, False)
+
+    threads = [threading.Thread(target=work, args=(i,)) for i in range(2)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    for h, b in zip(hosts, back):
+        assert np.array_equal(b, h)
