@@ -207,21 +207,20 @@ def _project(matrix: torch.Tensor, vectors_cm: torch.Tensor, k: int, mode: int, 
 
 def apply_temporal_filter(iq, basis, *, rank_start: int, rank_stop: int | None = None):
     """Filtered IQ keeping ranks [start, stop) via the smaller projector (gpu_clutter.py:219-241)."""
-    arrays = _inputs(iq, check_finite=False)  # the projection flags non-finite samples
-    frames = arrays[0].shape[-1]
     try:
+        arrays = _inputs(iq, check_finite=False)  # the projection flags non-finite samples
+        frames = arrays[0].shape[-1]
         start, stop = _rank_interval(frames, rank_start, rank_stop)
         vectors, subtract = _filter_vectors(basis, frames, start, stop)
+        result, flags = [], torch.zeros(len(arrays), dtype=torch.int32, device=arrays[0].device)
+        for i, a in enumerate(arrays):
+            m = _rows(a)
+            out = torch.empty_like(m)
+            _project(m, vectors, vectors.shape[0], (1 if subtract else 0) | 2, out, None, flags[i:])
+            result.append(out.reshape(a.shape))
     except ValueError:
-        _inputs(iq)  # non-finite IQ is reported first
+        _inputs(iq)  # non-finite IQ is reported before anything that follows its check
         raise
-    k = vectors.shape[0]
-    result, flags = [], torch.zeros(len(arrays), dtype=torch.int32, device=arrays[0].device)
-    for i, a in enumerate(arrays):
-        m = _rows(a)
-        out = torch.empty_like(m)
-        _project(m, vectors, k, (1 if subtract else 0) | 2, out, None, flags[i:])
-        result.append(out.reshape(a.shape))
     bits = flags.tolist()
     if any(b & 1 for b in bits):
         raise ValueError("IQ must be finite")
@@ -256,13 +255,13 @@ def filtered_power(iq, basis, *, rank_start: int, rank_stop: int | None = None) 
 def svd_clutter_filter(iq, *, rank_start: int, rank_stop: int | None = None, method: str = "gram",
                        precision: str = "complex128"):
     """Gram-EVD temporal filter keeping ranks [start, stop); no silent precision fallback (gpu_clutter.py:322-336)."""
-    arrays = _inputs(iq, check_finite=False)  # temporal_basis reports non-finite samples
     try:
+        arrays = _inputs(iq, check_finite=False)  # temporal_basis reports non-finite samples
         _rank_interval(arrays[0].shape[-1], rank_start, rank_stop)
-    except ValueError:
-        _inputs(iq)  # non-finite IQ is reported first
+        _, basis = temporal_basis(iq, method=method, precision=precision)
+    except (TypeError, ValueError):
+        _inputs(iq)  # non-finite IQ is reported before anything that follows its check
         raise
-    _, basis = temporal_basis(iq, method=method, precision=precision)
     return apply_temporal_filter(iq, basis, rank_start=rank_start, rank_stop=rank_stop)
 
 

@@ -470,3 +470,19 @@ def test_filter_flags_non_finite_rows_and_keeps_error_order():
             gpu_clutter.apply_temporal_filter(spike, basis, **ranks)
         with pytest.raises(np.linalg.LinAlgError, match="Nonfinite filtered IQ"):
             gpu_clutter.apply_temporal_filter(spike.to(torch.complex128) * 5e269, basis, **ranks)
+
+
+def test_non_finite_iq_is_reported_before_other_errors():
+    bad = torch.full((40, 36), complex(float("nan"), 0.0), dtype=torch.complex64, device="cuda")
+    eye = torch.eye(36, dtype=torch.complex128, device="cuda")
+    wide = torch.full((2, 514), complex(float("inf"), 0.0), dtype=torch.complex64, device="cuda")
+    calls = [lambda: gpu_clutter.svd_clutter_filter(bad, rank_start=1, method="evd"),
+             lambda: gpu_clutter.svd_clutter_filter(bad, rank_start=1, precision="half"),
+             lambda: gpu_clutter.svd_clutter_filter(bad[:, :35].contiguous(), rank_start=1, precision="tf32"),
+             lambda: gpu_clutter.svd_clutter_filter((bad, bad[:, :35]), rank_start=1),
+             lambda: gpu_clutter.apply_temporal_filter((bad, bad[:, :35]), eye, rank_start=1),
+             lambda: gpu_clutter.apply_temporal_filter(wide, torch.eye(514, dtype=torch.complex128, device="cuda"),
+                                                       rank_start=1)]
+    for call in calls:
+        with pytest.raises(ValueError, match="IQ must be finite"):
+            call()
