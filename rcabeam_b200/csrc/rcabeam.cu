@@ -1365,17 +1365,13 @@ rcabeam_status rcabeam_opw_offsets_forward_device(const void* rc, const void* cr
       !adjoint_geometry(&g, scan, voxels, nvl, xe, ye, angles, starts, offsets, c, fs, fd, fn, ns, nc, na, nt, frame0,
                         frames))
     return RCABEAM_ERROR_ARGUMENT;
-  // A warp per voxel until one thread per voxel fills the GPU by itself (2 x 128
-  // channels, 7 angles, 8 frames: 20000 voxels 2.1 against 3.5 ms, 100000 voxels
-  // 10.1 against 9.3 ms).
-  const bool warps = nvl < size_t(sm_count()) * 400;
-  const unsigned blocks = blocks_for(warps ? nvl * 32 : nvl, 128);
+  const unsigned blocks = blocks_for(nvl * 32, 128);
   if (complex128)
-    (warps ? adj::forward<double, 32> : adj::forward<double, 1>)<<<blocks, 128>>>(
-        g, static_cast<const double2*>(rc), static_cast<const double2*>(cr), static_cast<double2*>(iq), power);
+    adj::forward<double><<<blocks, 128>>>(g, static_cast<const double2*>(rc), static_cast<const double2*>(cr),
+                                          static_cast<double2*>(iq), power);
   else
-    (warps ? adj::forward<float, 32> : adj::forward<float, 1>)<<<blocks, 128>>>(
-        g, static_cast<const float2*>(rc), static_cast<const float2*>(cr), static_cast<float2*>(iq), power);
+    adj::forward<float><<<blocks, 128>>>(g, static_cast<const float2*>(rc), static_cast<const float2*>(cr),
+                                         static_cast<float2*>(iq), power);
   return launch_status();
 }
 
