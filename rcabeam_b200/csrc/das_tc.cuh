@@ -127,6 +127,15 @@ struct Args {
 constexpr float kReachLimit = 134217728.f;
 constexpr long long kNever = -(3ll << 61);
 
+// Transmit offsets are kept in units of 2^-bits samples, the finest in which 31 bits hold
+// any that a voxel (dx, dz, dy) from the first one can have: 29 bits next to it, 2 at the
+// limit, 0 beyond.  A unit for each voxel, so that a distant voxel in a tile does not
+// coarsen the others' offsets.
+__device__ __forceinline__ int offset_bits(double dx, double dz, double dy, double ks) {
+  const float far = float((fabs(dz) + fmax(fabs(dx), fabs(dy))) * ks);
+  return far < kReachLimit ? 29 - ilogbf(far + 1.f) : 0;
+}
+
 constexpr int kCtrlBytes = 512;  // barriers, stage tags, counters, TMEM slot
 
 template <bool BF16X3>
@@ -372,7 +381,7 @@ __global__ void __launch_bounds__(threads_for(STAGES), 1)
   double* angle_tab = reinterpret_cast<double*>(ctrl + kCtrlBytes);
   // Transmit delay (minus the angle's start) of (aperture, angle, voxel), in
   // 2^-32 samples = tx_base[aperture, angle] (the tile's first voxel) + tx_off
-  // times the tile's unit (2^-22 samples in a compact tile).
+  // times the voxel's unit (offset_bits).
   long long* tx_base = reinterpret_cast<long long*>(angle_tab + 3 * p.na);  // [2][na]
   int* tx_off = reinterpret_cast<int*>(tx_base + 2 * p.na);                 // [2][na][128]
   float2* tx_phase = reinterpret_cast<float2*>(tx_off + 2 * p.na * kVox);  // [2][na][128]
@@ -486,7 +495,7 @@ __global__ void __launch_bounds__(threads_for(STAGES), 1)
       // Voxels of this lane: slots lane + 32 j (group = slot / 64).
       double px[4], pz[4], py[4];
       bool pv[4];
-      float reach = 0.f;  // samples by which a transmit delay can differ from the first voxel's
+      int unit[4];
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
         const size_t q = size_t(tile) * kVox + lane + 32 * j;
@@ -496,14 +505,10 @@ __global__ void __launch_bounds__(threads_for(STAGES), 1)
         px[j] = double(p.scan[b3]);
         pz[j] = double(p.scan[b3 + 1]);
         py[j] = double(p.scan[b3 + 2]);
-        const float far = float((fabs(pz[j] - z0) + fmax(fabs(px[j] - x0), fabs(py[j] - y0))) * ks);
-        pv[j] = pv[j] && far < kReachLimit;
-        if (far < kReachLimit) reach = fmaxf(reach, far);
+        const int bits = offset_bits(px[j] - x0, pz[j] - z0, py[j] - y0, ks);
+        pv[j] = pv[j] && bits > 0;
+        unit[j] = bits > 0 ? 1 << (32 - bits) : 0;
       }
-      // Offsets in units of 2^-bits samples: the finest that holds the tile, 2^-22 at most.
-      reach = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(reach)));
-      const int bits = min(22, 29 - ilogbf(reach + 1.f));
-      const int unit = 1 << (32 - bits);
       // Per-tile transmit table, filled cooperatively by the builder warps.
       builders_sync();  // previous item's table reads are complete
       for (int e = warp * 32 + lane; e < 2 * p.na * kVox; e += kBuilders * 32) {
@@ -514,7 +519,7 @@ __global__ void __launch_bounds__(threads_for(STAGES), 1)
         const double x = double(p.scan[b3]), z = double(p.scan[b3 + 1]), y = double(p.scan[b3 + 2]);
         const double ref = fma(z0, angle_tab[3 * a], (config ? x0 : y0) * angle_tab[3 * a + 1]);
         const double path = fma(z, angle_tab[3 * a], (config ? x : y) * angle_tab[3 * a + 1]);
-        tx_off[e] = __double2int_rn((path - ref) * ks * double(1 << bits));
+        tx_off[e] = __double2int_rn((path - ref) * ks * double(1 << offset_bits(x - x0, z - z0, y - y0, ks)));
         if (v == 0) tx_base[ca] = das::fixed32(fma(ref, ks, -angle_tab[3 * a + 2] * p.fs));
         tx_phase[e] = demod_phase(kc, path);
       }
@@ -554,7 +559,7 @@ __global__ void __launch_bounds__(threads_for(STAGES), 1)
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
               const int ti = (config * p.na + a) * kVox + lane + 32 * j;
-              const long long at = rx[j] + base_tx + (long long)(tx_off[ti]) * unit;
+              const long long at = rx[j] + base_tx + (long long)(tx_off[ti]) * unit[j];
               i0[j] = int(at >> 32);
               w[j] = float(unsigned(at)) * 0x1p-32f;
               // Rows 1 ... ns - 3 are inside; the window's ends are decided in float64.

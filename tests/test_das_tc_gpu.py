@@ -108,3 +108,16 @@ def test_tc_many_angles_shallow_ring(storage, angles):
     expected = _oracle(*ref_in, ang, starts, grid, geom).reshape(6, 7, 5, 200)
     actual = rb.beamform_ensemble(rc, cr, ang, starts, grid, geom, iq_storage=storage)
     assert rel_l2(actual, expected) <= 5e-5
+
+
+@pytest.mark.parametrize("storage", ["float16", "bf16x2"])
+def test_tc_distant_voxel_in_a_tile(storage):
+    """One voxel 3 km away behind 126 close ones: the others' delays stay as fine as without it."""
+    grid = (np.array([0.0]), np.append(np.linspace(3e-3, 6e-3, 126), 3e3), np.array([0.0]))
+    rc, cr, _, starts, grid, geom = random_case(5, 200, 8, 3, 8, grid, fnumber=None, fs=20e6, fd=15e6,
+                                                starts=np.full(3, 2e-6))
+    angles = np.deg2rad([-10.0, 0.0, 10.0])
+    ref_in = (_quant(rc), _quant(cr)) if storage == "float16" else (rc, cr)
+    expected = _oracle(*ref_in, angles, starts, grid, geom).reshape(1, 127, 1, 8)
+    actual = rb.beamform_ensemble(rc, cr, angles, starts, grid, geom, iq_storage=storage)
+    assert rel_l2(actual, expected) <= 5e-5
