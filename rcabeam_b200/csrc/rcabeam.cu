@@ -743,11 +743,15 @@ static void project_dispatch(const void* iq, void* out, double* power, size_t ro
   if (flags && (mode & 2)) clutter::sample_flags<IN><<<296, 256>>>(static_cast<const IN*>(out), rows * nt, 4u, flags);
 }
 
-// Float64 Gram on the tensor cores: from 32768 samples on (1000 x 33: 16 us
-// against 15 us of gram_simt; 2048 x 200: 34 against 74 us), which also keeps
-// the few rows of tiny inputs in gram_simt's sequential order.
+// Float64 Gram on the tensor cores, where its 20 us of staging and slice sums are
+// repaid (complex64, us, gram_simt against gram_dmma: 1000 x 96 22 / 20, 512 x 128 18 / 23,
+// 2048 x 64 20.5 / 20.2, 2048 x 200 69 / 33).  Up to 32 frames its warps share few tiles and
+// gram_simt one: 12000 x 16 39 / 30 but 2048 x 16 15.8 / 16.0 and 8192 x 16 32 / 32; 12000 x 32
+// 42 / 45, 8192 x 32 33 / 46, 16384 x 32 78 / 57.  Small inputs also keep gram_simt's
+// sequential order.
 static bool gram_f64_eligible(size_t rows, size_t nt) {
-  return nt <= size_t(gramf64::kMaxFrames) && rows >= 256 && rows * nt >= 32768;
+  if (nt <= 32) return rows >= (nt <= 16 ? 12000 : 16384);
+  return nt <= size_t(gramf64::kMaxFrames) && rows * nt >= (size_t(1) << 17);
 }
 
 template <typename IN>

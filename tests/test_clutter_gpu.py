@@ -448,6 +448,14 @@ def test_float64_gram_tiles_and_slices(rows, nt, dtype):
     assert float(error) <= 16 * 2.0**-53 * rows**0.5
 
 
+@pytest.mark.parametrize("rows,nt", [(12000, 2), (12001, 16), (16384, 17), (16397, 32), (3973, 33), (1751, 75),
+                                     (600, 257)])
+@pytest.mark.parametrize("dtype", [torch.complex64, torch.complex128])
+def test_float64_gram_beside_its_line(rows, nt, dtype):
+    """The smallest inputs that the tensor-core form takes, per column count (bound as above)."""
+    test_float64_gram_tiles_and_slices(rows, nt, dtype)
+
+
 def test_filter_flags_non_finite_rows_and_keeps_error_order():
     """apply_temporal_filter reports non-finite IQ before a bad rank or basis, and an overflowing result."""
     iq = torch.ones((40, 36), dtype=torch.complex64, device="cuda")
