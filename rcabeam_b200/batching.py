@@ -53,7 +53,9 @@ def _declare():
     lib.rcabeam_batch_table_bytes.argtypes = [Z, arr, ctypes.POINTER(Z)]
     lib.rcabeam_batch_prepare.argtypes = [Z, arr, P, Z]
     lib.rcabeam_batch_run_device.argtypes = [Z, arr, P, Z, P, I, P]
-    for fn in (lib.rcabeam_batch_table_bytes, lib.rcabeam_batch_prepare, lib.rcabeam_batch_run_device):
+    lib.rcabeam_batch_launches.argtypes = [Z, arr, I, ctypes.POINTER(Z)]
+    for fn in (lib.rcabeam_batch_table_bytes, lib.rcabeam_batch_prepare, lib.rcabeam_batch_run_device,
+               lib.rcabeam_batch_launches):
         fn.restype = I
     lib._batch_declared = True
     return lib
@@ -140,15 +142,11 @@ class _SubQueue:
         self.ensembles = ensembles
 
     def kernel_launches(self) -> int:
-        """Kernels one launch() enqueues: the persistent kernel, or per ensemble its
-        delay-and-sum (XDoppler with its magnitude pass) and a completion stamp,
-        plus the start stamp."""
-        if self.ctas_per_sm:
-            return 1
-        total = 1
-        for e in self.ensembles:
-            total += 2 + (e.method == "xdoppler")
-        return total
+        """Kernels one launch() enqueues (one where the sub-queue runs persistently)."""
+        count = ctypes.c_size_t(0)
+        _lib.check(self.lib.rcabeam_batch_launches(len(self.indices), self.list, self.ctas_per_sm,
+                                                   ctypes.byref(count)), "batch_launches")
+        return count.value
 
     def launch(self, stream) -> None:
         _lib.check(self.lib.rcabeam_batch_run_device(len(self.indices), self.list, self.table.data_ptr() + self.base,
@@ -211,8 +209,11 @@ class BatchQueue:
         return out
 
 
+_TILE_VOXELS = 128  # voxels of one work item
+
+
 def _sample(e: Ensemble, tiles: int) -> int:
-    return min(e.voxels, 64 * tiles)
+    return min(e.voxels, _TILE_VOXELS * tiles)
 
 
 def autotune(ensembles, *, sample_tiles: int = 148 * 2, repeats: int = 2, cache: dict | None = None) -> dict:
@@ -263,10 +264,11 @@ def autotune(ensembles, *, sample_tiles: int = 148 * 2, repeats: int = 2, cache:
             if not reps:
                 budgets[method] = 1
                 continue
-            # Persistent kernel at 2 or 3 CTAs per SM, or per-ensemble grids (0): which one wins
-            # depends on the ensembles' size, so the sample is eight times the frame-chunk one.
-            results = {k: timed(BatchQueue(reps, ctas_per_sm=k, voxel_limit=8 * 64 * sample_tiles))
-                       for k in (0, 2, 3)}
+            # Persistent kernel (with all the CTAs that fit an SM: one, but for short ensembles) or
+            # per-ensemble grids (0): which one wins depends on the ensembles' size, so the
+            # sample is eight times the frame-chunk one.
+            results = {k: timed(BatchQueue(reps, ctas_per_sm=k, voxel_limit=8 * _TILE_VOXELS * sample_tiles))
+                       for k in (0, 3)}
             budgets[method] = min(results, key=results.get)
         cache["ctas_per_sm"] = budgets
     return {**{str(k): v for k, v in cache.items() if k != "ctas_per_sm"}, "ctas_per_sm": cache["ctas_per_sm"]}

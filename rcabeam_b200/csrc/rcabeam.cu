@@ -1546,6 +1546,13 @@ bool batch_plan(size_t n, const rcabeam_batch_ensemble* list, std::vector<batch:
   return true;
 }
 
+// Whether a queue runs as one persistent kernel: one method, and a layout that fits.
+bool batch_persistent(size_t n, const rcabeam_batch_ensemble* list, int ctas_per_sm, const das::Layout& layout) {
+  for (size_t i = 1; i < n; ++i)
+    if (list[i].method != list[0].method) return false;
+  return ctas_per_sm > 0 && layout.smem > 0;
+}
+
 batch::Queue batch_queue(void* table, size_t n, const BatchLayout& L, long long total, const das::Layout& layout,
                          unsigned long long* times) {
   unsigned char* t = static_cast<unsigned char*>(table);
@@ -1604,9 +1611,7 @@ rcabeam_status rcabeam_batch_run_device(size_t n, const rcabeam_batch_ensemble* 
     return RCABEAM_ERROR_CUDA;
   for (size_t i = 0; i < n; ++i)
     if (cudaMemsetAsync(list[i].pd, 0, 2 * list[i].nv * sizeof(float), st) != cudaSuccess) return RCABEAM_ERROR_CUDA;
-  bool one_method = true;
-  for (size_t i = 1; i < n; ++i) one_method = one_method && list[i].method == list[0].method;
-  if (ctas_per_sm == 0 || !one_method || !layout.smem) {
+  if (!batch_persistent(n, list, ctas_per_sm, layout)) {
     // Each ensemble through the single-ensemble kernels on the stream, a
     // completion stamp after each.
     batch::stamp<<<1, 1, 0, st>>>(times, 1);
@@ -1629,6 +1634,19 @@ rcabeam_status rcabeam_batch_run_device(size_t n, const rcabeam_batch_ensemble* 
   kern<<<unsigned(std::min(total, want)), layout.threads, layout.smem, st>>>(
       batch_queue(table, n, L, total, layout, times));
   return launch_status();
+}
+
+rcabeam_status rcabeam_batch_launches(size_t n, const rcabeam_batch_ensemble* list, int ctas_per_sm,
+                                      size_t* launches) {
+  BatchLayout L;
+  long long total = 0;
+  das::Layout layout{};
+  if (!launches || ctas_per_sm < 0 || ctas_per_sm > 3 || !batch_plan(n, list, nullptr, &L, &total, &layout))
+    return RCABEAM_ERROR_ARGUMENT;
+  *launches = 1;  // the persistent kernel, or the start stamp
+  if (!batch_persistent(n, list, ctas_per_sm, layout))
+    for (size_t i = 0; i < n; ++i) *launches += list[i].method == 1 ? 3 : 2;  // XDoppler: magnitudes too; a stamp
+  return RCABEAM_SUCCESS;
 }
 
 rcabeam_status rcabeam_simulate_scene_device(const float* scatterers, size_t n, const float* elements,

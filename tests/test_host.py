@@ -174,3 +174,23 @@ def test_downloads_convert_types(monkeypatch, elements, source, target):
     host = np.zeros(device.shape, target)
     _cuda_impl._download(device, host)
     assert np.array_equal(host, device.numpy())
+
+
+def test_queue_launches_follow_the_layout(built_library):
+    """One kernel where a method's ensembles share a layout; per ensemble one and a time stamp
+    (XDoppler two) where a long angle table beside wide stashes leaves no room, or methods differ."""
+    from rcabeam_b200 import batching
+
+    lib = batching._declare()
+
+    def launches(ctas, *specs):
+        items = [batching.BatchEnsembleC(*[256] * 9, 200, 8, na, nt, 500, 1540.0, 20e6, 5e6, -1.0,
+                                         batching.METHODS[method], 64) for method, nt, na in specs]
+        count = ctypes.c_size_t(0)
+        assert lib.rcabeam_batch_launches(len(items), (batching.BatchEnsembleC * len(items))(*items), ctas,
+                                          ctypes.byref(count)) == 0
+        return count.value
+
+    assert launches(3, ("dmas", 48, 5), ("dmas", 20, 7)) == 1
+    assert launches(3, ("dmas", 48, 5), ("dmas", 7, 64)) == 5
+    assert launches(0, ("dmas", 48, 5), ("xdoppler", 20, 7)) == launches(3, ("dmas", 48, 5), ("xdoppler", 20, 7)) == 6
