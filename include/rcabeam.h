@@ -321,17 +321,17 @@ rcabeam_status rcabeam_batch_prepare(size_t n, const rcabeam_batch_ensemble* lis
 
 /* Enqueues on `stream` (a cudaStream_t; capturable into a CUDA graph): clears
  * the counters and every pd, then runs the persistent kernel with ctas_per_sm
- * (1-3; at most as many as fit) CTAs per SM, or with ctas_per_sm = 0, for
- * queues of several methods, and where the ensembles share no layout that fits,
- * launches every ensemble through the single-ensemble kernels in queue order.  times (device, n + 1 uint64): start, then each
+ * (1-3; at most as many as fit) CTAs per SM, one launch per method in the order of
+ * the methods' first ensembles; a method whose ensembles share no layout that fits an
+ * SM, and with ctas_per_sm = 0 the whole queue in its order, goes through the
+ * single-ensemble kernels, ensemble by ensemble.  times (device, n + 1 uint64): start, then each
  * ensemble's completion, in global-timer nanoseconds. */
 rcabeam_status rcabeam_batch_run_device(size_t n, const rcabeam_batch_ensemble* list, void* table,
                                         size_t table_bytes, unsigned long long* times, int ctas_per_sm,
                                         void* stream);
 
-/* Kernels that rcabeam_batch_run_device launches for this queue: one where it runs
- * persistently, which a queue of one method whose ensembles share a layout that fits an
- * SM does; else the single-ensemble kernels and their time stamps. */
+/* Kernels that rcabeam_batch_run_device launches for this queue: one for each method
+ * that runs persistently; else the single-ensemble kernels and their time stamps. */
 rcabeam_status rcabeam_batch_launches(size_t n, const rcabeam_batch_ensemble* list, int ctas_per_sm,
                                       size_t* launches);
 

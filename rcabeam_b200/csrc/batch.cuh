@@ -8,8 +8,8 @@
 // ensembles share the GPU without launch gaps or tails.  XDoppler magnitudes are
 // finished per tile by the CTA that completes the tile's last frame chunk, and
 // the CTA that completes an ensemble's last item stamps its completion time.
-// A persistent launch serves one method (its kernel is compiled for it); queues
-// of several methods run as per-ensemble launches.
+// A persistent launch serves one method (its kernel is compiled for it); a queue of
+// several methods is grouped by method, one launch after another.
 #pragma once
 
 #include "common.cuh"
@@ -27,7 +27,8 @@ struct alignas(64) Ensemble {
   int method;              // 0 OPW, 1 XDoppler, 3 DMAS-CCF-ACF
   int width;               // frame pairs the kernel variant is compiled for
   int tiles;               // voxel tiles; items = tiles x shape.chunks
-  long long first_item;    // items before this ensemble
+  int index;               // position in the queue
+  long long first_item;    // items before this ensemble in its launch
   long long tile_base;     // first per-tile counter of this ensemble (XDoppler)
 };
 
@@ -39,7 +40,7 @@ struct Queue {
   unsigned long long* next;      // work counter
   unsigned* done;                // [n] completed items
   unsigned* tile_done;           // per (ensemble, tile) completed chunks (XDoppler)
-  unsigned long long* times;     // [n + 1]: kernel start, completion per ensemble (globaltimer ns)
+  unsigned long long* times;     // [queue + 1]: kernel start, completion per ensemble (globaltimer ns)
 };
 
 template <int MODE>
@@ -102,7 +103,7 @@ __global__ void __launch_bounds__(das::max_threads<MODE>(13), 1) run(const __gri
       if constexpr (MODE == das::kXdoppler)  // last chunk of this tile: the voxels' magnitudes are due
         last_chunk = atomicAdd(q.tile_done + e.tile_base + tile, 1u) + 1 == unsigned(sp.chunks);
       const unsigned d = atomicAdd(q.done + ei, 1u) + 1;
-      if (d == unsigned(e.tiles) * unsigned(sp.chunks)) q.times[1 + ei] = global_ns();
+      if (d == unsigned(e.tiles) * unsigned(sp.chunks)) q.times[1 + e.index] = global_ns();
     }
     if constexpr (MODE == das::kXdoppler) {
       __syncthreads();

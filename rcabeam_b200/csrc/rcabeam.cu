@@ -1452,120 +1452,169 @@ RowsPlan batch_item_plan(const das::Args& a, int method, int max_frames) {
                      : plan_rows<das::kOpw>(a, false, 1, max_frames);
 }
 
-// The table's ensembles and its layout; layout (of a persistent launch, smem 0
-// when the ensembles' items do not fit one) covers every ensemble's plan.
-bool batch_plan(size_t n, const rcabeam_batch_ensemble* list, std::vector<batch::Ensemble>* out, BatchLayout* L,
-                long long* total_items, das::Layout* layout) {
-  if (!n || !list || n > (1u << 20)) return false;
-  long long items = 0, tiles_xd = 0;
-  das::Layout lt{};
-  int consumers = 0, stash_unit = 0;
-  bool fits = true;
-  std::vector<batch::Ensemble> own;
-  if (!out) out = &own;
-  out->resize(n);
-  for (size_t i = 0; i < n; ++i) {
-    const rcabeam_batch_ensemble& d = list[i];
-    if (!d.rc || !d.cr || !d.scan || !d.xe || !d.ye || !d.angles || !d.starts || !d.pd || d.ns < 2 || !d.nc ||
-        !d.na || !d.nt || !d.nv || d.na > size_t(batch::kMaxAngles) || d.nv > INT32_MAX || d.ns > INT32_MAX ||
-        d.nc > INT32_MAX || d.nt > INT32_MAX || !(d.c > 0) || !(d.fs > 0) || !std::isfinite(d.c) ||
-        !std::isfinite(d.fs) || !std::isfinite(d.fd) || !std::isfinite(d.fn))
-      return false;
-    if (d.method != 0 && d.method != 1 && d.method != 3) return false;
-    const int fpc = d.frames_per_chunk ? d.frames_per_chunk : 64;
-    if (fpc != 16 && fpc != 32 && fpc != 64) return false;
-    batch::Ensemble e{};
-    das::Args& a = e.args;
-    a.rc = d.rc;
-    a.cr = d.cr;
-    a.scan = d.scan;
-    a.xe = d.xe;
-    a.ye = d.ye;
-    a.angles = d.angles;
-    a.starts = d.starts;
-    a.order = d.order;
-    a.pd = d.pd;
-    a.signal = nullptr;
-    a.ns = int(d.ns);
-    a.nc = int(d.nc);
-    a.na = int(d.na);
-    a.nt = int(d.nt);
-    a.nv = int(d.nv);
-    a.c = d.c;
-    a.fs = d.fs;
-    a.fd = d.fd;
-    a.fn = d.fn;
-    a.err = device_error_ptr();
-    // 64: the planned split; 16 or 32: items of at most that many frames.
-    const RowsPlan r = batch_item_plan(a, d.method, fpc == 64 ? INT32_MAX : fpc);
-    fits = fits && r.layout.smem;
-    e.method = d.method;
-    e.shape = r.shape;
-    e.maps = r.maps;
-    e.width = r.width;
-    e.tiles = int((d.nv + das::kTileVoxels - 1) / das::kTileVoxels);
-    e.first_item = items;
-    e.tile_base = tiles_xd;
-    items += (long long)e.tiles * e.shape.chunks;
-    if (d.method == 1) tiles_xd += e.tiles;
-    const int warps = r.layout.threads / 32 - r.layout.builders - r.layout.helpers;
-    consumers = std::max(consumers, warps);
-    stash_unit = std::max(stash_unit, r.layout.stash_bytes / (32 * warps));
-    lt.builders = i == 0 ? r.layout.builders : std::min(lt.builders, r.layout.builders);
-    lt.helpers = r.layout.helpers > 0 ? lt.builders : 0;
-    lt.stage_bytes = std::max(lt.stage_bytes, r.layout.stage_bytes);
-    lt.zero_bytes = std::max(lt.zero_bytes, r.layout.zero_bytes);
-    lt.angles = std::max(lt.angles, r.layout.angles);
-    lt.table_bytes = std::max(lt.table_bytes, r.layout.table_bytes);
-    (*out)[i] = e;
-  }
-  L->ens = 0;
-  L->next = L->ens + align256(n * sizeof(batch::Ensemble));
-  L->done = L->next + 256;
-  L->tile_done = L->done + align256(n * 4);
-  L->total = L->tile_done + align256(size_t(tiles_xd > 0 ? tiles_xd : 1) * 4);
-  *total_items = items;
-  // A launch's ring stages are the largest any ensemble plans for itself, or what
-  // is left of an SM's shared memory (less the kernel's own) beside the largest
-  // tables and stashes.
-  lt.threads = 32 * (lt.builders + lt.helpers + consumers);
-  lt.stages = 2 * lt.builders;
-  lt.stash_bytes = stash_unit * 32 * consumers;
-  const int fixed = das::kFixedBytes + 24 * lt.angles + lt.zero_bytes + lt.stash_bytes + lt.table_bytes;
-  const int room = std::max(226 * 1024 - fixed, 0) / lt.stages / 128 * 128;
-  if (room < lt.stage_bytes) {
-    lt.stage_bytes = room;
-    for (batch::Ensemble& e : *out) {
-      e.shape.rows = std::min(e.shape.rows, stage_rows(e.shape, 8, 2 * room));
-      e.shape.rows_deep = std::min(e.shape.rows_deep, stage_rows(e.shape, 8, room));
-      fits = fits && e.shape.rows >= 40;
-    }
-  }
-  lt.smem = fits ? fixed + lt.stages * lt.stage_bytes : 0;
-  if (layout) *layout = lt;
+// A queue's ensembles of one method: consecutive in the table, one persistent launch
+// (layout.smem 0: they share no layout that fits and run one by one).
+struct BatchGroup {
+  size_t first, n;  // table entries
+  long long items;
+  das::Layout layout;  // covers every ensemble's plan
+};
+
+// Table entry of queue position i; false when the description is invalid.
+bool batch_entry(const rcabeam_batch_ensemble& d, size_t i, batch::Ensemble* out, RowsPlan* plan) {
+  if (!d.rc || !d.cr || !d.scan || !d.xe || !d.ye || !d.angles || !d.starts || !d.pd || d.ns < 2 || !d.nc ||
+      !d.na || !d.nt || !d.nv || d.na > size_t(batch::kMaxAngles) || d.nv > INT32_MAX || d.ns > INT32_MAX ||
+      d.nc > INT32_MAX || d.nt > INT32_MAX || !(d.c > 0) || !(d.fs > 0) || !std::isfinite(d.c) ||
+      !std::isfinite(d.fs) || !std::isfinite(d.fd) || !std::isfinite(d.fn))
+    return false;
+  if (d.method != 0 && d.method != 1 && d.method != 3) return false;
+  const int fpc = d.frames_per_chunk ? d.frames_per_chunk : 64;
+  if (fpc != 16 && fpc != 32 && fpc != 64) return false;
+  batch::Ensemble e{};
+  das::Args& a = e.args;
+  a.rc = d.rc;
+  a.cr = d.cr;
+  a.scan = d.scan;
+  a.xe = d.xe;
+  a.ye = d.ye;
+  a.angles = d.angles;
+  a.starts = d.starts;
+  a.order = d.order;
+  a.pd = d.pd;
+  a.signal = nullptr;
+  a.ns = int(d.ns);
+  a.nc = int(d.nc);
+  a.na = int(d.na);
+  a.nt = int(d.nt);
+  a.nv = int(d.nv);
+  a.c = d.c;
+  a.fs = d.fs;
+  a.fd = d.fd;
+  a.fn = d.fn;
+  a.err = device_error_ptr();
+  // 64: the planned split; 16 or 32: items of at most that many frames.
+  *plan = batch_item_plan(a, d.method, fpc == 64 ? INT32_MAX : fpc);
+  e.method = d.method;
+  e.shape = plan->shape;
+  e.maps = plan->maps;
+  e.width = plan->width;
+  e.tiles = int((d.nv + das::kTileVoxels - 1) / das::kTileVoxels);
+  e.index = int(i);
+  *out = e;
   return true;
 }
 
-// Whether a queue runs as one persistent kernel: one method, and a layout that fits.
-bool batch_persistent(size_t n, const rcabeam_batch_ensemble* list, int ctas_per_sm, const das::Layout& layout) {
-  for (size_t i = 1; i < n; ++i)
-    if (list[i].method != list[0].method) return false;
-  return ctas_per_sm > 0 && layout.smem > 0;
+// Widens a group's layout so that it covers one more plan.
+void batch_widen(das::Layout* lt, const das::Layout& l, int* consumers, int* stash_unit) {
+  const int warps = l.threads / 32 - l.builders - l.helpers;
+  *consumers = std::max(*consumers, warps);
+  *stash_unit = std::max(*stash_unit, l.stash_bytes / (32 * warps));
+  lt->builders = lt->builders ? std::min(lt->builders, l.builders) : l.builders;
+  lt->helpers = l.helpers > 0 ? lt->builders : 0;
+  lt->stage_bytes = std::max(lt->stage_bytes, l.stage_bytes);
+  lt->zero_bytes = std::max(lt->zero_bytes, l.zero_bytes);
+  lt->angles = std::max(lt->angles, l.angles);
+  lt->table_bytes = std::max(lt->table_bytes, l.table_bytes);
 }
 
-batch::Queue batch_queue(void* table, size_t n, const BatchLayout& L, long long total, const das::Layout& layout,
+// The table's entries, grouped by method in the order of their first ensembles, and
+// the table's layout.
+bool batch_plan(size_t n, const rcabeam_batch_ensemble* list, std::vector<batch::Ensemble>* out,
+                std::vector<BatchGroup>* groups, BatchLayout* L) {
+  if (!n || !list || n > (1u << 20)) return false;
+  long long tiles_xd = 0;
+  out->clear();
+  groups->clear();
+  for (size_t lead = 0; lead < n; ++lead) {
+    if (std::any_of(list, list + lead, [&](const auto& d) { return d.method == list[lead].method; })) continue;
+    BatchGroup g{out->size(), 0, 0, {}};
+    das::Layout& lt = g.layout;
+    int consumers = 0, stash_unit = 0;
+    bool fits = true;
+    for (size_t i = lead; i < n; ++i) {
+      if (list[i].method != list[lead].method) continue;
+      batch::Ensemble e{};
+      RowsPlan r{};
+      if (!batch_entry(list[i], i, &e, &r)) return false;
+      e.first_item = g.items;
+      e.tile_base = tiles_xd;
+      g.items += (long long)e.tiles * e.shape.chunks;
+      if (e.method == 1) tiles_xd += e.tiles;
+      fits = fits && r.layout.smem;
+      batch_widen(&lt, r.layout, &consumers, &stash_unit);
+      out->push_back(e);
+    }
+    g.n = out->size() - g.first;
+    // The ring's stages are the largest any ensemble plans for itself, or what is left
+    // of an SM's shared memory (less the kernel's own) beside the largest tables and
+    // stashes.
+    lt.threads = 32 * (lt.builders + lt.helpers + consumers);
+    lt.stages = 2 * lt.builders;
+    lt.stash_bytes = stash_unit * 32 * consumers;
+    const int fixed = das::kFixedBytes + 24 * lt.angles + lt.zero_bytes + lt.stash_bytes + lt.table_bytes;
+    const int room = std::max(226 * 1024 - fixed, 0) / lt.stages / 128 * 128;
+    if (room < lt.stage_bytes) {
+      lt.stage_bytes = room;
+      for (size_t i = g.first; i < out->size(); ++i) {
+        das::Shape& sp = (*out)[i].shape;
+        sp.rows = std::min(sp.rows, stage_rows(sp, 8, 2 * room));
+        sp.rows_deep = std::min(sp.rows_deep, stage_rows(sp, 8, room));
+        fits = fits && sp.rows >= 40;
+      }
+    }
+    lt.smem = fits ? fixed + lt.stages * lt.stage_bytes : 0;
+    groups->push_back(g);
+  }
+  L->ens = 0;
+  L->next = L->ens + align256(n * sizeof(batch::Ensemble));
+  L->done = L->next + 256;  // one counter per group
+  L->tile_done = L->done + align256(n * 4);
+  L->total = L->tile_done + align256(size_t(tiles_xd > 0 ? tiles_xd : 1) * 4);
+  return true;
+}
+
+batch::Queue batch_queue(void* table, const BatchLayout& L, const BatchGroup& g, int counter,
                          unsigned long long* times) {
   unsigned char* t = static_cast<unsigned char*>(table);
   batch::Queue q{};
-  q.ens = reinterpret_cast<const batch::Ensemble*>(t + L.ens);
-  q.layout = layout;
-  q.n = int(n);
-  q.total_items = total;
-  q.next = reinterpret_cast<unsigned long long*>(t + L.next);
-  q.done = reinterpret_cast<unsigned*>(t + L.done);
+  q.ens = reinterpret_cast<const batch::Ensemble*>(t + L.ens) + g.first;
+  q.layout = g.layout;
+  q.n = int(g.n);
+  q.total_items = g.items;
+  q.next = reinterpret_cast<unsigned long long*>(t + L.next) + counter;
+  q.done = reinterpret_cast<unsigned*>(t + L.done) + g.first;
   q.tile_done = reinterpret_cast<unsigned*>(t + L.tile_done);
   q.times = times;
   return q;
+}
+
+// Entries [first, first + n) of the table through the single-ensemble kernels, a
+// completion stamp after each.
+rcabeam_status batch_grids(const std::vector<batch::Ensemble>& ens, size_t first, size_t n, unsigned long long* times,
+                           cudaStream_t stream) {
+  batch::stamp<<<1, 1, 0, stream>>>(times, 1);
+  for (size_t i = first; i < first + n; ++i) {
+    const rcabeam_status r = run_method(ens[i].args, ens[i].method, stream);
+    if (r != RCABEAM_SUCCESS) return r;
+    batch::stamp<<<1, 1, 0, stream>>>(times + 1 + ens[i].index, 0);
+  }
+  return launch_status();
+}
+
+rcabeam_status batch_run_group(void* table, const BatchLayout& L, const BatchGroup& g, int method, int counter,
+                               unsigned long long* times, int ctas_per_sm, cudaStream_t stream) {
+  using Kernel = void (*)(const batch::Queue);
+  const Kernel kern = method == 3   ? batch::run<das::kDmas>
+                      : method == 1 ? batch::run<das::kXdoppler>
+                                    : batch::run<das::kOpw>;
+  if (!open_smem(kern, 1024)) return RCABEAM_ERROR_CUDA;
+  int resident = 1;
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, kern, g.layout.threads, g.layout.smem) != cudaSuccess)
+    return RCABEAM_ERROR_CUDA;
+  const long long want = (long long)sm_count() * std::max(1, std::min(resident, ctas_per_sm));
+  kern<<<unsigned(std::min(g.items, want)), g.layout.threads, g.layout.smem, stream>>>(
+      batch_queue(table, L, g, counter, times));
+  return launch_status();
 }
 }  // namespace
 
@@ -1573,8 +1622,9 @@ extern "C" {
 
 rcabeam_status rcabeam_batch_table_bytes(size_t n, const rcabeam_batch_ensemble* list, size_t* bytes) {
   BatchLayout L;
-  long long total = 0;
-  if (!bytes || !batch_plan(n, list, nullptr, &L, &total, nullptr)) return RCABEAM_ERROR_ARGUMENT;
+  std::vector<batch::Ensemble> ens;
+  std::vector<BatchGroup> groups;
+  if (!bytes || !batch_plan(n, list, &ens, &groups, &L)) return RCABEAM_ERROR_ARGUMENT;
   *bytes = L.total;
   return RCABEAM_SUCCESS;
 }
@@ -1582,10 +1632,10 @@ rcabeam_status rcabeam_batch_table_bytes(size_t n, const rcabeam_batch_ensemble*
 rcabeam_status rcabeam_batch_prepare(size_t n, const rcabeam_batch_ensemble* list, void* table,
                                      size_t table_bytes) {
   BatchLayout L;
-  long long total = 0;
   std::vector<batch::Ensemble> ens;
-  if (!table || reinterpret_cast<uintptr_t>(table) % 256 != 0 ||
-      !batch_plan(n, list, &ens, &L, &total, nullptr) || table_bytes < L.total)
+  std::vector<BatchGroup> groups;
+  if (!table || reinterpret_cast<uintptr_t>(table) % 256 != 0 || !batch_plan(n, list, &ens, &groups, &L) ||
+      table_bytes < L.total)
     return RCABEAM_ERROR_ARGUMENT;
   return cudaMemcpy(static_cast<unsigned char*>(table) + L.ens, ens.data(), n * sizeof(batch::Ensemble),
                     cudaMemcpyHostToDevice) == cudaSuccess
@@ -1597,10 +1647,9 @@ rcabeam_status rcabeam_batch_run_device(size_t n, const rcabeam_batch_ensemble* 
                                         size_t table_bytes, unsigned long long* times, int ctas_per_sm,
                                         void* stream) {
   BatchLayout L;
-  long long total = 0;
-  das::Layout layout{};
   std::vector<batch::Ensemble> ens;
-  if (!table || !times || ctas_per_sm < 0 || ctas_per_sm > 3 || !batch_plan(n, list, &ens, &L, &total, &layout) ||
+  std::vector<BatchGroup> groups;
+  if (!table || !times || ctas_per_sm < 0 || ctas_per_sm > 3 || !batch_plan(n, list, &ens, &groups, &L) ||
       table_bytes < L.total)
     return RCABEAM_ERROR_ARGUMENT;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
@@ -1611,41 +1660,34 @@ rcabeam_status rcabeam_batch_run_device(size_t n, const rcabeam_batch_ensemble* 
     return RCABEAM_ERROR_CUDA;
   for (size_t i = 0; i < n; ++i)
     if (cudaMemsetAsync(list[i].pd, 0, 2 * list[i].nv * sizeof(float), st) != cudaSuccess) return RCABEAM_ERROR_CUDA;
-  if (!batch_persistent(n, list, ctas_per_sm, layout)) {
-    // Each ensemble through the single-ensemble kernels on the stream, a
-    // completion stamp after each.
-    batch::stamp<<<1, 1, 0, st>>>(times, 1);
-    for (size_t i = 0; i < n; ++i) {
-      const rcabeam_status r = run_method(ens[i].args, list[i].method, st);
-      if (r != RCABEAM_SUCCESS) return r;
-      batch::stamp<<<1, 1, 0, st>>>(times + 1 + i, 0);
-    }
-    return launch_status();
+  if (ctas_per_sm == 0) {  // each on its own, in queue order
+    std::sort(ens.begin(), ens.end(), [](const auto& a, const auto& b) { return a.index < b.index; });
+    return batch_grids(ens, 0, n, times, st);
   }
-  using Kernel = void (*)(const batch::Queue);
-  const Kernel kern = list[0].method == 3   ? batch::run<das::kDmas>
-                      : list[0].method == 1 ? batch::run<das::kXdoppler>
-                                            : batch::run<das::kOpw>;
-  if (!open_smem(kern, 1024)) return RCABEAM_ERROR_CUDA;
-  int resident = 1;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, kern, layout.threads, layout.smem) != cudaSuccess)
-    return RCABEAM_ERROR_CUDA;
-  const long long want = (long long)sm_count() * std::max(1, std::min(resident, ctas_per_sm));
-  kern<<<unsigned(std::min(total, want)), layout.threads, layout.smem, st>>>(
-      batch_queue(table, n, L, total, layout, times));
-  return launch_status();
+  for (size_t k = 0; k < groups.size(); ++k) {
+    const BatchGroup& g = groups[k];
+    const rcabeam_status r =
+        g.layout.smem ? batch_run_group(table, L, g, ens[g.first].method, int(k), times, ctas_per_sm, st)
+                      : batch_grids(ens, g.first, g.n, times, st);
+    if (r != RCABEAM_SUCCESS) return r;
+  }
+  return RCABEAM_SUCCESS;
 }
 
 rcabeam_status rcabeam_batch_launches(size_t n, const rcabeam_batch_ensemble* list, int ctas_per_sm,
                                       size_t* launches) {
   BatchLayout L;
-  long long total = 0;
-  das::Layout layout{};
-  if (!launches || ctas_per_sm < 0 || ctas_per_sm > 3 || !batch_plan(n, list, nullptr, &L, &total, &layout))
+  std::vector<batch::Ensemble> ens;
+  std::vector<BatchGroup> groups;
+  if (!launches || ctas_per_sm < 0 || ctas_per_sm > 3 || !batch_plan(n, list, &ens, &groups, &L))
     return RCABEAM_ERROR_ARGUMENT;
-  *launches = 1;  // the persistent kernel, or the start stamp
-  if (!batch_persistent(n, list, ctas_per_sm, layout))
-    for (size_t i = 0; i < n; ++i) *launches += list[i].method == 1 ? 3 : 2;  // XDoppler: magnitudes too; a stamp
+  // Persistent: one kernel.  One by one: a start stamp, and per ensemble its kernel
+  // (XDoppler: and its magnitudes) and a stamp.
+  *launches = ctas_per_sm == 0 ? 1 : 0;
+  for (const BatchGroup& g : groups) {
+    const bool persistent = ctas_per_sm > 0 && g.layout.smem;
+    *launches += persistent ? 1 : (ctas_per_sm > 0) + g.n * (ens[g.first].method == 1 ? 3 : 2);
+  }
   return RCABEAM_SUCCESS;
 }
 

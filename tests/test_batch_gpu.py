@@ -9,6 +9,8 @@ launch and from CUDA-graph replays, with autotuned frame chunks.
 
 from __future__ import annotations
 
+import ctypes
+
 import numpy as np
 import pytest
 import torch
@@ -102,6 +104,35 @@ def test_graph_replay_and_autotune():
         torch.cuda.synchronize()
         for e, w in zip(ens, want):
             assert rel_l2(e.power().cpu().numpy(), w.cpu().numpy()) <= 1e-5, e.method
+
+
+@pytest.mark.parametrize("ctas", [0, 1, 3])
+def test_mixed_list_through_the_c_interface(ctas):
+    """Methods in one list: power and completion times land at each ensemble's own position."""
+    ens = _queue(seed=9)
+    want = _single(ens)
+    lib, n = batching._declare(), len(ens)
+    items = (batching.BatchEnsembleC * n)(*[e.descriptor() for e in ens])
+    size = ctypes.c_size_t(0)
+    assert lib.rcabeam_batch_table_bytes(n, items, ctypes.byref(size)) == 0
+    table = torch.empty(size.value + 256, dtype=torch.uint8, device="cuda")
+    base = (table.data_ptr() + 255) // 256 * 256
+    times = torch.zeros(n + 1, dtype=torch.int64, device="cuda")
+    assert lib.rcabeam_batch_prepare(n, items, base, size.value) == 0
+    stream = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+    assert lib.rcabeam_batch_run_device(n, items, base, size.value, times.data_ptr(), ctas, stream) == 0
+    torch.cuda.synchronize()
+    for e, w in zip(ens, want):
+        assert rel_l2(e.power().cpu().numpy(), w.cpu().numpy()) <= 1e-5, e.method
+    done = times.cpu().numpy()
+    assert (done[1:] > done[0]).all()
+    methods = [e.method for e in ens]
+    first = {m: done[1:][[m == k for k in methods]].min() for m in set(methods)}
+    last = {m: done[1:][[m == k for k in methods]].max() for m in set(methods)}
+    if ctas:  # one launch per method, in the order of their first ensembles
+        assert last["opw"] <= first["xdoppler"] and last["xdoppler"] <= first["dmas"]
+    else:
+        assert (np.diff(done) > 0).all()
 
 
 def test_invalid_queue_entries_are_rejected():

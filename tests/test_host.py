@@ -177,8 +177,8 @@ def test_downloads_convert_types(monkeypatch, elements, source, target):
 
 
 def test_queue_launches_follow_the_layout(built_library):
-    """One kernel where a method's ensembles share a layout; per ensemble one and a time stamp
-    (XDoppler two) where a long angle table beside wide stashes leaves no room, or methods differ."""
+    """One kernel per method whose ensembles share a layout; per ensemble one and a time stamp
+    (XDoppler two) where a long angle table beside wide stashes leaves no room, or on request."""
     from rcabeam_b200 import batching
 
     lib = batching._declare()
@@ -193,4 +193,6 @@ def test_queue_launches_follow_the_layout(built_library):
 
     assert launches(3, ("dmas", 48, 5), ("dmas", 20, 7)) == 1
     assert launches(3, ("dmas", 48, 5), ("dmas", 7, 64)) == 5
-    assert launches(0, ("dmas", 48, 5), ("xdoppler", 20, 7)) == launches(3, ("dmas", 48, 5), ("xdoppler", 20, 7)) == 6
+    assert launches(0, ("dmas", 48, 5), ("xdoppler", 20, 7)) == 6
+    assert launches(3, ("dmas", 48, 5), ("xdoppler", 20, 7), ("dmas", 20, 5)) == 2
+    assert launches(3, ("dmas", 48, 5), ("xdoppler", 20, 7), ("dmas", 7, 64)) == 6
