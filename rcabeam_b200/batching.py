@@ -9,9 +9,9 @@ large ensembles share the GPU without launch gaps or per-ensemble tails, with
 a kernel compiled for that method alone) or as per-ensemble launches of the
 single-ensemble kernels (``ctas_per_sm`` 0), whichever ``autotune`` measures
 faster for that method on bounded samples of its ensembles (it also picks the
-most frames of an item per shape class).  The sub-queues run one after another on one stream (run concurrently, their
-sample windows compete for L2) and the whole queue is captured into one CUDA
-graph.  Per-ensemble completion times come from the device's global timer.
+most frames of an item per shape class).  The sub-queues run one after another
+on one stream (run concurrently, their sample windows compete for L2) and the
+whole queue is captured into one CUDA graph.  Per-ensemble completion times come from the device's global timer.
 
 Methods: "opw" (power of the coherent sum), "xdoppler" (|mean r conj(q)|) and
 "dmas" (DMAS-CCF-ACF), as in ``ensemble_pd_from_channels`` (reference
@@ -121,8 +121,9 @@ class Ensemble:
 
 class _SubQueue:
     """The ensembles of one method: device table, completion times, and how it runs:
-    ``ctas_per_sm`` 1-3 is the persistent kernel at that many CTAs per SM, 0 the
-    single-ensemble kernels launched per ensemble on the sub-queue's stream."""
+    ``ctas_per_sm`` 1-3 is the persistent kernel at that many CTAs per SM (at most as
+    many as fit), 0 the single-ensemble kernels launched per ensemble on the
+    sub-queue's stream."""
 
     def __init__(self, lib, indices, ensembles, ctas_per_sm: int, voxel_limit: int | None, device):
         self.lib = lib

@@ -469,14 +469,11 @@ __global__ void __launch_bounds__(kAsyncThreads, 2)
           const double2 r = subtract ? make_double2(xv[f].x - proj.x, xv[f].y - proj.y) : proj;
           pw += r.x * r.x + r.y * r.y;
           if (mode & 2) {
-            if constexpr (sizeof(IN) == 8)
-              {
+            if constexpr (sizeof(IN) == 8) {
               const float2 w = make_float2(float(r.x), float(r.y));
               bad_row |= !isfinite(w.x) || !isfinite(w.y);
               reinterpret_cast<float2*>(out)[row * nt + t] = w;
-            }
-            else
-              {
+            } else {
               bad_row |= !isfinite(r.x) || !isfinite(r.y);
               reinterpret_cast<double2*>(out)[row * nt + t] = r;
             }

@@ -1,7 +1,8 @@
 // Frame-batched RCA delay-and-sum on the CUDA cores (float32 arithmetic, exact
 // geometry): OPW, XDoppler, separate apertures, RC-FMAS, DMAS-CCF-ACF and the
-// subset statistics of St-SW from one staged pipeline.  The reference does the same
-// arithmetic per sample from a per-call geometry table (ensemble.cu:143-454).
+// subset statistics of St-SW from one staged pipeline (the last three from a few
+// thousand voxels on: das_generic.cuh).  The reference does the same arithmetic per
+// sample from a per-call geometry table (ensemble.cu:143-454).
 //
 // Work: an item is a tile of 128 voxels (consecutive in a spatially compact
 // order) x a chunk of up to 104 frames; a CTA runs one.  Its steps are the
@@ -179,9 +180,10 @@ __device__ __forceinline__ Shared carve(unsigned char* smem, const Layout& l) {
 
 // ------------------------------------------------------------------ delays --
 // Sample positions and demodulation cycles are summed as fixed-point numbers of
-// 2^-32 (a quarter of the float32 weight's last bit at its smallest): a step's
-// tap then costs a 64-bit and a 32-bit integer addition per voxel, and the
-// cycles wrap by themselves.
+// 2^-32: a step's tap then costs a 64-bit and a 32-bit integer addition per voxel, and
+// the cycles wrap by themselves.  The position's rounding is below that of the float32
+// weight formed from it for weights from 2^-8 on; smaller weights are off by up to
+// 2.3e-10 of a sample interval, against sums whose float32 rounding is 1e-7.
 constexpr long long kNever = -(1ll << 62);      // a delay outside every window
 constexpr double kFixedLimit = 536870912.0;     // |delay| < 2^29 samples
 
@@ -1008,13 +1010,13 @@ struct Consumer {
       ready = tag != kTagEnd && mbar_test(&sh.full[stage], (phase >> stage) & 1);
       if constexpr (MODE != kOpw) {
         if (tag != kTagEnd) {
-        int t = tag & kTagMask;
-        // The two-aperture methods fold once, between the apertures.
-        if constexpr (MODE == kXdoppler || MODE == kApertures) t = t >= p.nc ? 1 : 0;
-        if (t != open) {
-          if (open >= 0) fold(open);
-          open = t;
-        }
+          int t = tag & kTagMask;
+          // The two-aperture methods fold once, between the apertures.
+          if constexpr (MODE == kXdoppler || MODE == kApertures) t = t >= p.nc ? 1 : 0;
+          if (t != open) {
+            if (open >= 0) fold(open);
+            open = t;
+          }
         }
       }
       if (work && (meta.y >> block & 1)) {

@@ -68,7 +68,7 @@ static bool make_plane_map(CUtensorMap* map, const void* base, size_t nt, size_t
 
 // -------------------------------------------------- voxel traversal order --
 // Morton (Z-order) codes of isotropically quantized voxel positions, sorted
-// with a radix sort, give tiles of 64 consecutive voxels that are compact in
+// with a radix sort, give tiles of 128 consecutive voxels that are compact in
 // space -- which keeps each tile's sample window short.  Uses the caller's
 // geometry workspace as scratch; returns nullptr (identity order) when the
 // call is small or the scratch does not fit.
@@ -210,10 +210,6 @@ struct RowsPlan {
   int width;  // frame pairs the kernel variant is compiled for
 };
 
-// Items of up to 104 frames (OPW; fewer for the methods that keep partial
-// results in shared memory).  13 pairs per thread keep a tap's cost small beside
-// its 26 frames; up to 32 frames run 8 pairs, whose kernel leaves room for
-// several CTAs per SM.
 // Sample rows that `bytes` of a stage hold beside the taps.
 static int stage_rows(const das::Shape& sp, int elem, int bytes) {
   const int slack = sp.frames * elem + 64;  // threads past the last frame read on
@@ -221,6 +217,10 @@ static int stage_rows(const das::Shape& sp, int elem, int bytes) {
   return sp.boxes ? std::min(n / das::kBoxRows, das::kMaxBoxes) * das::kBoxRows : n;
 }
 
+// Items of up to 104 frames (OPW; fewer for the methods that keep partial
+// results in shared memory).  13 pairs per thread keep a tap's cost small beside
+// its 26 frames; up to 32 frames run 8 pairs, whose kernel leaves room for
+// several CTAs per SM.
 template <int MODE>
 static RowsPlan plan_items(const das::Args& a, bool half, int sms, int most) {
   constexpr int kStash = das::kStash<MODE>;
