@@ -531,9 +531,9 @@ struct Builder {
       turn = lt.builders;
     }
     --turn;
-    if (!ok)  // copies under way land before the CTA may leave
-      for (int st = warp; st < ring.stages; st += lt.builders)
-        mbar_wait(&sh.full[st], ((phase >> st) & 1) ^ 1, p.err, kErrWaitDrain);
+    // Copies under way land before the CTA may leave, also where consumers gave up waiting.
+    for (int st = warp; st < ring.stages; st += lt.builders)
+      mbar_wait(&sh.full[st], ((phase >> st) & 1) ^ 1, p.err, kErrWaitDrain);
   }
 
   // Both apertures, channel by channel; tag = first + aperture * nc + channel.
